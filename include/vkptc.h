@@ -65,12 +65,12 @@ typedef struct vkptc_config {
   int32_t device;            /* CUDA device ordinal */
   uint32_t block_size;       /* threads per block of the wavefront kernels; 0 = autotuned/default */
   uint32_t stack_depth;      /* traversal stack entries per thread kept in shared memory (the rest
-                                spill to global memory); 0 = 16 */
+                                spill to global memory); 0 = 12 */
   uint32_t math_mode;        /* 0 = parity (transcendentals in FP64, rounded once), 1 = fast FP32 */
   uint32_t collect_stats;    /* 1 = count node/leaf/triangle visits (device counters) */
   uint32_t wave_paths;       /* paths per wavefront wave (0 = 4 Mi) */
   uint32_t stage_timing;     /* 1 = CUDA-event timing of every stage launch */
-  uint32_t steps;            /* traversal steps between warp refills in the low 16 bits (0 = 4); the
+  uint32_t steps;            /* traversal steps between warp refills in the low 16 bits (0 = 8); the
                                 high 16 bits, when non-zero, refill a warp as soon as that many of its
                                 lanes are idle (at most 32), checked after every step */
   uint32_t bvh_mode;         /* traversal tree: VKPTC_BVH_REFERENCE (the reference builder's tree,
@@ -344,7 +344,8 @@ typedef struct vkptc_scene_delta {
 int32_t vkptc_update_scene_delta(vkptc_ctx* ctx, const vkptc_scene_delta* delta);
 /* Extension (no reference counterpart): copies one device array of the built
  * accelerator to host memory, for inspection and for checking the device
- * build against the host build.  what: VKPTC_ACCEL_WIDE_NODES (128 B each),
+ * build against the host build.  what: VKPTC_ACCEL_WIDE_NODES (128 B each: the children's
+ * boxes as centre and half extent, then their refs),
  * VKPTC_ACCEL_TRIANGLES (48 B each, leaf order), VKPTC_ACCEL_TIE_NODES (32 B
  * each, the reference binary tree), VKPTC_ACCEL_SHADING (16 B per primitive).
  * *bytes receives the array's size; out may be NULL to query it. */

@@ -44,7 +44,7 @@ __device__ __forceinline__ uint32_t mat_slot(const DevScene& s, uint32_t mat_ind
 // vertex flags): two evaluations with equal hashes took the same branches.
 template <bool kParity, bool kRecord>
 __device__ __forceinline__ float4 adj_primal(const DevScene& s, const DevSettings& st, const float* mat0,
-                                             uint32_t x, uint32_t y, uint32_t sample, SmemStack stk,
+                                             uint32_t x, uint32_t y, uint32_t sample, const TwoLevelStack& stk,
                                              uint32_t& err, AdjRec* rec, uint32_t& nrec, uint32_t rec_stride = 1u) {
   V3 o, d;
   uint64_t rng;
@@ -57,7 +57,7 @@ __device__ __forceinline__ float4 adj_primal(const DevScene& s, const DevSetting
   for (uint32_t depth = 0; depth < st.max_depth; ++depth) {
     float t;
     uint32_t prim;
-    trace_closest<false>(s, prep_ray(o, d, s.reference_tree != 0u), stk, t, prim, ts, err);
+    trace_closest<false>(s, o, d, stk, t, prim, ts, err);
     if (prim == kMiss) {
       rad = add(rad, mulv(thr, s.env));
       sig = mix64(sig ^ 0xFFFFFFFFull);
@@ -86,8 +86,7 @@ __device__ __forceinline__ float4 adj_primal(const DevScene& s, const DevSetting
     if (R.nee) {
       const V3 c = st.enable_mis ? mul(mulv(thr, R.q.radiance), R.w_n) : mulv(thr, R.q.radiance);
       bool vis = true;
-      if (R.q.remain > 0.004f) vis = !trace_any<false>(s, prep_ray(R.q.origin, R.q.dir, s.reference_tree != 0u),
-                                                       R.q.remain, stk, ts, err);
+      if (R.q.remain > 0.004f) vis = !trace_any<false>(s, R.q.origin, R.q.dir, R.q.remain, stk, ts, err);
       if (vis) {
         rad = add(rad, c);
         flags |= kVfNeeVis;
@@ -136,7 +135,7 @@ __global__ void __launch_bounds__(128, 5) k_adj_forward(DevScene s, DevSettings 
                                                      uint32_t first_sample, int cap, float4* rad, AdjRec* recs,
                                                      uint32_t* nrec_out, uint32_t* err) {
   extern __shared__ int2 smem_stack[];
-  SmemStack stk{smem_stack + threadIdx.x, static_cast<int>(blockDim.x), cap};
+  const TwoLevelStack stk = smem_stack_of(smem_stack + threadIdx.x, static_cast<int>(blockDim.x), cap);
   const uint32_t npx = st.width * st.height;
   const uint64_t n = static_cast<uint64_t>(npx) * spp;
   uint32_t local_err = 0u;
@@ -362,7 +361,7 @@ __global__ void __launch_bounds__(128, 5) k_adj_replay(DevScene s, DevSettings s
                                                     const float* path_weight, uint64_t base, uint32_t count,
                                                     AdjRec* recs, float4* gout, uint32_t* err) {
   extern __shared__ int2 smem_dyn[];
-  SmemStack stk{smem_dyn + threadIdx.x, static_cast<int>(blockDim.x), cap};
+  const TwoLevelStack stk = smem_stack_of(smem_dyn + threadIdx.x, static_cast<int>(blockDim.x), cap);
   const uint32_t npx = st.width * st.height;
   uint32_t local_err = 0u;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {

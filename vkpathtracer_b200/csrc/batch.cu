@@ -76,6 +76,8 @@ struct BatchExtendSource {
   const float4* ray_o;
   const float4* ray_d;
   float2* hit;
+  static constexpr bool kUniform = false;
+  __device__ __forceinline__ GeoView geo_at(uint32_t j) const { return job_geo(jobs, job[q[j]]); }
   __device__ __forceinline__ void load(uint32_t j, V3& o, V3& d, float& tm, GeoView& g) const {
     const uint32_t slot = q[j];
     g = job_geo(jobs, job[slot]);
@@ -97,6 +99,8 @@ struct BatchShadowSource {
   const float4* sh_d;
   const float4* sh_c;
   float4* rad;
+  static constexpr bool kUniform = false;
+  __device__ __forceinline__ GeoView geo_at(uint32_t j) const { return job_geo(jobs, job[q[j]]); }
   __device__ __forceinline__ void load(uint32_t j, V3& o, V3& d, float& tm, GeoView& g) const {
     const uint32_t slot = q[j];
     g = job_geo(jobs, job[slot]);

@@ -59,8 +59,10 @@ struct LoopExtendSource {
   const DevJob* jobs;
   PathSoA A;
   float2* hit;
+  static constexpr bool kUniform = false;
+  __device__ __forceinline__ GeoView geo_at(uint32_t j) const { return job_geo(jobs, A.job[j]); }
   __device__ __forceinline__ void load(uint32_t j, V3& o, V3& d, float& tm, GeoView& g) const {
-    g = job_geo(jobs, A.job[j]);
+    g = geo_at(j);
     const float4 a = A.o[j], b = A.d[j];
     o = mk(a.x, a.y, a.z);
     d = mk(b.x, b.y, b.z);
@@ -75,6 +77,8 @@ struct LoopShadowSource {
   const DevJob* jobs;
   LoopPool P;
   PathSoA B;   // the next generation (destinations of surviving paths)
+  static constexpr bool kUniform = false;
+  __device__ __forceinline__ GeoView geo_at(uint32_t j) const { return job_geo(jobs, __float_as_uint(P.sh_d[j].w)); }
   __device__ __forceinline__ void load(uint32_t j, V3& o, V3& d, float& tm, GeoView& g) const {
     const float4 a = P.sh_o[j], b = P.sh_d[j];
     g = job_geo(jobs, __float_as_uint(b.w));

@@ -1220,9 +1220,7 @@ __global__ void k_wide_write(WideArrays W, uint32_t n_wide, WideNode* __restrict
   const WTemp w = W.w[x];
   WideNode n;
   for (int k = 0; k < 4; ++k) {
-    n.lox[k] = n.loy[k] = n.loz[k] = 1.0f;
-    n.hix[k] = n.hiy[k] = n.hiz[k] = -1.0f;
-    n.child[k] = kEmptyChild;
+    ClearWideSlot(n, k);
     n.meta[k] = 0;
   }
   n.meta[0] = w.nslots;
@@ -1230,12 +1228,7 @@ __global__ void k_wide_write(WideArrays W, uint32_t n_wide, WideNode* __restrict
     for (int k = 0; k < 4; ++k) W.slot_bin[4 * W.final_id[x] + k] = k < w.nslots ? w.slot[k] : -1;
   for (int k = 0; k < w.nslots; ++k) {
     const BinNode c = W.bin[w.slot[k]];
-    n.lox[k] = c.lo[0];
-    n.loy[k] = c.lo[1];
-    n.loz[k] = c.lo[2];
-    n.hix[k] = c.hi[0];
-    n.hiy[k] = c.hi[1];
-    n.hiz[k] = c.hi[2];
+    SetWideSlot(n, k, c.lo, c.hi);
     n.child[k] = c.count > 0 ? ~static_cast<int32_t>((static_cast<uint32_t>(c.first) << 3) |
                                                      static_cast<uint32_t>(c.count - 1))
                              : W.final_id[w.child[k]];
@@ -1595,12 +1588,7 @@ __global__ void k_refit_wide(WideNode* __restrict__ wide, uint32_t n_wide, const
     const int32_t b = slot_bin[4 * w + k];
     if (b < 0) continue;
     const BinNode c = bin[b];
-    wide[w].lox[k] = c.lo[0];
-    wide[w].loy[k] = c.lo[1];
-    wide[w].loz[k] = c.lo[2];
-    wide[w].hix[k] = c.hi[0];
-    wide[w].hiy[k] = c.hi[1];
-    wide[w].hiz[k] = c.hi[2];
+    SetWideSlot(wide[w], k, c.lo, c.hi);
   }
 }
 

@@ -522,20 +522,11 @@ void CollapseToWide(const SceneGeometry& geo, const std::vector<BinNode>& bin,
     out.depth = std::max(out.depth, level + 1u);
     out.stack_required = std::max(out.stack_required, stack_here);
     WideNode wn{};
-    for (int k = 0; k < 4; ++k) {
-      wn.lox[k] = wn.loy[k] = wn.loz[k] = 1.0f;
-      wn.hix[k] = wn.hiy[k] = wn.hiz[k] = -1.0f;
-      wn.child[k] = kEmptyChild;
-    }
+    for (int k = 0; k < 4; ++k) ClearWideSlot(wn, k);
     wn.meta[0] = static_cast<int32_t>(slots.size());
     for (size_t s = 0; s < slots.size(); ++s) {
       const BinNode& c = bin[static_cast<size_t>(slots[s])];
-      wn.lox[s] = c.lo[0];
-      wn.loy[s] = c.lo[1];
-      wn.loz[s] = c.lo[2];
-      wn.hix[s] = c.hi[0];
-      wn.hiy[s] = c.hi[1];
-      wn.hiz[s] = c.hi[2];
+      SetWideSlot(wn, static_cast<int>(s), c.lo, c.hi);
     }
     for (size_t s = 0; s < slots.size(); ++s) {
       const BinNode& c = bin[static_cast<size_t>(slots[s])];

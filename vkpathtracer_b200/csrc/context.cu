@@ -308,7 +308,6 @@ DevScene dev_scene(const vkptc_ctx* c) {
   s.iris_one_minus_round = 1.0f - roundness;
   s.squeeze = std::isfinite(c->cam.squeeze) ? std::max(0.01f, c->cam.squeeze) : 1.0f;
   s.stack_required = c->wide.stack_required;
-  s.reference_tree = c->wide.reference_topology ? 1u : 0u;
   s.watertight = c->config.triangle_test == VKPTC_TRIANGLE_WATERTIGHT ? 1u : 0u;
   s.sdf = c->sdf_count ? c->d_sdf.ptr : nullptr;
   s.sdf_count = c->sdf_count;
@@ -341,8 +340,8 @@ int stack_cap(const vkptc_ctx* c) {
   return static_cast<int>(std::max<uint32_t>(1u, c->wide.stack_required));
 }
 
-constexpr int kDefaultSmemEntries = 16;
-constexpr int kDefaultSteps = 4;
+constexpr int kDefaultSmemEntries = 12;
+constexpr int kDefaultSteps = 8;
 
 int32_t ensure_stack_smem(vkptc_ctx* c, const LaunchShape& ls);
 

@@ -36,6 +36,8 @@ size_t SpillEntries(const LaunchShape& ls) {
 // Each source supplies queries to persistent_traverse() and consumes results.
 struct RaysSource {   // batched ray queries from a ray array
   GeoView geo;
+  static constexpr bool kUniform = true;
+  __device__ __forceinline__ const GeoView& geo_at(uint32_t) const { return geo; }
   const float* rays;
   const float* tmax;
   uint32_t* prim_out;
@@ -57,6 +59,8 @@ struct RaysSource {   // batched ray queries from a ray array
 
 struct ExtendSource {  // closest hit for the queued paths of a wave
   GeoView geo;
+  static constexpr bool kUniform = true;
+  __device__ __forceinline__ const GeoView& geo_at(uint32_t) const { return geo; }
   const uint32_t* q;
   const float4* ray_o;
   const float4* ray_d;
@@ -76,6 +80,8 @@ struct ExtendSource {  // closest hit for the queued paths of a wave
 
 struct ShadowSource {  // any hit for the NEE queries; adds the term when visible
   GeoView geo;
+  static constexpr bool kUniform = true;
+  __device__ __forceinline__ const GeoView& geo_at(uint32_t) const { return geo; }
   const float4* sh_o;
   const float4* sh_d;
   const float4* sh_c;
@@ -122,9 +128,13 @@ __device__ __forceinline__ void run_persistent(const Src& src, uint32_t n, uint3
   if (lerr) atomicOr(err, lerr);
 }
 
+// The traversal kernels run at 64 registers (at least 1024 threads per SM):
+// they wait on node and triangle loads more than on anything else, and at 74
+// registers (24 warps per SM instead of 32) a full-HD frame of the 2M-triangle
+// grid took 37.2 ms instead of 30.7.
 // =============================================================== ray queries
 template <bool kAny, bool kStats, bool kWt>
-__global__ void __launch_bounds__(256) k_trace_rays(DevScene s, RaysSource src, uint32_t n, uint32_t* fetch, int scap,
+__global__ void __launch_bounds__(256, 4) k_trace_rays(DevScene s, RaysSource src, uint32_t n, uint32_t* fetch, int scap,
                                                     int2* spill, int total, int steps, DevCounters* ctr, uint32_t* err) {
   run_persistent<RaysSource, kAny, kStats, kWt>(src, n, fetch, scap, spill, total, steps, &ctr->nodes, &ctr->leaves,
                                                 &ctr->tris, &ctr->ext_rays, err);
@@ -187,7 +197,7 @@ __global__ void __launch_bounds__(256) k_raygen(DevScene s, DevSettings st, Wave
 // Closest-hit traversal of the current extension queue (persistent warps).
 // Zeroes the next queue's and the shadow queue's sizes for the shade stage.
 template <bool kStats, bool kWt>
-__global__ void __launch_bounds__(256) k_extend(DevScene s, WaveState w, uint32_t cur, int scap, int2* spill,
+__global__ void __launch_bounds__(256, 4) k_extend(DevScene s, WaveState w, uint32_t cur, int scap, int2* spill,
                                                 int total, int steps, DevCounters* ctr, uint32_t* err) {
   const uint32_t n = w.counts[cur];
   if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -278,7 +288,7 @@ __global__ void __launch_bounds__(256, 3) k_shade(DevScene s, DevSettings st, Wa
 // Any-hit visibility of the NEE queries (persistent warps); adds the NEE term
 // of every visible query to its path's radiance.
 template <bool kStats, bool kWt>
-__global__ void __launch_bounds__(256) k_shadow(DevScene s, WaveState w, int scap, int2* spill, int total, int steps,
+__global__ void __launch_bounds__(256, 4) k_shadow(DevScene s, WaveState w, int scap, int2* spill, int total, int steps,
                                                 DevCounters* ctr, uint32_t* err) {
   const uint32_t n = w.counts[2];
   const ShadowSource src{geo_of(s), w.sh_o, w.sh_d, w.sh_c, w.sh_path, w.rad};
@@ -291,7 +301,7 @@ __global__ void __launch_bounds__(256) k_shadow(DevScene s, WaveState w, int sca
 template <bool kStats, bool kWt>
 __global__ void __launch_bounds__(256) k_shadow_transmissive(DevScene s, WaveState w, int cap, DevCounters* ctr, uint32_t* err) {
   extern __shared__ int2 smem_stack[];
-  SmemStack stk{smem_stack + threadIdx.x, static_cast<int>(blockDim.x), cap};
+  const TwoLevelStack stk = smem_stack_of(smem_stack + threadIdx.x, static_cast<int>(blockDim.x), cap);
   const uint32_t n = w.counts[2];
   uint32_t local_err = 0u;
   for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
@@ -305,16 +315,14 @@ __global__ void __launch_bounds__(256) k_shadow_transmissive(DevScene s, WaveSta
       float remain = o4.w;
       bool visible = true;
       if (!s.has_transmissive) {
-        const RayPrep r = prep_ray(so, sd, s.reference_tree != 0u, kWt);
-        visible = !trace_any<kStats, kWt>(s, r, remain, stk, st, local_err);
+        visible = !trace_any<kStats, kWt>(s, so, sd, remain, stk, st, local_err);
       } else {
         // Closest-hit loop that steps through up to 8 transmissive occluders
         // (src/pathtracer/ScalarCpuPathTracer.cpp:1067-1087).
         for (uint32_t skips = 0; skips < 8u && remain > 0.004f; ++skips) {
-          const RayPrep r = prep_ray(so, sd, s.reference_tree != 0u, kWt);
           float t;
           uint32_t prim;
-          trace_closest<kStats, kWt>(s, r, stk, t, prim, st, local_err);
+          trace_closest<kStats, kWt>(s, so, sd, stk, t, prim, st, local_err);
           if (s.sdf_count != 0u) sdf_closest(s.sdf, s.sdf_count, so, sd, t, prim, sdf_n);
           if (prim == kMiss || t >= remain) break;
           const uint32_t mat_index = (prim & kSdfTag) ? sdf_material(s.sdf, prim & ~kSdfTag)
