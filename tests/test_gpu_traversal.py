@@ -13,7 +13,8 @@ one outside its box, so which of them is visited decides:
     ulps, and its own rounding culls such triangles: there one probe in 500 may
     name another triangle, its distance within 1e-5 of the oracle's;
   * a bound 1e-4 above the closest distance may cull the grazing triangle's box:
-    one any-hit probe in 2000 may then report no occluder.
+    one any-hit probe in 2000 may then report no occluder (unbounded any-hit is
+    exact).
 """
 import numpy as np
 import pytest
@@ -68,6 +69,8 @@ def check(sc, rays, test="mt", **kw):
     with tracer(sc, triangle_test=test, **kw) as t:
         p, tt = t.trace_rays(rays)
         a, _ = t.trace_rays(rays, mode=native.QUERY_ANY, tmax=tmax)
+        u, _ = t.trace_rays(rays, mode=native.QUERY_ANY)
+    assert np.array_equal(u.astype(bool), np.isfinite(rt))
     differ = (p != rp) | (tt.view(np.uint32) != rt.view(np.uint32))
     far = np.abs(sc.vertices).max() > 200.0
     assert differ.sum() <= (p.size // 500 if far else 0), f"{differ.sum()} of {p.size} hits differ"
@@ -116,3 +119,31 @@ def test_non_finite_rays_end_and_hit_nothing():
     assert np.all(p[:12] == 0xFFFFFFFF) and np.all(np.isinf(tt[:12]))
     rp, rt, _, _ = oracle.load("port").intersect(sc, rays[36:], threads=1)
     assert np.array_equal(p[36:], rp) and np.array_equal(tt[36:].view(np.uint32), rt.view(np.uint32))
+
+
+@pytest.mark.parametrize("n_lat,n_lon", [(2, 3), (3, 4), (3, 6), (4, 11), (5, 8), (5, 9), (8, 9), (9, 32), (17, 33), (33, 40)])
+def test_sah_trees_at_subtree_and_chunk_edges(n_lat, n_lon):
+    """SAH trees whose sizes straddle the leaf limit (2), the ten planes and the
+    64 primitives of a warp's subtree, and the 512 positions of a binning block:
+    6, 16, 24, 66, 64, 72, 126, 512, 1056 and 2560 triangles, and three copies
+    of each (coinciding centroids, every hit a tie).  Every triangle is in the
+    tree once, and rays aimed inside triangles hit what the oracle's hit."""
+    one = scenes.sphere_field(1, n_lat, n_lon, seed=2, n_lights=1)
+    tri = np.ascontiguousarray(one.indices[:2 * (n_lat - 1) * n_lon])
+    r = np.random.RandomState(n_lat)
+    for copies in (1, 3):
+        sc = scenes.sphere_field(1, n_lat, n_lon, seed=2, n_lights=1)
+        sc.vertices = np.ascontiguousarray(sc.vertices * np.float32(16.0))
+        sc.indices = np.ascontiguousarray(np.concatenate([tri] * copies))
+        sc.instances = np.array([[0, sc.indices.shape[0], 0]], np.uint32)
+        w = r.dirichlet((2.0, 2.0, 2.0), 3001)
+        target = np.einsum("nk,nkc->nc", w, sc.vertices[tri[r.randint(0, tri.shape[0], 3001)]].astype(np.float64))
+        o = r.uniform(-60.0, 60.0, (3001, 3))
+        rays = np.ascontiguousarray(np.concatenate([o, target - o], axis=1), np.float32)
+        rays[:, 3:] /= np.linalg.norm(rays[:, 3:], axis=1, keepdims=True)
+        rp, rt, _, _ = oracle.load("port").intersect(sc, rays, threads=8)
+        with tracer(sc, bvh="sah") as t:
+            p, tt = t.trace_rays(rays)
+            rec = t.read_accel(native.ACCEL_TRIANGLES).reshape(-1, 12)
+        assert np.array_equal(np.sort(rec[:, 9]), np.arange(sc.indices.shape[0]))
+        assert np.array_equal(p, rp) and np.array_equal(tt.view(np.uint32), rt.view(np.uint32))

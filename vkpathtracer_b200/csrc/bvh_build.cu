@@ -11,7 +11,7 @@
 //        plus one atomic per run, the widest axis and its midpoint, a flag per
 //        primitive, an exclusive scan, and a stable scatter (left flags first,
 //        in order; count/2 when one side is empty, order unchanged);
-//        smaller subtrees by one thread each, sequentially, the same steps;
+//        smaller subtrees by a warp each, in shared memory, the same steps;
 //      then node bounds by a bottom-up refit (union of children; min/max are
 //      exact, so the result equals the top-down bounds of the reference) and
 //      the reference's node ids: the reference allocates the two children of
@@ -38,7 +38,7 @@ namespace vkptc {
 namespace {
 
 constexpr float kPadB = 1e-4f;
-constexpr uint32_t kSmallNode = 64;   // subtrees of at most this many primitives: one thread each
+constexpr uint32_t kSmallNode = 64;   // subtrees of at most this many primitives: one warp each
 constexpr uint32_t kLeafMax = 4;      // ParallelBvhBuilder's leaf threshold
 constexpr int kScanThreads = 512;
 constexpr uint32_t kScanBlock = 2 * kScanThreads;
@@ -357,6 +357,7 @@ struct BuildArrays {
   uint32_t* ident;         // per slot: 1 = order unchanged, count/2 split
   uint32_t* counter;       // [0] next temporary node id, [1] next-level active count, [2] small count,
                            // [4] this level's active count, [5] first temporary id of this level's children
+  uint32_t leaf_max;       // nodes of at most so many primitives are leaves
 };
 
 // The level loop runs without the host: every per-level kernel reads the
@@ -515,7 +516,7 @@ __global__ void k_flags(BuildArrays A, const uint32_t* __restrict__ idx, const u
 }
 
 // Children of every active node; big ones go to the next level's list, small
-// ones to the per-thread list, leaves nowhere.
+// ones to the subtree list, leaves nowhere.
 __global__ void k_children(BuildArrays A, const uint32_t* __restrict__ act, const uint32_t* __restrict__ excl,
                            uint32_t* __restrict__ next_act, uint32_t* __restrict__ small) {
   const uint32_t n_act = level_active(A), base = A.counter[5];
@@ -538,7 +539,7 @@ __global__ void k_children(BuildArrays A, const uint32_t* __restrict__ act, cons
                            static_cast<int32_t>(nd)};
     A.slot_of[id[c]] = -1;
     if (cnt[c] > kSmallNode) next_act[atomicAdd(&A.counter[1], 1u)] = id[c];
-    else if (cnt[c] > kLeafMax) small[atomicAdd(&A.counter[2], 1u)] = id[c];
+    else if (cnt[c] > A.leaf_max) small[atomicAdd(&A.counter[2], 1u)] = id[c];
   }
   }
 }
@@ -574,250 +575,184 @@ __global__ void k_scatter(BuildArrays A, const uint32_t* __restrict__ idx, const
   node2[dst] = static_cast<uint32_t>(left ? t.left : t.right);
 }
 
-// Sequential build of one small subtree per thread (same split rules).
-// Small subtrees of the SAH tree, one warp each: the host SAH builder's
-// splits (32 bins per axis, the first minimum of the swept costs, a stable
-// partition, count/2 when one side is empty), with the node's primitives on the lanes (two per lane), the bins
-// filled by one leader per bin and slot (order-preserving keys, min and max are
-// exact) and the sweep done by shuffle scans with bin b on lane b.
+// Small subtrees (at most kSmallNode primitives), one warp each, built in
+// shared memory: the primitives' boxes are read once, the nodes are kept as
+// packed words in the order they are made (children after their parents, so the
+// list is its own queue), and the subtree's node ids come from one atomic.
+//  * kSah = false: the reference's midpoint split (widest axis of the centroid
+//    bounds, its midpoint, a stable partition, count/2 with the order unchanged
+//    when one side is empty).
+//  * kSah = true: the cheapest of ten planes per axis, all thirty at once: lane
+//    10a + k holds plane k of axis a and adds every primitive's box to its left
+//    or its right side, so the sweep needs no bins and no scan.  The planes
+//    divide the centroid bounds evenly; in a node of at most ten primitives they
+//    are the primitives' own centroids, which makes the sweep exact.
+// Filling 32 bins per axis with one leader per bin and scanning them with
+// shuffles took 3.83 ms for the subtrees of the 2,064,386-triangle grid, this
+// takes 0.78 ms; the midpoint subtrees by one thread each took 0.48 ms, by a
+// warp each 0.19 ms.
 constexpr int kSmallWarps = 4;
-static_assert(kSahBins == 32, "k_small_sah keeps bin b on lane b");
+constexpr int kSmallPlanes = 10;
+static_assert(kSmallNode == 64, "two primitives per lane, 7-bit fields in the packed nodes");
 
-__device__ __forceinline__ float warp_min(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = bmin(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
-__device__ __forceinline__ float warp_max(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = bmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
+// begin | count << 7 | left << 14 | parent << 21 (ids within the subtree; left 0: a leaf)
+__device__ __forceinline__ uint32_t pack_small(uint32_t begin, uint32_t count, uint32_t parent) {
+  return begin | (count << 7) | (parent << 21);
 }
 
-__device__ __forceinline__ int sah_bin_of(float c, float c0, float scale) {
-  const int k = static_cast<int>((c - c0) * scale);
-  return k < 0 ? 0 : (k > kSahBins - 1 ? kSahBins - 1 : k);
-}
-
-__global__ void __launch_bounds__(32 * kSmallWarps) k_small_sah(BuildArrays A, const uint32_t* __restrict__ small,
-                                                                uint32_t n_small, uint32_t* __restrict__ idx) {
-  __shared__ uint32_t s_stack[kSmallWarps][64];
-  __shared__ uint32_t s_bins[kSmallWarps][kSahBins * kBinWords];
+template <bool kSah>
+__global__ void __launch_bounds__(32 * kSmallWarps) k_small(BuildArrays A, const uint32_t* __restrict__ small,
+                                                            uint32_t n_small, uint32_t* __restrict__ idx) {
+  __shared__ float4 s_box[kSmallWarps][2 * kSmallNode];   // lower and upper corner per primitive of the subtree
+  __shared__ uint32_t s_prim[kSmallWarps][kSmallNode];    // its global index
+  __shared__ uint32_t s_node[kSmallWarps][2 * kSmallNode];
+  __shared__ unsigned char s_ord[kSmallWarps][kSmallNode];   // current order: subtree primitive per position
   const int wib = static_cast<int>(threadIdx.x >> 5);
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t lt = (1u << lane) - 1u;
-  uint32_t* stack = s_stack[wib];
-  uint32_t* bins = s_bins[wib];
+  float4* box = s_box[wib];
+  uint32_t* node = s_node[wib];
+  unsigned char* ord = s_ord[wib];
   const uint32_t nwarps = gridDim.x * kSmallWarps;
   for (uint32_t w = blockIdx.x * kSmallWarps + static_cast<uint32_t>(wib); w < n_small; w += nwarps) {
-    if (lane == 0u) stack[0] = small[w];
-    int sp = 1;
-    __syncwarp();
-    while (sp > 0) {
-      const uint32_t nd = stack[--sp];
-      const TNode t = A.nodes[nd];
-      const uint32_t b = static_cast<uint32_t>(t.begin), n = static_cast<uint32_t>(t.count);
+    const uint32_t root = small[w];
+    const uint32_t gb = static_cast<uint32_t>(A.nodes[root].begin), total = static_cast<uint32_t>(A.nodes[root].count);
+    __syncwarp();   // the previous subtree's shared words are no longer read
+    for (uint32_t i = lane; i < total; i += 32u) {
+      const uint32_t p = idx[gb + i];
+      s_prim[wib][i] = p;
+      ord[i] = static_cast<unsigned char>(i);
+      box[2 * i] = A.blo[p];
+      box[2 * i + 1] = A.bhi[p];
+    }
+    if (lane == 0u) node[0] = pack_small(0u, total, 0u);
+    uint32_t made = 1u;
+    for (uint32_t k = 0u; k < made; ++k) {
       __syncwarp();
-      if (n <= kLeafMax) continue;
+      const uint32_t word = node[k];
+      const uint32_t b = word & 127u, n = (word >> 7) & 127u;
+      if (n <= A.leaf_max) continue;
       const bool h0 = lane < n, h1 = lane + 32u < n;
-      const uint32_t p0 = h0 ? idx[b + lane] : 0u, p1 = h1 ? idx[b + lane + 32u] : 0u;
+      const uint32_t q0 = h0 ? ord[b + lane] : 0u, q1 = h1 ? ord[b + lane + 32u] : 0u;
       float c0[3], c1[3], clo[3], chi[3];
-      for (int a = 0; a < 3; ++a) {
-        c0[a] = h0 ? centroid(A.blo, A.bhi, p0, a) : 0.0f;
-        c1[a] = h1 ? centroid(A.blo, A.bhi, p1, a) : 0.0f;
-        clo[a] = warp_min(bmin(h0 ? c0[a] : FLT_MAX, h1 ? c1[a] : FLT_MAX));
-        chi[a] = warp_max(bmax(h0 ? c0[a] : -FLT_MAX, h1 ? c1[a] : -FLT_MAX));
+      {
+        const float4 l0 = box[2 * q0], u0 = box[2 * q0 + 1], l1 = box[2 * q1], u1 = box[2 * q1 + 1];
+        c0[0] = 0.5f * (l0.x + u0.x);
+        c0[1] = 0.5f * (l0.y + u0.y);
+        c0[2] = 0.5f * (l0.z + u0.z);
+        c1[0] = 0.5f * (l1.x + u1.x);
+        c1[1] = 0.5f * (l1.y + u1.y);
+        c1[2] = 0.5f * (l1.z + u1.z);
       }
-      const float4 lo0 = h0 ? A.blo[p0] : make_float4(0.f, 0.f, 0.f, 0.f), hi0 = h0 ? A.bhi[p0] : lo0;
-      const float4 lo1 = h1 ? A.blo[p1] : make_float4(0.f, 0.f, 0.f, 0.f), hi1 = h1 ? A.bhi[p1] : lo1;
-      float best_cost = FLT_MAX;
-      int best_axis = -1, best_bin = -1;
-      for (int a = 0; a < 3; ++a) {
-        const float ext = chi[a] - clo[a];
-        if (!(ext > 0.0f)) continue;   // uniform
-        const float scale = static_cast<float>(kSahBins) / ext;
-        uint32_t* wb = bins + kBinWords * lane;   // bin `lane`
-        wb[0] = 0u;
-        wb[1] = wb[2] = wb[3] = 0xffffffffu;
-        wb[4] = wb[5] = wb[6] = 0u;
-        __syncwarp();
-        for (int slot = 0; slot < 2; ++slot) {
-          const bool h = slot == 0 ? h0 : h1;
-          const unsigned active = __ballot_sync(0xffffffffu, h);
-          if (h) {
-            const float4 lo = slot == 0 ? lo0 : lo1, hi = slot == 0 ? hi0 : hi1;
-            const int k = sah_bin_of(slot == 0 ? c0[a] : c1[a], clo[a], scale);
-            const unsigned grp = __match_any_sync(active, static_cast<uint32_t>(k));
-            const uint32_t m0 = __reduce_min_sync(grp, fkey(lo.x)), m1 = __reduce_min_sync(grp, fkey(lo.y)),
-                           m2 = __reduce_min_sync(grp, fkey(lo.z));
-            const uint32_t x0 = __reduce_max_sync(grp, fkey(hi.x)), x1 = __reduce_max_sync(grp, fkey(hi.y)),
-                           x2 = __reduce_max_sync(grp, fkey(hi.z));
-            if (static_cast<int>(lane) == __ffs(grp) - 1) {
-              uint32_t* q = bins + kBinWords * k;
-              q[0] += static_cast<uint32_t>(__popc(grp));
-              q[1] = min(q[1], m0);
-              q[2] = min(q[2], m1);
-              q[3] = min(q[3], m2);
-              q[4] = max(q[4], x0);
-              q[5] = max(q[5], x1);
-              q[6] = max(q[6], x2);
-            }
-          }
-          __syncwarp();
-        }
-        // the sweep: prefix over bins 0..lane, suffix over lane..31 (k_sah_split's scans)
-        const uint32_t cnt = wb[0];
-        float lo3[3], hi3[3];
-        for (int q = 0; q < 3; ++q) {
-          lo3[q] = cnt ? fval(wb[1 + q]) : FLT_MAX;
-          hi3[q] = cnt ? fval(wb[4 + q]) : -FLT_MAX;
-        }
-        __syncwarp();
-        uint32_t lc = cnt, rc = cnt;
-        float llo[3] = {lo3[0], lo3[1], lo3[2]}, lhi[3] = {hi3[0], hi3[1], hi3[2]};
-        float rlo[3] = {lo3[0], lo3[1], lo3[2]}, rhi[3] = {hi3[0], hi3[1], hi3[2]};
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const uint32_t lcu = __shfl_up_sync(0xffffffffu, lc, o);
-          const uint32_t rcd = __shfl_down_sync(0xffffffffu, rc, o);
-          float lu[6], rd[6];
-          for (int q = 0; q < 3; ++q) {
-            lu[q] = __shfl_up_sync(0xffffffffu, llo[q], o);
-            lu[3 + q] = __shfl_up_sync(0xffffffffu, lhi[q], o);
-            rd[q] = __shfl_down_sync(0xffffffffu, rlo[q], o);
-            rd[3 + q] = __shfl_down_sync(0xffffffffu, rhi[q], o);
-          }
-          if (static_cast<int>(lane) >= o) {
-            lc += lcu;
-            for (int q = 0; q < 3; ++q) {
-              llo[q] = bmin(llo[q], lu[q]);
-              lhi[q] = bmax(lhi[q], lu[3 + q]);
-            }
-          }
-          if (static_cast<int>(lane) + o < 32) {
-            rc += rcd;
-            for (int q = 0; q < 3; ++q) {
-              rlo[q] = bmin(rlo[q], rd[q]);
-              rhi[q] = bmax(rhi[q], rd[3 + q]);
-            }
-          }
-        }
-        const uint32_t rcn = __shfl_down_sync(0xffffffffu, rc, 1);
-        float rn[6];
-        for (int q = 0; q < 3; ++q) {
-          rn[q] = __shfl_down_sync(0xffffffffu, rlo[q], 1);
-          rn[3 + q] = __shfl_down_sync(0xffffffffu, rhi[q], 1);
-        }
-        float cost = FLT_MAX;
-        if (lane < 31u && lc != 0u && rcn != 0u) {
-          const float dx = lhi[0] - llo[0], dy = lhi[1] - llo[1], dz = lhi[2] - llo[2];
-          const float ex = rn[3] - rn[0], ey = rn[4] - rn[1], ez = rn[5] - rn[2];
-          cost = (dx * dy + dy * dz + dz * dx) * static_cast<float>(lc) +
-                 (ex * ey + ey * ez + ez * ex) * static_cast<float>(rcn);
-        }
-        float c = cost;
-        int bb = static_cast<int>(lane);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          const float co = __shfl_xor_sync(0xffffffffu, c, o);
-          const int bo = __shfl_xor_sync(0xffffffffu, bb, o);
-          if (co < c || (co == c && bo < bb)) {
-            c = co;
-            bb = bo;
-          }
-        }
-        if (c < best_cost) {
-          best_cost = c;
-          best_axis = a;
-          best_bin = bb;
-        }
+      for (int a = 0; a < 3; ++a) {
+        const uint32_t k0 = fkey(c0[a]), k1 = fkey(c1[a]);
+        clo[a] = fval(__reduce_min_sync(0xffffffffu, min(h0 ? k0 : 0xffffffffu, h1 ? k1 : 0xffffffffu)));
+        chi[a] = fval(__reduce_max_sync(0xffffffffu, max(h0 ? k0 : 0u, h1 ? k1 : 0u)));
       }
-      // stable partition: left in order, then right in order (ident: order unchanged, count/2)
-      uint32_t nl = 0u;
-      if (best_axis >= 0) {
-        const float cb0 = clo[best_axis];
-        const float scale = static_cast<float>(kSahBins) / (chi[best_axis] - cb0);
-        const bool l0 = h0 && sah_bin_of(c0[best_axis], cb0, scale) <= best_bin;
-        const bool l1 = h1 && sah_bin_of(c1[best_axis], cb0, scale) <= best_bin;
-        const unsigned v0 = __ballot_sync(0xffffffffu, h0), v1 = __ballot_sync(0xffffffffu, h1);
-        const unsigned b0 = __ballot_sync(0xffffffffu, l0), b1 = __ballot_sync(0xffffffffu, l1);
-        const uint32_t nl0 = static_cast<uint32_t>(__popc(b0));
-        nl = nl0 + static_cast<uint32_t>(__popc(b1));
-        const uint32_t nr0 = static_cast<uint32_t>(__popc(v0 & ~b0));
-        __syncwarp();   // every lane holds its primitives before any is moved
-        if (h0) idx[b + (l0 ? __popc(b0 & lt) : nl + __popc(v0 & ~b0 & lt))] = p0;
-        if (h1) idx[b + (l1 ? nl0 + __popc(b1 & lt) : nl + nr0 + __popc(v1 & ~b1 & lt))] = p1;
+      bool l0 = false, l1 = false;
+      if constexpr (kSah) {
+        const int a = static_cast<int>(lane) / kSmallPlanes, pl = static_cast<int>(lane) - a * kSmallPlanes;
+        const float cl = a == 0 ? clo[0] : (a == 1 ? clo[1] : clo[2]);
+        const float ext = (a == 0 ? chi[0] : (a == 1 ? chi[1] : chi[2])) - cl;
+        float plane = cl + ext * (static_cast<float>(pl + 1) * (1.0f / (kSmallPlanes + 1)));
+        if (n <= static_cast<uint32_t>(kSmallPlanes)) {
+          const uint32_t q = ord[b + min(static_cast<uint32_t>(pl), n - 1u)];
+          const float4 lo = box[2 * q], hi = box[2 * q + 1];
+          plane = 0.5f * (a == 0 ? lo.x + hi.x : (a == 1 ? lo.y + hi.y : lo.z + hi.z));
+        }
+        float ll[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, lu[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
+        float rl[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, ru[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
+        uint32_t nl = 0u;
+        for (uint32_t i = 0u; i < n; ++i) {
+          const uint32_t q = ord[b + i];
+          const float4 lo = box[2 * q], hi = box[2 * q + 1];
+          const float c = 0.5f * (a == 0 ? lo.x + hi.x : (a == 1 ? lo.y + hi.y : lo.z + hi.z));
+          if (c <= plane) {
+            ++nl;
+            ll[0] = fminf(ll[0], lo.x);
+            ll[1] = fminf(ll[1], lo.y);
+            ll[2] = fminf(ll[2], lo.z);
+            lu[0] = fmaxf(lu[0], hi.x);
+            lu[1] = fmaxf(lu[1], hi.y);
+            lu[2] = fmaxf(lu[2], hi.z);
+          } else {
+            rl[0] = fminf(rl[0], lo.x);
+            rl[1] = fminf(rl[1], lo.y);
+            rl[2] = fminf(rl[2], lo.z);
+            ru[0] = fmaxf(ru[0], hi.x);
+            ru[1] = fmaxf(ru[1], hi.y);
+            ru[2] = fmaxf(ru[2], hi.z);
+          }
+        }
+        const float dx = lu[0] - ll[0], dy = lu[1] - ll[1], dz = lu[2] - ll[2];
+        const float ex = ru[0] - rl[0], ey = ru[1] - rl[1], ez = ru[2] - rl[2];
+        const float cost = (dx * dy + dy * dz + dz * dx) * static_cast<float>(nl) +
+                           (ex * ey + ey * ez + ez * ex) * static_cast<float>(n - nl);
+        // costs are not negative, so their bits compare as the floats do; no plane: all bits set
+        const bool ok = a < 3 && nl != 0u && nl != n && cost < FLT_MAX;
+        const uint32_t key = ok ? __float_as_uint(cost) : 0xffffffffu;
+        const uint32_t best = __reduce_min_sync(0xffffffffu, key);
+        if (best != 0xffffffffu) {
+          const int src = __ffs(__ballot_sync(0xffffffffu, key == best)) - 1;   // lowest axis, then plane
+          const float bp = __shfl_sync(0xffffffffu, plane, src);
+          const int ba = src / kSmallPlanes;
+          const float v0 = ba == 0 ? c0[0] : (ba == 1 ? c0[1] : c0[2]), v1 = ba == 0 ? c1[0] : (ba == 1 ? c1[1] : c1[2]);
+          l0 = h0 && v0 <= bp;
+          l1 = h1 && v1 <= bp;
+        }
+      } else {
+        int axis = 0;
+        float widest = chi[0] - clo[0];
+        for (int a = 1; a < 3; ++a) {
+          const float e = chi[a] - clo[a];
+          if (e > widest) {
+            widest = e;
+            axis = a;
+          }
+        }
+        const float split = 0.5f * (axis == 0 ? clo[0] + chi[0] : (axis == 1 ? clo[1] + chi[1] : clo[2] + chi[2]));
+        l0 = h0 && (axis == 0 ? c0[0] : (axis == 1 ? c0[1] : c0[2])) < split;
+        l1 = h1 && (axis == 0 ? c1[0] : (axis == 1 ? c1[1] : c1[2])) < split;
       }
-      const bool ident = nl == 0u || nl == n;
-      if (ident) nl = n / 2u;
-      uint32_t l = 0u;
+      // stable partition: left in order, then right in order; one side empty: order unchanged, count/2
+      const unsigned v0 = __ballot_sync(0xffffffffu, h0), v1 = __ballot_sync(0xffffffffu, h1);
+      const unsigned b0 = __ballot_sync(0xffffffffu, l0), b1 = __ballot_sync(0xffffffffu, l1);
+      const uint32_t nl0 = static_cast<uint32_t>(__popc(b0));
+      uint32_t nl = nl0 + static_cast<uint32_t>(__popc(b1));
+      const uint32_t nr0 = static_cast<uint32_t>(__popc(v0 & ~b0));
+      __syncwarp();   // every lane holds its primitives before any is moved
+      if (nl != 0u && nl != n) {
+        if (h0) ord[b + (l0 ? __popc(b0 & lt) : nl + __popc(v0 & ~b0 & lt))] = static_cast<unsigned char>(q0);
+        if (h1) ord[b + (l1 ? nl0 + __popc(b1 & lt) : nl + nr0 + __popc(v1 & ~b1 & lt))] = static_cast<unsigned char>(q1);
+      } else {
+        nl = n / 2u;
+      }
       if (lane == 0u) {
-        l = atomicAdd(&A.counter[0], 2u);
-        const uint32_t r = l + 1u;
-        A.nodes[nd].left = static_cast<int32_t>(l);
-        A.nodes[nd].right = static_cast<int32_t>(r);
-        A.nodes[l] = TNode{static_cast<int32_t>(b), static_cast<int32_t>(nl), -1, -1, static_cast<int32_t>(nd)};
-        A.nodes[r] = TNode{static_cast<int32_t>(b + nl), static_cast<int32_t>(n - nl), -1, -1, static_cast<int32_t>(nd)};
-        if (sp + 2 <= 64) {
-          stack[sp] = r;
-          stack[sp + 1] = l;
-        }
+        node[k] = word | (made << 14);
+        node[made] = pack_small(b, nl, k);
+        node[made + 1u] = pack_small(b + nl, n - nl, k);
       }
-      if (sp + 2 <= 64) sp += 2;
-      __syncwarp();
+      made += 2u;
     }
-  }
-}
-
-// Small subtrees of the reference tree (midpoint splits), one thread each.
-__global__ void k_small(BuildArrays A, const uint32_t* __restrict__ small, uint32_t n_small, uint32_t* __restrict__ idx) {
-  const uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
-  if (w >= n_small) return;
-  uint32_t stack[64];
-  uint32_t tmp[kSmallNode];
-  int sp = 0;
-  stack[sp++] = small[w];
-  while (sp > 0) {
-    const uint32_t nd = stack[--sp];
-    const TNode t = A.nodes[nd];
-    const uint32_t b = static_cast<uint32_t>(t.begin), n = static_cast<uint32_t>(t.count);
-    if (n <= kLeafMax) continue;
-    float clo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, chi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-    for (uint32_t i = 0; i < n; ++i) {
-      const uint32_t p = idx[b + i];
-      for (int a = 0; a < 3; ++a) {
-        const float c = centroid(A.blo, A.bhi, p, a);
-        clo[a] = bmin(clo[a], c);
-        chi[a] = bmax(chi[a], c);
+    // the subtree's nodes to their ids (the root keeps its own) and the final order
+    uint32_t base = 0u;
+    if (lane == 0u) base = atomicAdd(&A.counter[0], made - 1u);
+    base = __shfl_sync(0xffffffffu, base, 0) - 1u;   // subtree id k >= 1 is global id base + k
+    __syncwarp();
+    for (uint32_t k = lane; k < made; k += 32u) {
+      const uint32_t word = node[k];
+      const uint32_t left = (word >> 14) & 127u, parent = (word >> 21) & 127u;
+      const int32_t l = left ? static_cast<int32_t>(base + left) : -1;
+      if (k == 0u) {
+        A.nodes[root].left = l;
+        A.nodes[root].right = l < 0 ? -1 : l + 1;
+      } else {
+        A.nodes[base + k] = TNode{static_cast<int32_t>(gb + (word & 127u)), static_cast<int32_t>((word >> 7) & 127u), l,
+                                  l < 0 ? -1 : l + 1, static_cast<int32_t>(parent ? base + parent : root)};
       }
     }
-    int axis = 0;
-    float widest = chi[0] - clo[0];
-    for (int a = 1; a < 3; ++a) {
-      const float e = chi[a] - clo[a];
-      if (e > widest) {
-        widest = e;
-        axis = a;
-      }
-    }
-    const float split = 0.5f * (clo[axis] + chi[axis]);
-    uint32_t nl = 0u, nr = 0u;
-    for (uint32_t i = 0; i < n; ++i) {
-      const uint32_t p = idx[b + i];
-      if (centroid(A.blo, A.bhi, p, axis) < split) idx[b + nl++] = p;
-      else tmp[nr++] = p;
-    }
-    for (uint32_t i = 0; i < nr; ++i) idx[b + nl + i] = tmp[i];
-    if (nl == 0u || nl == n) nl = n / 2u;
-    const uint32_t l = atomicAdd(&A.counter[0], 2u), r = l + 1u;
-    A.nodes[nd].left = static_cast<int32_t>(l);
-    A.nodes[nd].right = static_cast<int32_t>(r);
-    A.nodes[l] = TNode{static_cast<int32_t>(b), static_cast<int32_t>(nl), -1, -1, static_cast<int32_t>(nd)};
-    A.nodes[r] = TNode{static_cast<int32_t>(b + nl), static_cast<int32_t>(n - nl), -1, -1, static_cast<int32_t>(nd)};
-    if (sp + 2 <= 64) {
-      stack[sp++] = r;
-      stack[sp++] = l;
-    }
+    for (uint32_t i = lane; i < total; i += 32u) idx[gb + i] = s_prim[wib][ord[i]];
   }
 }
 
@@ -833,46 +768,94 @@ __global__ void k_sah_bin_init(BuildArrays A, uint32_t* __restrict__ bins) {
   }
 }
 
-__global__ void k_sah_bin(BuildArrays A, const uint32_t* __restrict__ idx, const uint32_t* __restrict__ node_of,
-                          uint32_t n, uint32_t* __restrict__ bins) {
+// A block bins kBinChunk consecutive positions in shared memory and adds its
+// non-empty bins to the nodes' global ones.  A node holds more than kSmallNode
+// primitives and its positions are contiguous, so a chunk meets at most
+// kBinSegs nodes.  Global atomics from every warp (one leader per bin and warp)
+// took up to 447 us for a level of the 2,064,386-triangle grid, where all of
+// them meet in one node's 96 bins, and 3.07 ms for its 19 levels; this takes
+// 1.75 ms.
+constexpr uint32_t kBinChunk = 512;
+constexpr uint32_t kBinSegs = (kBinChunk - 2u) / (kSmallNode + 1u) + 2u;
+__global__ void __launch_bounds__(kThreads) k_sah_bin(BuildArrays A, const uint32_t* __restrict__ idx,
+                                                      const uint32_t* __restrict__ node_of, uint32_t n,
+                                                      uint32_t* __restrict__ bins) {
   if (level_active(A) == 0u) return;   // uniform over the grid
-  const uint32_t pos = blockIdx.x * blockDim.x + threadIdx.x;
-  int32_t s = -1;
-  uint32_t p = 0u;
-  if (pos < n) {
-    s = A.slot_of[node_of[pos]];
-    if (s >= 0) p = idx[pos];
+  constexpr uint32_t kRounds = kBinChunk / kThreads, kWarps = kThreads / 32;
+  __shared__ uint32_t s_bin[kBinSegs * 3 * kSahBins * kBinWords];
+  __shared__ int32_t s_slot[kBinSegs];                  // the level's slot of each segment
+  __shared__ uint32_t s_heads[kRounds * kWarps];        // first positions of segments per warp and round
+  const uint32_t start = blockIdx.x * kBinChunk;
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+  int32_t slot[kRounds];
+  unsigned heads[kRounds];
+#pragma unroll
+  for (uint32_t r = 0; r < kRounds; ++r) {
+    const uint32_t pos = start + r * kThreads + threadIdx.x;
+    slot[r] = -1;
+    bool head = false;
+    if (pos < n) {
+      const uint32_t nd = node_of[pos];
+      slot[r] = A.slot_of[nd];
+      head = slot[r] >= 0 && (pos == start || node_of[pos - 1u] != nd);
+    }
+    heads[r] = __ballot_sync(0xffffffffu, head);
+    if (lane == 0u) s_heads[r * kWarps + warp] = static_cast<uint32_t>(__popc(heads[r]));
   }
-  const unsigned active = __ballot_sync(0xffffffffu, s >= 0);
-  if (s < 0) return;
-  const uint32_t* k = A.cb + 6 * s;
-  const float4 lo = A.blo[p], hi = A.bhi[p];
-  const uint32_t klo[3] = {fkey(lo.x), fkey(lo.y), fkey(lo.z)};
-  const uint32_t khi[3] = {fkey(hi.x), fkey(hi.y), fkey(hi.z)};
-  for (int a = 0; a < 3; ++a) {
-    const float c0 = fval(k[a]), ext = fval(k[3 + a]) - c0;
-    int bin = 0;
-    if (ext > 0.0f) {
-      bin = static_cast<int>((centroid(A.blo, A.bhi, p, a) - c0) * (static_cast<float>(kSahBins) / ext));
-      bin = bin < 0 ? 0 : (bin > kSahBins - 1 ? kSahBins - 1 : bin);
+  __syncthreads();
+  uint32_t segs = 0u, seg[kRounds];
+#pragma unroll
+  for (uint32_t r = 0; r < kRounds; ++r) {
+    for (uint32_t w = 0; w < kWarps; ++w) {
+      if (w == warp) seg[r] = segs + static_cast<uint32_t>(__popc(heads[r] & (0xffffffffu >> (31u - lane)))) - 1u;
+      segs += s_heads[r * kWarps + w];
     }
-    const uint32_t key = (static_cast<uint32_t>(s) * 3u + static_cast<uint32_t>(a)) * kSahBins + static_cast<uint32_t>(bin);
-    const unsigned grp = __match_any_sync(active, key);
-    const int leader = __ffs(grp) - 1;
-    const uint32_t mlo0 = __reduce_min_sync(grp, klo[0]), mlo1 = __reduce_min_sync(grp, klo[1]),
-                   mlo2 = __reduce_min_sync(grp, klo[2]);
-    const uint32_t mhi0 = __reduce_max_sync(grp, khi[0]), mhi1 = __reduce_max_sync(grp, khi[1]),
-                   mhi2 = __reduce_max_sync(grp, khi[2]);
-    if (static_cast<int>(threadIdx.x & 31u) == leader) {
-      uint32_t* w = bins + kBinWords * key;
-      atomicAdd(w, static_cast<uint32_t>(__popc(grp)));
-      atomicMin(w + 1, mlo0);
-      atomicMin(w + 2, mlo1);
-      atomicMin(w + 3, mlo2);
-      atomicMax(w + 4, mhi0);
-      atomicMax(w + 5, mhi1);
-      atomicMax(w + 6, mhi2);
+    if ((heads[r] >> lane) & 1u) s_slot[seg[r]] = slot[r];
+  }
+  if (segs == 0u) return;   // uniform over the block
+  const uint32_t words = segs * 3u * kSahBins * kBinWords;
+  for (uint32_t i = threadIdx.x; i < words; i += kThreads) {
+    const uint32_t f = i % kBinWords;
+    s_bin[i] = f >= 1u && f <= 3u ? 0xffffffffu : 0u;
+  }
+  __syncthreads();
+#pragma unroll
+  for (uint32_t r = 0; r < kRounds; ++r) {
+    if (slot[r] < 0) continue;
+    const uint32_t p = idx[start + r * kThreads + threadIdx.x];
+    const uint32_t* k = A.cb + 6 * slot[r];
+    const float4 lo = A.blo[p], hi = A.bhi[p];
+    const uint32_t klo[3] = {fkey(lo.x), fkey(lo.y), fkey(lo.z)};
+    const uint32_t khi[3] = {fkey(hi.x), fkey(hi.y), fkey(hi.z)};
+    const float c[3] = {0.5f * (lo.x + hi.x), 0.5f * (lo.y + hi.y), 0.5f * (lo.z + hi.z)};
+#pragma unroll
+    for (uint32_t a = 0; a < 3; ++a) {
+      const float c0 = fval(k[a]), ext = fval(k[3 + a]) - c0;
+      int bin = 0;
+      if (ext > 0.0f) {
+        bin = static_cast<int>((c[a] - c0) * (static_cast<float>(kSahBins) / ext));
+        bin = bin < 0 ? 0 : (bin > kSahBins - 1 ? kSahBins - 1 : bin);
+      }
+      uint32_t* w = s_bin + kBinWords * ((seg[r] * 3u + a) * kSahBins + static_cast<uint32_t>(bin));
+      atomicAdd(w, 1u);
+      atomicMin(w + 1, klo[0]);
+      atomicMin(w + 2, klo[1]);
+      atomicMin(w + 3, klo[2]);
+      atomicMax(w + 4, khi[0]);
+      atomicMax(w + 5, khi[1]);
+      atomicMax(w + 6, khi[2]);
     }
+  }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < words; i += kThreads) {
+    const uint32_t bin = i / kBinWords, f = i - bin * kBinWords;
+    if (s_bin[bin * kBinWords] == 0u) continue;
+    const uint32_t sg = bin / (3u * kSahBins);
+    uint32_t* w = bins + static_cast<size_t>(kBinWords) * (static_cast<size_t>(s_slot[sg]) * 3u * kSahBins + (bin - sg * 3u * kSahBins)) + f;
+    const uint32_t v = s_bin[i];
+    if (f == 0u) atomicAdd(w, v);
+    else if (f <= 3u) atomicMin(w, v);
+    else atomicMax(w, v);
   }
 }
 
@@ -1289,6 +1272,7 @@ cudaError_t read_scalar(const T* d, T& h, cudaStream_t s) {
 cudaError_t build_tree(const float4* blo, const float4* bhi, uint32_t n, bool sah, uint32_t* order, TNode* nodes,
                        uint32_t& n_nodes, Scratch& sc) {
   cudaStream_t s = sc.s;
+  const uint32_t leaf_max = sah ? kSahLeafMax : kLeafMax;
   const uint32_t cap_nodes = 2u * n;
   int32_t* slot_of = sc.get<int32_t>(cap_nodes);
   uint32_t* node_of = sc.get<uint32_t>(n);
@@ -1297,11 +1281,11 @@ cudaError_t build_tree(const float4* blo, const float4* bhi, uint32_t n, bool sa
   uint32_t* flag = sc.get<uint32_t>(n);
   uint32_t* excl = sc.get<uint32_t>(n + 1u);
   // Nodes of one level above kSmallNode primitives are disjoint: at most n / 65 of them;
-  // small subtree roots (5..64 primitives) are disjoint too.
+  // small subtree roots (leaf_max + 1..64 primitives) are disjoint too.
   const uint32_t max_act = n / (kSmallNode + 1u) + 2u;
   uint32_t* act = sc.get<uint32_t>(max_act);
   uint32_t* next = sc.get<uint32_t>(max_act);
-  uint32_t* small = sc.get<uint32_t>(n / (kLeafMax + 1u) + 2u);
+  uint32_t* small = sc.get<uint32_t>(n / (leaf_max + 1u) + 2u);
   uint32_t* counter = sc.get<uint32_t>(8);
   uint32_t* cb = sc.get<uint32_t>(6ull * max_act);
   int32_t* axis = sc.get<int32_t>(max_act);
@@ -1310,7 +1294,7 @@ cudaError_t build_tree(const float4* blo, const float4* bhi, uint32_t n, bool sa
   uint32_t* ident = sc.get<uint32_t>(max_act);
   uint32_t* bins = sah ? sc.get<uint32_t>(static_cast<size_t>(kBinWords) * 3u * kSahBins * max_act) : nullptr;
   if (sc.err != cudaSuccess) return sc.err;
-  BuildArrays A{blo, bhi, nodes, slot_of, cb, axis, split, nl, ident, counter};
+  BuildArrays A{blo, bhi, nodes, slot_of, cb, axis, split, nl, ident, counter, leaf_max};
   k_fill_u32<<<grid_for(cap_nodes), kThreads, 0, s>>>(reinterpret_cast<uint32_t*>(slot_of), cap_nodes, 0xffffffffu);
   k_fill_u32<<<grid_for(n), kThreads, 0, s>>>(node_of, n, 0u);
   k_root<<<1, 1, 0, s>>>(nodes, n, slot_of);
@@ -1320,7 +1304,7 @@ cudaError_t build_tree(const float4* blo, const float4* bhi, uint32_t n, bool sa
     init[4] = 1u;   // the root is the first level's one active node
     const uint32_t zero = 0u;
     BB_TRY(cudaMemcpyAsync(act, &zero, 4, cudaMemcpyHostToDevice, s));
-  } else if (n > kLeafMax) {
+  } else if (n > leaf_max) {
     init[2] = 1u;   // the root is a small subtree
     const uint32_t zero = 0u;
     BB_TRY(cudaMemcpyAsync(small, &zero, 4, cudaMemcpyHostToDevice, s));
@@ -1343,7 +1327,7 @@ cudaError_t build_tree(const float4* blo, const float4* bhi, uint32_t n, bool sa
     k_centroid_bounds<<<grid_for(n), kThreads, 0, s>>>(A, idx, node_of, n);
     if (sah) {
       k_sah_bin_init<<<bin_grid, kThreads, 0, s>>>(A, bins);
-      k_sah_bin<<<grid_for(n), kThreads, 0, s>>>(A, idx, node_of, n, bins);
+      k_sah_bin<<<grid_for(n, kBinChunk), kThreads, 0, s>>>(A, idx, node_of, n, bins);
       k_sah_split<<<split_grid, 128, 0, s>>>(A, bins);
     } else {
       k_midpoint_split<<<act_grid, kThreads, 0, s>>>(A);
@@ -1369,11 +1353,9 @@ cudaError_t build_tree(const float4* blo, const float4* bhi, uint32_t n, bool sa
   BB_TRY(read_scalar(counter + 2, n_small, s));
   k_small_base<<<1, 1, 0, s>>>(A);
   if (n_small > 0u) {
-    if (sah)
-      k_small_sah<<<std::min((n_small + kSmallWarps - 1u) / kSmallWarps, 148u * 16u), 32 * kSmallWarps, 0, s>>>(
-          A, small, n_small, idx);
-    else
-      k_small<<<grid_for(n_small, 64), 64, 0, s>>>(A, small, n_small, idx);
+    const unsigned small_grid = std::min((n_small + kSmallWarps - 1u) / kSmallWarps, 148u * 16u);
+    if (sah) k_small<true><<<small_grid, 32 * kSmallWarps, 0, s>>>(A, small, n_small, idx);
+    else k_small<false><<<small_grid, 32 * kSmallWarps, 0, s>>>(A, small, n_small, idx);
   }
   BB_TRY(cudaGetLastError());
   return read_scalar(counter, n_nodes, s);
@@ -1396,10 +1378,14 @@ cudaError_t finish_tree(const float4* blo, const float4* bhi, const uint32_t* or
   return cudaGetLastError();
 }
 
+// Each wide node starts at a binary internal node of its own (at a leaf only
+// when that is the root).
+uint32_t wide_capacity(uint32_t n_bin) { return n_bin / 2u + 1u; }
+
 cudaError_t collapse(const BinNode* bin, uint32_t n_bin, WideNode* out, uint32_t& n_wide, uint32_t& depth,
                      uint32_t& stack_required, Scratch& sc, int32_t* slot_bin = nullptr) {
   cudaStream_t s = sc.s;
-  const uint32_t cap = n_bin;   // wide nodes <= binary internal nodes + 1
+  const uint32_t cap = wide_capacity(n_bin);
   WideArrays W{bin, sc.get<WTemp>(cap), sc.get<uint32_t>(8), sc.get<uint32_t>(cap), sc.get<uint32_t>(cap),
                sc.get<int32_t>(cap), slot_bin};
   uint32_t* cur = sc.get<uint32_t>(cap);
@@ -1800,7 +1786,7 @@ cudaError_t BuildAccelOnDevice(const DeviceSceneArrays& sc_in, bool sah, cudaStr
     out.reference_topology = false;
   }
   WideNode* wide = nullptr;
-  BB_TRY(dmalloc(wide, n_trav, stream));
+  BB_TRY(dmalloc(wide, wide_capacity(n_trav), stream));
   out.nodes = reinterpret_cast<float4*>(wide);
   if (keep_refit) BB_TRY(dmalloc(out.refit->slot_bin, 4ull * n_trav, stream));
   BB_TRY(collapse(trav, n_trav, wide, out.wide_nodes, out.depth, out.stack_required, sc,

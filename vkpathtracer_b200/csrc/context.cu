@@ -512,7 +512,7 @@ int32_t upload_accel(vkptc_ctx* c, const std::vector<BinNode>& bin, const std::v
     const auto t0 = std::chrono::steady_clock::now();
     std::vector<BinNode> sah;
     std::vector<uint32_t> sah_prims;
-    BuildSahBvh(c->geo, 4u, sah, sah_prims);
+    BuildSahBvh(c->geo, kSahLeafMax, sah, sah_prims);
     CollapseToWide(c->geo, sah, sah_prims, bin, prim_indices, c->wide);
     build_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
   } else {

@@ -7,7 +7,7 @@
 //    accepted when 1e-4 < t < best; evaluated in the reference's exact
 //    operation order without fused multiply-adds, so t is bit-identical.
 //  * Boxes only cull.  Every triangle box is padded by 1e-4 as in the reference.
-//    The node test below places a slab within about 2^-24 (|o| + 4 |c - o|) of
+//    The node test below places a slab within about 2^-24 (|o| + 3 |c - o|) of
 //    where it is, which the padding covers for coordinates of a few hundred, so
 //    every triangle the reference could hit is reached there.
 //  * The reference treats an axis with |d| <= 1e-4 as "parallel" and there only
@@ -32,7 +32,7 @@
 //    the four children against 24 scalar multiply-adds and 24 min/max (which
 //    run at half rate) with corner bounds.
 //  * |d| is clamped to [1e-20, 1e20] for the box test, so there is no special
-//    case for a zero component, and 1/d is the approximate reciprocal.
+//    case for a zero component.
 //  * The children are ordered by three compare-exchanges: the nearest is exact,
 //    the rest are pushed as they come.  A full sort (five) measured 1-3 % slower.
 //  * A leaf is its own cursor: the leaf reference of the triangles not yet
@@ -101,12 +101,11 @@ struct RayPrep {
 
 // 1/d for the box test: |d| clamped to [1e-20, 1e20] keeps it finite and
 // non-zero (a component of 0 tests as a very long slab, i.e. whether the origin
-// lies inside), the approximate reciprocal is within 2^-23 of it.
+// lies inside).  The approximate reciprocal was 0.5 % faster, and one grazing hit
+// in ten more differed from the reference's on rays aimed at vertices from 20
+// scene radii away.
 __device__ __forceinline__ float box_inverse(float d) {
-  const float a = fminf(fmaxf(fabsf(d), 1e-20f), 1e20f);
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
-  return copysignf(r, d);
+  return copysignf(__frcp_rn(fminf(fmaxf(fabsf(d), 1e-20f), 1e20f)), d);
 }
 
 __device__ __forceinline__ RayPrep prep_ray(V3 o, V3 d) {
