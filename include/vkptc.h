@@ -68,7 +68,7 @@ typedef struct vkptc_config {
                                 spill to global memory); 0 = 12 */
   uint32_t math_mode;        /* 0 = parity (transcendentals in FP64, rounded once), 1 = fast FP32 */
   uint32_t collect_stats;    /* 1 = count node/leaf/triangle visits (device counters) */
-  uint32_t wave_paths;       /* paths per wavefront wave (0 = 4 Mi) */
+  uint32_t wave_paths;       /* paths per wavefront wave (0 = 16 Mi) */
   uint32_t stage_timing;     /* 1 = CUDA-event timing of every stage launch */
   uint32_t steps;            /* traversal steps between warp refills in the low 16 bits (0 = 8); the
                                 high 16 bits, when non-zero, refill a warp as soon as that many of its

@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) k_batch(const DevJob* __restr
     }
     {
       const BatchExtendSource src{jobs, P.ext[cur], P.job, P.ray_o, P.ray_d, P.hit};
-      persistent_traverse<BatchExtendSource, false, kStats, kWt>(src, n_ext, &P.ctl[kCtlFetchExt], stk, steps, st_e, lerr);
+      persistent_traverse<BatchExtendSource, false, kStats, kWt>(src, n_ext, &P.ctl[kCtlFetchExt], stk, steps, st_e, st_e, lerr);
     }
     if (!grid_barrier(P.ctl, P.barrier_spins)) break;
 
@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) k_batch(const DevJob* __restr
     {
       const uint32_t n_sh = P.ctl[kCtlShadow];
       const BatchShadowSource src{jobs, P.shq, P.job, P.sh_o, P.sh_d, P.sh_c, P.rad};
-      persistent_traverse<BatchShadowSource, true, kStats, kWt>(src, n_sh, &P.ctl[kCtlFetchShadow], stk, steps, st_s, lerr);
+      persistent_traverse<BatchShadowSource, true, kStats, kWt>(src, n_sh, &P.ctl[kCtlFetchShadow], stk, steps, st_s, st_s, lerr);
     }
     if (!grid_barrier(P.ctl, P.barrier_spins)) break;
 

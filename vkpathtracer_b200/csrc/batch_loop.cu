@@ -181,35 +181,6 @@ __global__ void k_lp_init(uint32_t* ctl) {
   if (i < static_cast<uint32_t>(kLoopCtlWords)) ctl[i] = 0u;
 }
 
-// Order in which REGEN hands out a sample's pixels: 1 = 8x4 tiles, band of
-// four rows by band (a warp's 32 camera rays cover a compact 8x4 block);
-// 0 = scanline order.  Each path still writes its own pixel's staging slot,
-// so films do not depend on the order.
-#ifndef VKPTC_TILE_ORDER
-#define VKPTC_TILE_ORDER 1
-#endif
-// The i-th pixel (y*W+x) of the tile order: bands of 4 rows (the last may be
-// shorter), each band cut into 8-pixel-wide tiles left to right (the last may
-// be narrower), each tile in row order.  A bijection on [0, W*H).
-__device__ __forceinline__ uint32_t tile_order_pixel(uint32_t i, uint32_t W, uint32_t H) {
-  const uint32_t band = i / (4u * W);
-  const uint32_t y0 = 4u * band;
-  const uint32_t bh = min(4u, H - y0);
-  const uint32_t r = i - y0 * W;                 // index inside the band
-  const uint32_t full = W / 8u;                  // full-width tiles in the band
-  uint32_t x, y;
-  if (r < full * 8u * bh) {
-    const uint32_t t = r / (8u * bh), k = r - t * 8u * bh;
-    x = 8u * t + (k & 7u);
-    y = y0 + (k >> 3);
-  } else {                                       // the narrow last tile
-    const uint32_t tw = W - 8u * full, k = r - full * 8u * bh;
-    x = 8u * full + k % tw;
-    y = y0 + k / tw;
-  }
-  return y * W + x;
-}
-
 // 1: REGEN claims work items and queue slots once per block and iteration;
 // 0: once per warp (ballot + shuffle).
 #ifndef VKPTC_REGEN_BLOCK
@@ -272,11 +243,7 @@ __global__ void __launch_bounds__(256) k_lp_regen(const DevJob* __restrict__ job
       const uint32_t W = J.settings.width;
       const uint32_t idx = static_cast<uint32_t>(g - J.path_base);
       const uint32_t sl = idx / J.pixels;
-#if VKPTC_TILE_ORDER
       const uint32_t px = tile_order_pixel(idx - sl * J.pixels, W, J.settings.height);
-#else
-      const uint32_t px = idx - sl * J.pixels;
-#endif
       const uint32_t local = sl * J.pixels + px;   // the staging slot: sample-major, then pixel (y*W+x)
       V3 o, d;
       uint64_t rng;
@@ -305,7 +272,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_lp_extend(const DevJob
   TraceStats st;
   uint32_t lerr = 0u;
   const LoopExtendSource src{jobs, P.gen[cur], P.hit};
-  persistent_traverse<LoopExtendSource, false, kStats, kWt>(src, n, &P.ctl[kLFetchExt], stk, steps, st, lerr);
+  persistent_traverse<LoopExtendSource, false, kStats, kWt>(src, n, &P.ctl[kLFetchExt], stk, steps, st, st, lerr);
   flush_stats<kStats>(ctr, st, false);
   if (lerr) atomicOr(err, lerr);
 }
@@ -412,7 +379,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_lp_shadow(const DevJob
   uint32_t lerr = 0u;
   // The queries of the previous shading stage; their survivors are generation `cur` now.
   const LoopShadowSource src{jobs, P, P.gen[cur]};
-  persistent_traverse<LoopShadowSource, true, kStats, kWt>(src, n, &P.ctl[kLFetchShadow], stk, steps, st, lerr);
+  persistent_traverse<LoopShadowSource, true, kStats, kWt>(src, n, &P.ctl[kLFetchShadow], stk, steps, st, st, lerr);
   flush_stats<kStats>(ctr, st, true);
   if (lerr) atomicOr(err, lerr);
 }

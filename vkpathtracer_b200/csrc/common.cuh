@@ -173,6 +173,7 @@ struct DevScene {
   uint32_t prim_count;
   uint32_t has_transmissive;
   uint32_t has_effects;       // some material has a procedural effect (1..19)
+  uint32_t has_exotic;        // some material is transmissive, clear-coated, sheen or toon
   V3 env;
   const float4* env_map;      // equirectangular texels (rgb, w unused), or null
   uint32_t env_w, env_h;
@@ -203,6 +204,31 @@ struct DevSettings {
   float firefly_clamp;
   uint32_t frame;
 };
+
+// Camera paths are handed out in 8x4 pixel tiles, so a warp's rays cover a
+// compact block.  Each path still writes its own pixel, so films do not depend
+// on the order.
+// The i-th pixel (y*W+x) of the tile order: bands of 4 rows (the last may be
+// shorter), each band cut into 8-pixel-wide tiles left to right (the last may
+// be narrower), each tile in row order.  A bijection on [0, W*H).
+__device__ __forceinline__ uint32_t tile_order_pixel(uint32_t i, uint32_t W, uint32_t H) {
+  const uint32_t band = i / (4u * W);
+  const uint32_t y0 = 4u * band;
+  const uint32_t bh = min(4u, H - y0);
+  const uint32_t r = i - y0 * W;                 // index inside the band
+  const uint32_t full = W / 8u;                  // full-width tiles in the band
+  uint32_t x, y;
+  if (r < full * 8u * bh) {
+    const uint32_t t = r / (8u * bh), k = r - t * 8u * bh;
+    x = 8u * t + (k & 7u);
+    y = y0 + (k >> 3);
+  } else {                                       // the narrow last tile
+    const uint32_t tw = W - 8u * full, k = r - full * 8u * bh;
+    x = 8u * full + k % tw;
+    y = y0 + k / tw;
+  }
+  return y * W + x;
+}
 
 // Warp-aggregated append: one atomic per warp for all active lanes that want
 // a slot; returns this lane's slot (or unspecified when !want).

@@ -8,10 +8,11 @@
 //   hemisphere / Phong lobe     src/pathtracer/ScalarCpuPathTracer.cpp:978-1020
 //   FilmBuffer add / resolve    src/pathtracer/FilmBuffer.cpp:80-91, 160-214
 // split into wavefront stages that exchange structure-of-arrays queues:
-//   raygen -> for each depth: extend (closest hit) -> shade (material, NEE
-//   set-up, BSDF sample, Russian roulette; appends shadow queries and the next
-//   extension queue with warp-aggregated atomics) -> shadow (any hit) ->
-//   accumulate into the film in sample order.
+//   raygen -> for each depth: trace (closest hits of this depth's paths and the
+//   previous depth's shadow queries, one launch) -> shade (material, NEE set-up,
+//   BSDF sample, Russian roulette; appends shadow queries and the next extension
+//   queue with warp-aggregated atomics) -> accumulate into the film in sample
+//   order.  Scenes with SDF primitives add two load-balanced stages (below).
 // The per-path RNG stream is keyed exactly as the reference keys it, so the
 // wavefront reordering does not change any random number a path draws, and
 // the stages add radiance terms in the reference's order (emission, then the
@@ -57,75 +58,135 @@ struct RaysSource {   // batched ray queries from a ray array
   }
 };
 
-struct ExtendSource {  // closest hit for the queued paths of a wave
+// A wave's traversal queries: the extension rays of the queued paths (closest
+// hit), then the shadow queries of the previous depth's shading (its term is
+// added when visible).  A shadow query is any-hit; with kTrans (the scene has
+// transmissive materials) it is the reference's closest-hit loop that steps
+// through up to 8 transmissive occluders
+// (src/pathtracer/ScalarCpuPathTracer.cpp:1067-1087), bounded by the distance
+// that is left, and goes on in the same lane after each of them.
+constexpr uint32_t kDroppedQuery = 0xFFFFFFFFu;   // sh_path of a query an SDF occludes
+
+template <bool kTrans>
+struct WaveTraceSource {
   GeoView geo;
-  static constexpr bool kUniform = true;
-  __device__ __forceinline__ const GeoView& geo_at(uint32_t) const { return geo; }
   const uint32_t* q;
   const float4* ray_o;
   const float4* ray_d;
   float2* hit;
-  __device__ __forceinline__ void load(uint32_t j, V3& o, V3& d, float& tm, GeoView& g) const {
-    g = geo;
-    const uint32_t p = q[j];
-    const float4 a = ray_o[p], b = ray_d[p];
-    o = mk(a.x, a.y, a.z);
-    d = mk(b.x, b.y, b.z);
-    tm = kInf;
-  }
-  __device__ __forceinline__ void finish(uint32_t j, float t, uint32_t prim) const {
-    hit[q[j]] = make_float2(t, __uint_as_float(prim));
-  }
-};
-
-struct ShadowSource {  // any hit for the NEE queries; adds the term when visible
-  GeoView geo;
-  static constexpr bool kUniform = true;
-  __device__ __forceinline__ const GeoView& geo_at(uint32_t) const { return geo; }
-  const float4* sh_o;
-  const float4* sh_d;
+  float4* sh_o;         // kTrans rewrites origin's w (the distance left)
+  float4* sh_d;         // and direction's w (occluders passed, bits)
   const float4* sh_c;
   const uint32_t* sh_path;
   float4* rad;
+  uint32_t n_ext;
+  const float4* shade;
+  const float* materials;
+  uint32_t material_count;
+  static constexpr bool kUniform = true;
+  __device__ __forceinline__ const GeoView& geo_at(uint32_t) const { return geo; }
+  __device__ __forceinline__ bool shadow(uint32_t j) const { return j >= n_ext; }
+  __device__ __forceinline__ bool any(uint32_t j) const { return !kTrans && j >= n_ext; }
   __device__ __forceinline__ void load(uint32_t j, V3& o, V3& d, float& tm, GeoView& g) const {
     g = geo;
-    const float4 a = sh_o[j], b = sh_d[j];
+    const bool sh = j >= n_ext;
+    const uint32_t k = sh ? j - n_ext : q[j];
+    const float4 a = (sh ? sh_o : ray_o)[k], b = (sh ? sh_d : ray_d)[k];
     o = mk(a.x, a.y, a.z);
     d = mk(b.x, b.y, b.z);
-    tm = a.w;
+    tm = sh ? a.w : kInf;
   }
-  __device__ __forceinline__ void finish(uint32_t j, float, uint32_t occluded) const {
-    if (occluded) return;
-    const uint32_t p = sh_path[j];
-    const float4 c = sh_c[j];
-    float4 r = rad[p];
+  // Returns true when the query goes on from a new origin.
+  __device__ __forceinline__ bool finish(uint32_t j, float t, uint32_t prim, V3& o, V3 d, float& tmax) const {
+    if (j < n_ext) {
+      hit[q[j]] = make_float2(t, __uint_as_float(prim));
+      return false;
+    }
+    const uint32_t k = j - n_ext;
+    if constexpr (kTrans) {
+      if (prim != kMiss) {
+        const uint32_t mat_index = __float_as_uint(__ldg(shade + prim).w);
+        const uint32_t mi = mat_index < material_count - 1u ? mat_index : material_count - 1u;
+        const float* mm = materials + 16u * mi;
+        if (!(static_cast<uint32_t>(mm[7] + 0.5f) == 5u || mm[10] > 0.05f)) return false;   // occluded
+        const float adv = t + 0.004f;
+        const float left = sh_o[k].w - adv;
+        const uint32_t passed = __float_as_uint(sh_d[k].w) + 1u;
+        if (passed < 8u && left > 0.004f) {
+          o = add(o, mul(d, adv));
+          tmax = left;
+          sh_o[k].w = left;
+          sh_d[k].w = __uint_as_float(passed);
+          return true;
+        }
+      }
+    } else {
+      if (prim) return false;
+    }
+    const uint32_t path = sh_path[k];
+    if (path == kDroppedQuery) return false;
+    const float4 c = sh_c[k];
+    float4 r = rad[path];
     r.x = r.x + c.x;
     r.y = r.y + c.y;
     r.z = r.z + c.z;
-    rad[p] = r;
+    rad[path] = r;
+    return false;
   }
 };
 
-template <class Src, bool kAny, bool kStats, bool kWt = false>
-__device__ __forceinline__ void run_persistent(const Src& src, uint32_t n, uint32_t* fetch,
-                                               int scap, int2* spill, int total, int steps,
-                                               unsigned long long* c_nodes, unsigned long long* c_leaves,
-                                               unsigned long long* c_tris, unsigned long long* c_rays, uint32_t* err) {
-  extern __shared__ int2 smem_stack[];
-  const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x;
-  const int gstride = static_cast<int>(gridDim.x * blockDim.x);
-  TwoLevelStack stk{smem_stack + threadIdx.x, static_cast<int>(blockDim.x), scap,
-                    spill ? spill + gtid : nullptr, gstride, total};
-  TraceStats st;
-  uint32_t lerr = 0u;
-  persistent_traverse<Src, kAny, kStats, kWt>(src, n, fetch, stk, steps, st, lerr);
-  if (kStats) {
-    warp_count(c_nodes, st.nodes);
-    warp_count(c_leaves, st.leaves);
-    warp_count(c_tris, st.tris);
-    warp_count(c_rays, st.rays);
+// SDF closest hits of the extension queue, folded into the triangle hits.
+struct WaveSdfExtSource {
+  const float4* sdf;
+  uint32_t sdf_count;
+  const uint32_t* q;
+  const float4* ray_o;
+  const float4* ray_d;
+  float2* hit;
+  __device__ __forceinline__ void load(uint32_t j, SdfLane& L) const {
+    L.sdf = sdf;
+    L.count = sdf_count;
+    const uint32_t p = q[j];
+    const float4 a = ray_o[p], b = ray_d[p];
+    const float2 h = hit[p];
+    L.o = mk(a.x, a.y, a.z);
+    L.d = mk(b.x, b.y, b.z);
+    L.best = h.x;
+    L.prim = __float_as_uint(h.y);
   }
-  if (lerr) atomicOr(err, lerr);
+  __device__ __forceinline__ void finish(uint32_t j, const SdfLane& L) const {
+    hit[q[j]] = make_float2(L.best, __uint_as_float(L.prim));
+  }
+};
+
+// SDF occlusion of the shadow queries: an occluded query is dropped (its bound
+// set to 0, so the triangle any-hit does no work for it either).
+struct WaveSdfShadowSource {
+  const float4* sdf;
+  uint32_t sdf_count;
+  float4* sh_o;
+  const float4* sh_d;
+  uint32_t* sh_path;
+  __device__ __forceinline__ void load(uint32_t k, SdfLane& L) const {
+    L.sdf = sdf;
+    L.count = sdf_count;
+    const float4 a = sh_o[k], b = sh_d[k];
+    L.o = mk(a.x, a.y, a.z);
+    L.d = mk(b.x, b.y, b.z);
+    L.best = a.w;
+    L.prim = 0u;
+  }
+  __device__ __forceinline__ void finish(uint32_t k, const SdfLane& L) const {
+    if (L.prim == 0u) return;
+    sh_path[k] = kDroppedQuery;
+    sh_o[k].w = 0.0f;
+  }
+};
+
+__device__ __forceinline__ TwoLevelStack launch_stack(int2* smem_stack, int scap, int2* spill, int total) {
+  const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x;
+  return TwoLevelStack{smem_stack + threadIdx.x, static_cast<int>(blockDim.x), scap, spill ? spill + gtid : nullptr,
+                       static_cast<int>(gridDim.x * blockDim.x), total};
 }
 
 // The traversal kernels run at 64 registers (at least 1024 threads per SM):
@@ -136,8 +197,18 @@ __device__ __forceinline__ void run_persistent(const Src& src, uint32_t n, uint3
 template <bool kAny, bool kStats, bool kWt>
 __global__ void __launch_bounds__(256, 4) k_trace_rays(DevScene s, RaysSource src, uint32_t n, uint32_t* fetch, int scap,
                                                     int2* spill, int total, int steps, DevCounters* ctr, uint32_t* err) {
-  run_persistent<RaysSource, kAny, kStats, kWt>(src, n, fetch, scap, spill, total, steps, &ctr->nodes, &ctr->leaves,
-                                                &ctr->tris, &ctr->ext_rays, err);
+  extern __shared__ int2 smem_stack[];
+  TraceStats st;
+  uint32_t lerr = 0u;
+  persistent_traverse<RaysSource, kAny ? kQueryAny : kQueryClosest, kStats, kWt>(
+      src, n, fetch, launch_stack(smem_stack, scap, spill, total), steps, st, st, lerr);
+  if (kStats) {
+    warp_count(&ctr->nodes, st.nodes);
+    warp_count(&ctr->leaves, st.leaves);
+    warp_count(&ctr->tris, st.tris);
+    warp_count(&ctr->ext_rays, st.rays);
+  }
+  if (lerr) atomicOr(err, lerr);
 }
 
 cudaError_t LaunchTraceRays(const DevScene& s, const float* rays, const float* tmax, uint64_t n, bool any_hit,
@@ -166,13 +237,39 @@ cudaError_t LaunchTraceRays(const DevScene& s, const float* rays, const float* t
   return cudaGetLastError();
 }
 
+// Control words of a wave (WaveState::counts).
+constexpr int kWaveExt = 0;           // extension queue sizes: words 0, 1
+constexpr int kWaveShadow = 2;        // shadow queue size by the depth that fills it (even, odd): words 2, 3
+constexpr int kWaveFetch = 4;         // query counters of the trace stage; word 5: its shadow part alone
+constexpr int kWaveFetchSdf = 6, kWaveFetchSdfShadow = 7;
+
 // ==================================================================== raygen
+// Slots of a wave: the tile's pixels in 8x4 tiles, 32 pixels at a time, all
+// samples of 32 pixels before the next, so that neighbouring warps' paths start
+// in the same place (the slots of the last, incomplete 32 are sample-major).
+__device__ __forceinline__ uint32_t wave_slot(uint32_t k, uint32_t sl, uint32_t tile_px, uint32_t samples) {
+  const uint32_t full = tile_px & ~31u;
+  if (k < full) return (k & ~31u) * samples + sl * 32u + (k & 31u);
+  return full * samples + sl * (tile_px - full) + (k - full);
+}
+
 template <bool kParity>
 __global__ void __launch_bounds__(256) k_raygen(DevScene s, DevSettings st, WaveState w, WaveTile tile) {
   const uint32_t tile_px = tile.w * tile.h;
   const uint32_t n = tile_px * tile.sample_count;
+  const uint32_t full = tile_px & ~31u, rest = tile_px - full;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const uint32_t sl = i / tile_px, pl = i - sl * tile_px;
+    uint32_t sl, k;
+    if (i < full * tile.sample_count) {
+      const uint32_t g = (i >> 5) / tile.sample_count;
+      sl = (i >> 5) - g * tile.sample_count;
+      k = 32u * g + (i & 31u);
+    } else {
+      const uint32_t r = i - full * tile.sample_count;
+      sl = r / rest;
+      k = full + r - sl * rest;
+    }
+    const uint32_t pl = tile_order_pixel(k, tile.w, tile.h);
     const uint32_t x = tile.x + pl % tile.w, y = tile.y + pl / tile.w;
     V3 o, d;
     uint64_t rng;
@@ -184,59 +281,98 @@ __global__ void __launch_bounds__(256) k_raygen(DevScene s, DevSettings st, Wave
     w.rad[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     w.q[0][i] = i;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    w.counts[0] = n;
-    w.counts[1] = 0u;
-    w.counts[2] = 0u;
-    w.counts[3] = 0u;   // extension fetch counter
-    w.counts[4] = 0u;   // shadow fetch counter
-  }
+  if (blockIdx.x == 0 && threadIdx.x < 8u) w.counts[threadIdx.x] = threadIdx.x == kWaveExt ? n : 0u;
 }
 
-// ==================================================================== extend
-// Closest-hit traversal of the current extension queue (persistent warps).
-// Zeroes the next queue's and the shadow queue's sizes for the shade stage.
-template <bool kStats, bool kWt>
-__global__ void __launch_bounds__(256, 4) k_extend(DevScene s, WaveState w, uint32_t cur, int scap, int2* spill,
-                                                int total, int steps, DevCounters* ctr, uint32_t* err) {
-  const uint32_t n = w.counts[cur];
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    w.counts[cur ^ 1u] = 0u;
-    w.counts[2] = 0u;
+// ===================================================================== trace
+// The closest hits of depth `depth`'s paths and the shadow queries depth - 1's
+// shading left (persistent warps): neither touches what the other reads or
+// writes, and one launch has one tail instead of two.  `parts`: 1 the
+// extension rays, 2 the shadow queries, 3 both.  Zeroes the next extension
+// queue's size and the shadow queue size the coming shading appends to.
+template <bool kStats, bool kWt, bool kTrans>
+__global__ void __launch_bounds__(256, 4) k_trace(DevScene s, WaveState w, const uint32_t* q, uint32_t depth,
+                                                  uint32_t parts, int scap, int2* spill, int total, int steps,
+                                                  DevCounters* ctr, uint32_t* err) {
+  extern __shared__ int2 smem_stack[];
+  const uint32_t cur = depth & 1u;
+  const uint32_t n_ext = (parts & 1u) ? w.counts[kWaveExt + cur] : 0u;
+  const uint32_t n_sh = (parts & 2u) ? w.counts[kWaveShadow + (cur ^ 1u)] : 0u;
+  if (blockIdx.x == 0 && threadIdx.x == 0 && (parts & 1u)) {
+    w.counts[kWaveExt + (cur ^ 1u)] = 0u;
+    w.counts[kWaveShadow + cur] = 0u;
+    w.counts[kWaveFetchSdf] = 0u;
+    w.counts[kWaveFetchSdfShadow] = 0u;
   }
-  const ExtendSource src{geo_of(s), w.q[cur], w.ray_o, w.ray_d, w.hit};
-  run_persistent<ExtendSource, false, kStats, kWt>(src, n, &w.counts[3], scap, spill, total, steps, &ctr->nodes,
-                                                   &ctr->leaves, &ctr->tris, &ctr->ext_rays, err);
+  const WaveTraceSource<kTrans> src{geo_of(s), q, w.ray_o, w.ray_d, w.hit, w.sh_o, w.sh_d, w.sh_c, w.sh_path, w.rad,
+                                    n_ext, s.shade, s.materials, s.material_count};
+  TraceStats st, st_sh;
+  uint32_t lerr = 0u;
+  persistent_traverse<WaveTraceSource<kTrans>, kQueryMixed, kStats, kWt>(
+      src, n_ext + n_sh, &w.counts[kWaveFetch + ((parts & 1u) ? 0 : 1)], launch_stack(smem_stack, scap, spill, total),
+      steps, st, st_sh, lerr);
+  if (kStats) {
+    warp_count(&ctr->nodes, st.nodes);
+    warp_count(&ctr->leaves, st.leaves);
+    warp_count(&ctr->tris, st.tris);
+    warp_count(&ctr->ext_rays, st.rays);
+    warp_count(&ctr->shadow_nodes, st_sh.nodes);
+    warp_count(&ctr->shadow_leaves, st_sh.leaves);
+    warp_count(&ctr->shadow_tris, st_sh.tris);
+    warp_count(&ctr->shadow_rays, st_sh.rays);
+  }
+  if (lerr) atomicOr(err, lerr);
 }
 
-constexpr uint32_t kSmemLights = 64;   // lights staged in shared memory by the shade stage
+// ======================================================================= SDF
+// One sphere-tracing step per lane and call, lanes refilled as their queries
+// finish, so a warp is not held by its longest march (inside the shading stage
+// the marches took nine tenths of a frame of the SDF gallery).
+constexpr int kWaveSdfSteps = 8;   // march steps between refills
 
-template <bool kParity, bool kEffects>
-__global__ void __launch_bounds__(256, 3) k_shade(DevScene s, DevSettings st, WaveState w, uint32_t cur,
-                                               uint32_t depth, DevCounters* ctr) {
-  __shared__ float sm_lights[16 * kSmemLights];
-  const bool staged = s.light_count <= kSmemLights;
-  if (staged) {
-    for (uint32_t k = threadIdx.x; k < 16u * s.light_count; k += blockDim.x) sm_lights[k] = s.lights[k];
-    __syncthreads();
+__device__ __forceinline__ void flush_sdf(DevCounters* ctr, const SdfCount& c) {
+  warp_count(&ctr->sdf_tests, c.tests);
+  warp_count(&ctr->sdf_steps, c.steps);
+  warp_count(&ctr->sdf_hits, c.hits);
+}
+
+__global__ void __launch_bounds__(256) k_sdf(DevScene s, WaveState w, const uint32_t* q, uint32_t depth,
+                                             DevCounters* ctr) {
+  const uint32_t n = w.counts[kWaveExt + (depth & 1u)];
+  SdfCount c;
+  const WaveSdfExtSource src{s.sdf, s.sdf_count, q, w.ray_o, w.ray_d, w.hit};
+  sdf_persistent<WaveSdfExtSource, false>(src, n, &w.counts[kWaveFetchSdf], kWaveSdfSteps, c);
+  flush_sdf(ctr, c);
+}
+
+__global__ void __launch_bounds__(256) k_sdf_shadow(DevScene s, WaveState w, uint32_t depth, DevCounters* ctr) {
+  const uint32_t n = w.counts[kWaveShadow + (depth & 1u)];
+  SdfCount c;
+  const WaveSdfShadowSource src{s.sdf, s.sdf_count, w.sh_o, w.sh_d, w.sh_path};
+  sdf_persistent<WaveSdfShadowSource, true>(src, n, &w.counts[kWaveFetchSdfShadow], kWaveSdfSteps, c);
+  flush_sdf(ctr, c);
+}
+
+// ===================================================================== shade
+// Variants as in the loop driver: code no path of the scene can reach
+// (procedural effects, SDF hits, transmissive / clear-coat / sheen / toon
+// materials and the environment map) is compiled out, because the stage waits
+// on instruction fetch more than on anything else.
+template <bool kParity, bool kEffects, bool kSdf, bool kExotic>
+__global__ void __launch_bounds__(256, 3) k_shade(DevScene s, DevSettings st, WaveState w, const uint32_t* q,
+                                                  uint32_t* qn, uint32_t depth, DevCounters* ctr) {
+  const uint32_t cur = depth & 1u;
+  const uint32_t n = w.counts[kWaveExt + cur];
+  if (blockIdx.x == 0 && threadIdx.x == 0) {   // the next trace stage claims from 0
+    w.counts[kWaveFetch] = 0u;
+    w.counts[kWaveFetch + 1] = 0u;
   }
-  const float* lights = staged ? sm_lights : s.lights;
-  const uint32_t n = w.counts[cur];
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    w.counts[3] = 0u;   // the extension stage of the next depth fetches from 0
-    w.counts[4] = 0u;   // the shadow stage of this depth fetches from 0
-  }
-  const uint32_t* q = w.q[cur];
-  uint32_t* qn = w.q[cur ^ 1u];
+  uint32_t shadow_tests = 0u;
   for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
     const uint32_t j = base + threadIdx.x;
-    bool emit_next = false, emit_shadow = false;
     uint32_t p = 0u;
-    uint32_t shadow_tests = 0u;
-    SdfCount sdf_n;
-    // shadow query payload
-    V3 sh_o = mk(0, 0, 0), sh_d = mk(0, 0, 0), sh_c = mk(0, 0, 0);
-    float sh_t = 0.0f;
+    ShadeOut R;
+    R.next = R.shadow = false;
     if (j < n) {
       p = q[j];
       const float4 o4 = w.ray_o[p], d4 = w.ray_d[p], t4 = w.thr[p], r4 = w.rad[p];
@@ -248,7 +384,7 @@ __global__ void __launch_bounds__(256, 3) k_shade(DevScene s, DevSettings st, Wa
       P.rad = mk(r4.x, r4.y, r4.z);
       P.segs = r4.w;
       P.rng = w.rng[p];
-      const ShadeOut R = shade_bounce<kParity, kEffects>(s, st, lights, depth, P, h2.x, __float_as_uint(h2.y));
+      R = shade_bounce<kParity, kEffects, kSdf, kExotic>(s, st, s.lights, depth, P, h2.x, __float_as_uint(h2.y), true);
       if (R.next) {
         w.ray_o[p] = make_float4(P.o.x, P.o.y, P.o.z, 0.0f);
         w.ray_d[p] = make_float4(P.d.x, P.d.y, P.d.z, 0.0f);
@@ -256,53 +392,31 @@ __global__ void __launch_bounds__(256, 3) k_shade(DevScene s, DevSettings st, Wa
         w.rng[p] = P.rng;
       }
       w.rad[p] = make_float4(P.rad.x, P.rad.y, P.rad.z, P.segs);
-      emit_next = R.next;
-      emit_shadow = R.shadow;
-      shadow_tests = R.shadow_tests;
-      sdf_n = R.sdf;
-      sh_o = R.sh_o;
-      sh_d = R.sh_d;
-      sh_c = R.sh_c;
-      sh_t = R.sh_t;
+      shadow_tests += R.shadow_tests;
     }
     // Warp-aggregated appends (the whole warp reaches these together).
-    const uint32_t slot_n = warp_append(&w.counts[cur ^ 1u], emit_next);
-    if (emit_next) qn[slot_n] = p;
-    const uint32_t slot_s = warp_append(&w.counts[2], emit_shadow);
-    if (emit_shadow) {
+    const uint32_t slot_n = warp_append(&w.counts[kWaveExt + (cur ^ 1u)], R.next);
+    if (R.next) qn[slot_n] = p;
+    const uint32_t slot_s = warp_append(&w.counts[kWaveShadow + cur], R.shadow);
+    if (R.shadow) {
       w.sh_path[slot_s] = p;
-      w.sh_o[slot_s] = make_float4(sh_o.x, sh_o.y, sh_o.z, sh_t);
-      w.sh_d[slot_s] = make_float4(sh_d.x, sh_d.y, sh_d.z, 0.0f);
-      w.sh_c[slot_s] = make_float4(sh_c.x, sh_c.y, sh_c.z, 0.0f);
-    }
-    warp_count(&ctr->shadow_tests, shadow_tests);
-    if (s.sdf_count != 0u) {
-      warp_count(&ctr->sdf_tests, sdf_n.tests);
-      warp_count(&ctr->sdf_steps, sdf_n.steps);
-      warp_count(&ctr->sdf_hits, sdf_n.hits);
+      w.sh_o[slot_s] = make_float4(R.sh_o.x, R.sh_o.y, R.sh_o.z, R.sh_t);
+      w.sh_d[slot_s] = make_float4(R.sh_d.x, R.sh_d.y, R.sh_d.z, 0.0f);
+      w.sh_c[slot_s] = make_float4(R.sh_c.x, R.sh_c.y, R.sh_c.z, 0.0f);
     }
   }
+  warp_count(&ctr->shadow_tests, shadow_tests);
 }
 
-// ==================================================================== shadow
-// Any-hit visibility of the NEE queries (persistent warps); adds the NEE term
-// of every visible query to its path's radiance.
+// Scenes with transmissive materials and SDF primitives: each shadow query's
+// closest-hit loop tests the SDF primitives after the triangles (one query per
+// thread; scenes without SDF primitives take these queries in k_trace).
 template <bool kStats, bool kWt>
-__global__ void __launch_bounds__(256, 4) k_shadow(DevScene s, WaveState w, int scap, int2* spill, int total, int steps,
-                                                DevCounters* ctr, uint32_t* err) {
-  const uint32_t n = w.counts[2];
-  const ShadowSource src{geo_of(s), w.sh_o, w.sh_d, w.sh_c, w.sh_path, w.rad};
-  run_persistent<ShadowSource, true, kStats, kWt>(src, n, &w.counts[4], scap, spill, total, steps, &ctr->shadow_nodes,
-                                             &ctr->shadow_leaves, &ctr->shadow_tris, &ctr->shadow_rays, err);
-}
-
-// Scenes with transmissive materials: the reference's closest-hit loop that
-// steps through up to 8 transmissive occluders (one query per thread).
-template <bool kStats, bool kWt>
-__global__ void __launch_bounds__(256) k_shadow_transmissive(DevScene s, WaveState w, int cap, DevCounters* ctr, uint32_t* err) {
+__global__ void __launch_bounds__(256) k_shadow_transmissive(DevScene s, WaveState w, uint32_t depth, int cap,
+                                                             DevCounters* ctr, uint32_t* err) {
   extern __shared__ int2 smem_stack[];
   const TwoLevelStack stk = smem_stack_of(smem_stack + threadIdx.x, static_cast<int>(blockDim.x), cap);
-  const uint32_t n = w.counts[2];
+  const uint32_t n = w.counts[kWaveShadow + (depth & 1u)];
   uint32_t local_err = 0u;
   for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
     const uint32_t j = base + threadIdx.x;
@@ -314,30 +428,26 @@ __global__ void __launch_bounds__(256) k_shadow_transmissive(DevScene s, WaveSta
       const V3 sd = mk(d4.x, d4.y, d4.z);
       float remain = o4.w;
       bool visible = true;
-      if (!s.has_transmissive) {
-        visible = !trace_any<kStats, kWt>(s, so, sd, remain, stk, st, local_err);
-      } else {
-        // Closest-hit loop that steps through up to 8 transmissive occluders
-        // (src/pathtracer/ScalarCpuPathTracer.cpp:1067-1087).
-        for (uint32_t skips = 0; skips < 8u && remain > 0.004f; ++skips) {
-          float t;
-          uint32_t prim;
-          trace_closest<kStats, kWt>(s, so, sd, stk, t, prim, st, local_err);
-          if (s.sdf_count != 0u) sdf_closest(s.sdf, s.sdf_count, so, sd, t, prim, sdf_n);
-          if (prim == kMiss || t >= remain) break;
-          const uint32_t mat_index = (prim & kSdfTag) ? sdf_material(s.sdf, prim & ~kSdfTag)
-                                                      : __float_as_uint(__ldg(s.shade + prim).w);
-          const uint32_t mi = mat_index < s.material_count - 1u ? mat_index : s.material_count - 1u;
-          const float* mm = s.materials + 16u * mi;
-          const bool tr = static_cast<uint32_t>(mm[7] + 0.5f) == 5u || mm[10] > 0.05f;
-          if (!tr) {
-            visible = false;
-            break;
-          }
-          const float adv = t + 0.004f;
-          so = add(so, mul(sd, adv));
-          remain -= adv;
+      // Closest-hit loop that steps through up to 8 transmissive occluders
+      // (src/pathtracer/ScalarCpuPathTracer.cpp:1067-1087).
+      for (uint32_t skips = 0; skips < 8u && remain > 0.004f; ++skips) {
+        float t;
+        uint32_t prim;
+        trace_closest<kStats, kWt>(s, so, sd, stk, t, prim, st, local_err);
+        if (s.sdf_count != 0u) sdf_closest(s.sdf, s.sdf_count, so, sd, t, prim, sdf_n);
+        if (prim == kMiss || t >= remain) break;
+        const uint32_t mat_index = (prim & kSdfTag) ? sdf_material(s.sdf, prim & ~kSdfTag)
+                                                    : __float_as_uint(__ldg(s.shade + prim).w);
+        const uint32_t mi = mat_index < s.material_count - 1u ? mat_index : s.material_count - 1u;
+        const float* mm = s.materials + 16u * mi;
+        const bool tr = static_cast<uint32_t>(mm[7] + 0.5f) == 5u || mm[10] > 0.05f;
+        if (!tr) {
+          visible = false;
+          break;
         }
+        const float adv = t + 0.004f;
+        so = add(so, mul(sd, adv));
+        remain -= adv;
       }
       if (visible) {
         const uint32_t p = w.sh_path[j];
@@ -369,15 +479,16 @@ __global__ void __launch_bounds__(256) k_accumulate(DevSettings st, WaveState w,
                                                     DevCounters* ctr) {
   const uint32_t tile_px = tile.w * tile.h;
   for (uint32_t base = blockIdx.x * blockDim.x; base < tile_px; base += gridDim.x * blockDim.x) {
-    const uint32_t pl = base + threadIdx.x;
+    const uint32_t k = base + threadIdx.x;
     uint32_t samples = 0u, segs = 0u, dropped = 0u;
-    if (pl < tile_px) {
+    if (k < tile_px) {
+      const uint32_t pl = tile_order_pixel(k, tile.w, tile.h);
       const uint32_t x = tile.x + pl % tile.w, y = tile.y + pl / tile.w;
       const size_t px = static_cast<size_t>(y) * film.width + x;
       float4 acc = film.sum[px];
       uint32_t cnt = film.count[px];
       for (uint32_t sl = 0; sl < tile.sample_count; ++sl) {
-        const float4 r = w.rad[sl * tile_px + pl];
+        const float4 r = w.rad[wave_slot(k, sl, tile_px, tile.sample_count)];
         if (!(isfinite(r.x) && isfinite(r.y) && isfinite(r.z))) {
           ++dropped;   // dropped before the film, like the reference's shade_pixel
           continue;
@@ -404,68 +515,83 @@ __global__ void __launch_bounds__(256) k_accumulate(DevSettings st, WaveState w,
   }
 }
 
+namespace {
+
+using TraceFn = void (*)(DevScene, WaveState, const uint32_t*, uint32_t, uint32_t, int, int2*, int, int, DevCounters*,
+                         uint32_t*);
+// [stats][watertight][transmissive shadow queries]
+TraceFn trace_fn(bool stats, bool wt, bool trans) {
+  static const TraceFn t[2][2][2] = {
+      {{k_trace<false, false, false>, k_trace<false, false, true>}, {k_trace<false, true, false>, k_trace<false, true, true>}},
+      {{k_trace<true, false, false>, k_trace<true, false, true>}, {k_trace<true, true, false>, k_trace<true, true, true>}}};
+  return t[stats ? 1 : 0][wt ? 1 : 0][trans ? 1 : 0];
+}
+
+using ShadeFn = void (*)(DevScene, DevSettings, WaveState, const uint32_t*, uint32_t*, uint32_t, DevCounters*);
+template <bool kP, bool kE>
+ShadeFn shade_fn_pe(bool sdf, bool exotic) {
+  static const ShadeFn t[2][2] = {{k_shade<kP, kE, false, false>, k_shade<kP, kE, false, true>},
+                                  {k_shade<kP, kE, true, false>, k_shade<kP, kE, true, true>}};
+  return t[sdf ? 1 : 0][exotic ? 1 : 0];
+}
+ShadeFn shade_fn(bool parity, bool effects, bool sdf, bool exotic) {
+  if (parity) return effects ? shade_fn_pe<true, true>(sdf, exotic) : shade_fn_pe<true, false>(sdf, exotic);
+  return effects ? shade_fn_pe<false, true>(sdf, exotic) : shade_fn_pe<false, false>(sdf, exotic);
+}
+
+}  // namespace
+
+// Per wave: raygen, then per depth one trace and one shade launch (the shadow
+// queries of a depth are traced with the next depth's extension rays; the last
+// depth queues none), then the film.  The launches a scene with SDF primitives
+// adds: its closest hits after the trace, its occlusion of the shadow queries
+// after the shading -- or, with transmissive materials, their whole loop there.
 cudaError_t LaunchWave(const DevScene& s, const DevSettings& st, const WaveState& w, const WaveTile& tile,
                        const Film& film, bool parity, bool stats, const LaunchShape& ls, DevCounters* ctr,
                        uint32_t* err, StageTimer* timer) {
   const size_t smem = StackSmemBytes(ls.block, ls.smem_entries);
   const size_t smem_full = StackSmemBytes(ls.block, ls.stack_cap);
+  const bool sdf = s.sdf_count != 0u, wt = s.watertight != 0u;
+  const bool trans_sdf = sdf && s.has_transmissive;   // shadow queries by k_shadow_transmissive
+  const TraceFn trace = trace_fn(stats, wt, s.has_transmissive && !sdf);
+  const ShadeFn shade = shade_fn(parity, s.has_effects, sdf, s.has_exotic || s.env_map != nullptr);
   StageTimer dummy;
   StageTimer& tm = timer ? *timer : dummy;
   tm.begin(0, ls.stream);
   if (parity) k_raygen<true><<<ls.grid, ls.block, 0, ls.stream>>>(s, st, w, tile);
   else k_raygen<false><<<ls.grid, ls.block, 0, ls.stream>>>(s, st, w, tile);
   tm.end(ls.stream);
-  uint32_t cur = 0u;
   for (uint32_t depth = 0; depth < st.max_depth; ++depth) {
-    tm.begin(1, ls.stream);
-#define VKPTC_EXT(S, W) \
-  k_extend<S, W><<<ls.grid, ls.block, smem, ls.stream>>>(s, w, cur, ls.smem_entries, ls.spill, ls.stack_cap, ls.steps, ctr, err)
-    if (s.watertight) {
-      if (stats) VKPTC_EXT(true, true);
-      else VKPTC_EXT(false, true);
-    } else {
-      if (stats) VKPTC_EXT(true, false);
-      else VKPTC_EXT(false, false);
+    const uint32_t* q = w.q[depth & 1u];
+    const bool queries = depth > 0u && st.enable_nee && !trans_sdf;   // the previous depth's shadow queries
+    auto run_trace = [&](uint32_t parts) {
+      trace<<<ls.grid, ls.block, smem, ls.stream>>>(s, w, q, depth, parts, ls.smem_entries, ls.spill, ls.stack_cap,
+                                                    ls.steps, ctr, err);
+    };
+    if (timer && queries) {   // stage timing separates the two kinds of query
+      tm.begin(3, ls.stream);
+      run_trace(2u);
+      tm.end(ls.stream);
     }
-#undef VKPTC_EXT
+    tm.begin(1, ls.stream);
+    run_trace(queries && !timer ? 3u : 1u);
+    if (sdf) k_sdf<<<ls.grid, ls.block, 0, ls.stream>>>(s, w, q, depth, ctr);
     tm.end(ls.stream);
     tm.begin(2, ls.stream);
-    if (s.has_effects) {
-      if (parity) k_shade<true, true><<<ls.grid, ls.block, 0, ls.stream>>>(s, st, w, cur, depth, ctr);
-      else k_shade<false, true><<<ls.grid, ls.block, 0, ls.stream>>>(s, st, w, cur, depth, ctr);
-    } else {
-      if (parity) k_shade<true, false><<<ls.grid, ls.block, 0, ls.stream>>>(s, st, w, cur, depth, ctr);
-      else k_shade<false, false><<<ls.grid, ls.block, 0, ls.stream>>>(s, st, w, cur, depth, ctr);
-    }
+    shade<<<ls.grid, ls.block, 0, ls.stream>>>(s, st, w, q, w.q[(depth & 1u) ^ 1u], depth, ctr);
     tm.end(ls.stream);
-    if (st.enable_nee) {
+    if (st.enable_nee && sdf) {
       tm.begin(3, ls.stream);
+      if (!trans_sdf) k_sdf_shadow<<<ls.grid, ls.block, 0, ls.stream>>>(s, w, depth, ctr);
 #define VKPTC_SHT(S, W) \
-  k_shadow_transmissive<S, W><<<ls.grid, ls.block, smem_full, ls.stream>>>(s, w, ls.stack_cap, ctr, err)
-#define VKPTC_SH(S, W) \
-  k_shadow<S, W><<<ls.grid, ls.block, smem, ls.stream>>>(s, w, ls.smem_entries, ls.spill, ls.stack_cap, ls.steps, ctr, err)
-      if (s.has_transmissive) {
-        if (s.watertight) {
-          if (stats) VKPTC_SHT(true, true);
-          else VKPTC_SHT(false, true);
-        } else {
-          if (stats) VKPTC_SHT(true, false);
-          else VKPTC_SHT(false, false);
-        }
-      } else {
-        if (s.watertight) {
-          if (stats) VKPTC_SH(true, true);
-          else VKPTC_SH(false, true);
-        } else {
-          if (stats) VKPTC_SH(true, false);
-          else VKPTC_SH(false, false);
-        }
-      }
-#undef VKPTC_SH
+  k_shadow_transmissive<S, W><<<ls.grid, ls.block, smem_full, ls.stream>>>(s, w, depth, ls.stack_cap, ctr, err)
+      else if (wt && stats) VKPTC_SHT(true, true);
+      else if (wt) VKPTC_SHT(false, true);
+      else if (stats) VKPTC_SHT(true, false);
+      else VKPTC_SHT(false, false);
 #undef VKPTC_SHT
       tm.end(ls.stream);
     }
-    cur ^= 1u;
   }
   tm.begin(4, ls.stream);
   k_accumulate<<<ls.grid, ls.block, 0, ls.stream>>>(st, w, tile, film, ctr);
@@ -617,10 +743,10 @@ cudaError_t ConfigureStackSmem(size_t bytes) {
     if (e == cudaSuccess) e = set_smem(k_trace_rays<true, false, W>, b);
     if (e == cudaSuccess) e = set_smem(k_trace_rays<false, true, W>, b);
     if (e == cudaSuccess) e = set_smem(k_trace_rays<false, false, W>, b);
-    if (e == cudaSuccess) e = set_smem(k_extend<true, W>, b);
-    if (e == cudaSuccess) e = set_smem(k_extend<false, W>, b);
-    if (e == cudaSuccess) e = set_smem(k_shadow<true, W>, b);
-    if (e == cudaSuccess) e = set_smem(k_shadow<false, W>, b);
+    if (e == cudaSuccess) e = set_smem(k_trace<true, W, false>, b);
+    if (e == cudaSuccess) e = set_smem(k_trace<true, W, true>, b);
+    if (e == cudaSuccess) e = set_smem(k_trace<false, W, false>, b);
+    if (e == cudaSuccess) e = set_smem(k_trace<false, W, true>, b);
     if (e == cudaSuccess) e = set_smem(k_shadow_transmissive<true, W>, b);
     if (e == cudaSuccess) e = set_smem(k_shadow_transmissive<false, W>, b);
   };
@@ -632,8 +758,8 @@ cudaError_t ConfigureStackSmem(size_t bytes) {
 int ExtendBlocksPerSm(int block, size_t smem, bool watertight) {
   int blocks = 0;
   const cudaError_t e = watertight
-      ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_extend<false, true>, block, smem)
-      : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_extend<false, false>, block, smem);
+      ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_trace<false, true, false>, block, smem)
+      : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_trace<false, false, false>, block, smem);
   if (e != cudaSuccess) return 1;
   return blocks > 0 ? blocks : 1;
 }

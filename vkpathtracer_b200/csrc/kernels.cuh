@@ -9,7 +9,7 @@ namespace vkptc {
 
 // Queue and path-state buffers of one wave (structure of arrays, indexed by
 // path slot).  A wave is `sample_count` samples of every pixel of one
-// rectangular tile: slot = sample_local * tile_pixels + pixel_local.
+// rectangular tile, in the order of wave_slot() (kernels.cu).
 struct WaveState {
   // path state
   uint64_t* rng;
@@ -23,8 +23,8 @@ struct WaveState {
   float4* sh_o;       // origin xyz, w = max distance
   float4* sh_d;       // direction xyz
   float4* sh_c;       // contribution to add when visible
-  // queues: q[0], q[1] ping-pong extension queues; counts[0..1] their sizes,
-  // counts[2] the shadow queue size
+  // queues: q[0], q[1] ping-pong extension queues; counts: their sizes, the
+  // shadow queue's and the stages' fetch counters (8 words, kernels.cu)
   uint32_t* q[2];
   uint32_t* counts;
   uint32_t capacity;
@@ -93,7 +93,7 @@ struct StageTimer {
   }
 };
 
-// One wave: raygen, max_depth x (extend, shade, shadow), accumulate.
+// One wave: raygen, max_depth x (trace, shade), accumulate.
 cudaError_t LaunchWave(const DevScene& s, const DevSettings& st, const WaveState& w, const WaveTile& tile,
                        const Film& film, bool parity, bool stats, const LaunchShape& ls, DevCounters* ctr,
                        uint32_t* err, StageTimer* timer);

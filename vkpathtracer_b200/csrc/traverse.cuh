@@ -394,6 +394,10 @@ __host__ __device__ __forceinline__ GeoView geo_of(const DevScene& s) {
   return GeoView{s.nodes, s.tris, s.tie, s.prim_count};
 }
 
+// What a kernel's queries ask for: the closest hit, any hit, or a mixture that
+// the source decides per query (Src::any(j)).
+constexpr int kQueryClosest = 0, kQueryAny = 1, kQueryMixed = 2;
+
 struct LaneState {
   RayPrep r;
   WtRay w;          // watertight test constants (unused by the Moller-Trumbore kernels)
@@ -401,13 +405,15 @@ struct LaneState {
   int32_t best;     // closest: triangle record of the best hit; any: 0 when occluded; -1: none
   int32_t ref;      // >= 0: wide node to visit; < 0: leaf, from its next triangle on
   int sp;
+  bool any;         // kQueryMixed: this query ends at its first hit
 };
 
-template <bool kAny, bool kWt>
+// tmax: hits at or beyond it do not count (infinity: no bound).
+template <bool kWt>
 __device__ __forceinline__ void lane_begin(LaneState& L, V3 o, V3 d, float tmax) {
   L.r = prep_ray(o, d);
   if constexpr (kWt) L.w = prep_wt(L.r);
-  L.t = kAny ? tmax : kInf;
+  L.t = tmax;
   L.best = -1;
   L.ref = 0;
   L.sp = 0;
@@ -429,7 +435,7 @@ __device__ __forceinline__ void lane_enter(LaneState& L, int32_t ref, TraceStats
 // branches per step gained 10 % on camera rays of a sparse scene and lost as
 // much on others.  tie() returns the scene's tie records.  Returns true when
 // the query has finished.
-template <bool kAny, bool kStats, bool kWt, class TieFn>
+template <int kMode, bool kStats, bool kWt, class TieFn>
 __device__ __forceinline__ bool lane_step(LaneState& L, const float4* nodes, const float4* tris, const TieFn& tie,
                                           const TwoLevelStack& stk, TraceStats& st, uint32_t& err) {
   if (L.ref < 0) {
@@ -437,13 +443,14 @@ __device__ __forceinline__ bool lane_step(LaneState& L, const float4* nodes, con
     const float4* tp = tris + 3u * (u >> 3);
     const float4 a = __ldg(tp), b = __ldg(tp + 1), cc = __ldg(tp + 2);
     const float th = tri_test<kWt>(a, b, cc, L.r, L.w);
-    if (th > kEps && (kAny ? th < L.t : th <= L.t) && leaf_rule_ok<kWt>(tie(), __float_as_uint(cc.z), L.r)) {
-      if (kAny) {
+    if (th > kEps && (kMode == kQueryAny ? th < L.t : th <= L.t) &&
+        leaf_rule_ok<kWt>(tie(), __float_as_uint(cc.z), L.r)) {
+      if (kMode == kQueryAny) {
         L.best = 0;
         return true;
       }
       bool take = th < L.t;
-      if (!take && L.best >= 0) {   // L.best < 0: only th == inf == L.t, which is no hit
+      if (!take && L.best >= 0) {   // L.best < 0: th is the query's bound, which is no hit
         const float4 ic = __ldg(tris + 3u * static_cast<uint32_t>(L.best) + 2);
         take = tie_candidate_wins(tie(), L.r, parallel_eps<kWt>(), __float_as_uint(ic.z), __float_as_uint(ic.w),
                                   __float_as_uint(cc.z), __float_as_uint(cc.w));
@@ -451,6 +458,7 @@ __device__ __forceinline__ bool lane_step(LaneState& L, const float4* nodes, con
       if (take) {
         L.t = th;
         L.best = static_cast<int32_t>(u >> 3);
+        if (kMode == kQueryMixed && L.any) return true;
       }
     }
     if (u & 7u) {
@@ -509,7 +517,7 @@ __device__ __forceinline__ bool lane_step(LaneState& L, const float4* nodes, con
   while (L.sp > 0) {
     --L.sp;
     const int2 e = stk.get(L.sp);
-    if (kAny || __int_as_float(e.y) <= L.t) {
+    if (kMode == kQueryAny || __int_as_float(e.y) <= L.t) {
       lane_enter<kStats>(L, e.x, st);
       return false;
     }
@@ -527,9 +535,9 @@ __device__ __forceinline__ void trace_closest(const DevScene& s, V3 o, V3 d, con
   best_prim = kMiss;
   if (s.prim_count == 0u) return;
   LaneState L;
-  lane_begin<false, kWt>(L, o, d, kInf);
+  lane_begin<kWt>(L, o, d, kInf);
   const auto tie = [&]() { return s.tie; };
-  while (!lane_step<false, kStats, kWt>(L, s.nodes, s.tris, tie, stk, st, err)) {
+  while (!lane_step<kQueryClosest, kStats, kWt>(L, s.nodes, s.tris, tie, stk, st, err)) {
   }
   best_t = L.t;
   if (L.best >= 0) best_prim = __float_as_uint(__ldg(s.tris + 3u * static_cast<uint32_t>(L.best) + 2).y);
@@ -541,9 +549,9 @@ __device__ __forceinline__ bool trace_any(const DevScene& s, V3 o, V3 d, float t
                                           TraceStats& st, uint32_t& err) {
   if (s.prim_count == 0u || !(tmax > kEps)) return false;
   LaneState L;
-  lane_begin<true, kWt>(L, o, d, tmax);
+  lane_begin<kWt>(L, o, d, tmax);
   const auto tie = [&]() { return s.tie; };
-  while (!lane_step<true, kStats, kWt>(L, s.nodes, s.tris, tie, stk, st, err)) {
+  while (!lane_step<kQueryAny, kStats, kWt>(L, s.nodes, s.tris, tie, stk, st, err)) {
   }
   return L.best >= 0;
 }
@@ -554,16 +562,20 @@ __device__ __forceinline__ bool trace_any(const DevScene& s, V3 o, V3 d, float t
 //   Src::kUniform: one scene serves the whole launch (its pointers then stay in
 //   uniform registers), and Src::geo_at(j): query j's scene, for the rare reads
 //   of the tie records.
+// kQueryMixed: Src::any(j) says whether query j ends at its first hit, and
+// Src::finish(j, t, prim, o, d, tmax) may return true to go on with a new
+// origin and bound (o and tmax updated) as the same query.
 // Each warp keeps its lanes busy: whenever lanes are idle it claims that many
 // query ids with one atomic (warp-aggregated) and refills them.  `steps`
 // packs two limits: the low 16 bits are the most traversal steps between
 // refills; the high bits, when non-zero, a refill threshold -- the warp
 // leaves the step loop for a refill as soon as that many lanes are idle
 // (checked after every step).  Without a threshold the lanes run the full
-// number of steps between refills.
-template <class Src, bool kAny, bool kStats, bool kWt = false>
-__device__ __forceinline__ void persistent_traverse(const Src& src, uint32_t n, uint32_t* fetch,
-                                                    TwoLevelStack stk, int steps, TraceStats& st, uint32_t& err) {
+// number of steps between refills.  st: the work of closest-hit queries, st_any
+// that of any-hit queries (the same object where a launch has one kind).
+template <class Src, int kMode, bool kStats, bool kWt = false>
+__device__ __forceinline__ void persistent_traverse(const Src& src, uint32_t n, uint32_t* fetch, TwoLevelStack stk,
+                                                    int steps, TraceStats& st, TraceStats& st_any, uint32_t& err) {
   const unsigned lane_id = threadIdx.x & 31u;
   const int max_steps = steps & 0xFFFF;
   const int refill_min = steps >> 16;
@@ -578,11 +590,31 @@ __device__ __forceinline__ void persistent_traverse(const Src& src, uint32_t n, 
   bool exhausted = false;
   uint32_t tag = 0u;
   const auto tie = [&]() { return src.geo_at(tag).tie; };
-  const auto finish = [&](uint32_t j, const LaneState& l) {
-    uint32_t prim = kAny ? 0u : kMiss;
-    if (l.best >= 0) prim = kAny ? 1u : __float_as_uint(__ldg(tris + 3u * static_cast<uint32_t>(l.best) + 2).y);
-    src.finish(j, l.t, prim);
-    if (kStats) ++st.rays;
+  // The end of query j: its result stored, or (mixed) the lane restarted.
+  // Returns true when the query goes on.
+  const auto finish = [&](uint32_t j, LaneState& l) {
+    const bool any = kMode == kQueryAny || (kMode == kQueryMixed && l.any);
+    uint32_t prim = any ? 0u : kMiss;
+    if (l.best >= 0) prim = any ? 1u : __float_as_uint(__ldg(tris + 3u * static_cast<uint32_t>(l.best) + 2).y);
+    if constexpr (kMode == kQueryMixed) {
+      V3 o = mk(l.r.ox, l.r.oy, l.r.oz);
+      const V3 d = mk(l.r.dx, l.r.dy, l.r.dz);
+      float tmax;
+      if (src.finish(j, l.t, prim, o, d, tmax)) {
+        lane_begin<kWt>(l, o, d, tmax);
+        return true;
+      }
+    } else {
+      src.finish(j, l.t, prim);
+    }
+    if (kStats) ++(any ? st_any : st).rays;
+    return false;
+  };
+  const auto step = [&](LaneState& l) {
+    if constexpr (kStats && kMode == kQueryMixed) {
+      if (src.shadow(tag)) return lane_step<kMode, kStats, kWt>(l, nodes, tris, tie, stk, st_any, err);
+    }
+    return lane_step<kMode, kStats, kWt>(l, nodes, tris, tie, stk, st, err);
   };
   while (true) {
     const unsigned idle = __ballot_sync(0xffffffffu, !active);
@@ -602,8 +634,9 @@ __device__ __forceinline__ void persistent_traverse(const Src& src, uint32_t n, 
             nodes = g.nodes;
             tris = g.tris;
           }
-          lane_begin<kAny, kWt>(L, o, d, tmax);
-          if (g.prim_count == 0u || (kAny && !(tmax > kEps))) {
+          if constexpr (kMode == kQueryMixed) L.any = src.any(j);
+          lane_begin<kWt>(L, o, d, kMode == kQueryClosest ? kInf : tmax);
+          if (g.prim_count == 0u || (kMode != kQueryClosest && !(tmax > kEps))) {
             finish(j, L);
           } else {
             tag = j;
@@ -616,8 +649,7 @@ __device__ __forceinline__ void persistent_traverse(const Src& src, uint32_t n, 
     if (refill_min == 0) {
       if (active) {
         for (int k = 0; k < max_steps; ++k) {
-          if (lane_step<kAny, kStats, kWt>(L, nodes, tris, tie, stk, st, err)) {
-            finish(tag, L);
+          if (step(L) && !finish(tag, L)) {
             active = false;
             break;
           }
@@ -625,10 +657,7 @@ __device__ __forceinline__ void persistent_traverse(const Src& src, uint32_t n, 
       }
     } else {
       for (int k = 0; k < max_steps; ++k) {
-        if (active && lane_step<kAny, kStats, kWt>(L, nodes, tris, tie, stk, st, err)) {
-          finish(tag, L);
-          active = false;
-        }
+        if (active && step(L) && !finish(tag, L)) active = false;
         const unsigned idle_now = __ballot_sync(0xffffffffu, !active);
         if (idle_now == 0xffffffffu || (!exhausted && __popc(idle_now) >= refill_min)) break;
       }
