@@ -15,6 +15,7 @@
 // grouped by material, butterfly sums) into per-warp shared-memory slots,
 // then per-block partials, then a fixed-order FP64 reduction: the gradient is
 // deterministic for a given launch shape.
+#define VKPTC_INLINE_UNIT 1   // common.cuh
 #include "adjoint.cuh"
 #include <algorithm>
 

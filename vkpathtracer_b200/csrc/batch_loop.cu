@@ -300,12 +300,10 @@ __global__ void __launch_bounds__(256) k_lp_sdf_shadow(const DevJob* __restrict_
 // stage takes their hits); without, the shading code carries no SDF steps.
 // kExotic: some job has a transmissive, clear-coat, sheen or toon material or
 // an environment map; without, those branches are compiled out.
-#ifndef VKPTC_LEAN_SHADE_BLOCKS
-#define VKPTC_LEAN_SHADE_BLOCKS 3
-#endif
+// 80 registers: the 64-job step takes 522 ms, 526 at 64 registers, 538 at 48.
 template <bool kParity, bool kEffects, bool kSdf, bool kExotic>
-__global__ void __launch_bounds__(256, (kEffects || kSdf || kExotic) ? 3 : VKPTC_LEAN_SHADE_BLOCKS) k_lp_shade(const DevJob* __restrict__ jobs, LoopPool P, DevCounters* ctr,
-                                                  uint32_t sdf_staged) {
+__global__ void __launch_bounds__(256, 3) k_lp_shade(const DevJob* __restrict__ jobs, LoopPool P,
+                                                     DevCounters* ctr) {
   const uint32_t cur = P.ctl[kLCur];
   const uint32_t n = P.ctl[kLCount0 + cur];
   const PathSoA A = P.gen[cur], B = P.gen[cur ^ 1u];
@@ -330,9 +328,8 @@ __global__ void __launch_bounds__(256, (kEffects || kSdf || kExotic) ? 3 : VKPTC
       pr.rad = mk(r4.x, r4.y, r4.z);
       pr.segs = r4.w;
       pr.rng = A.rng[j];
-      R = shade_bounce<kParity, kEffects, kSdf, kExotic>(J.scene, J.settings, J.scene.lights, depth, pr, h2.x,
-                                                         __float_as_uint(h2.y),
-                                          sdf_staged != 0u);
+      R = shade_bounce<kParity, kEffects, kSdf, kExotic, true>(J.scene, J.settings, J.scene.lights, depth, pr, h2.x,
+                                                               __float_as_uint(h2.y));
       next = R.next;
       fin = !R.next;
       shadow = R.shadow;
@@ -464,7 +461,7 @@ LoopTraceFn shadow_fn(bool stats, int occ, bool wt) {
 }
 
 // Shading stage variants: [parity][effects][sdf][exotic].
-using LoopShadeFn = void (*)(const DevJob*, LoopPool, DevCounters*, uint32_t);
+using LoopShadeFn = void (*)(const DevJob*, LoopPool, DevCounters*);
 template <bool kP, bool kE>
 LoopShadeFn shade_fn_pe(bool sdf, bool exotic) {
   static const LoopShadeFn t[2][2] = {{k_lp_shade<kP, kE, false, false>, k_lp_shade<kP, kE, false, true>},
@@ -545,8 +542,7 @@ cudaError_t LaunchBatchLoopIteration(const DevJob* jobs, uint32_t job_count, uns
   mark(3);
   k_lp_drain<<<g.finish, bl.block, 0, s>>>(jobs, P);
   mark(4);
-  const uint32_t staged = bl.sdf ? 1u : 0u;
-  shade_fn(bl.parity, bl.effects, bl.sdf, bl.exotic)<<<g.shade, bl.block, 0, s>>>(jobs, P, ctr, staged);
+  shade_fn(bl.parity, bl.effects, bl.sdf, bl.exotic)<<<g.shade, bl.block, 0, s>>>(jobs, P, ctr);
   mark(5);
   k_lp_decide<<<1, 32, 0, s>>>(total, P, handle);
   return cudaGetLastError();

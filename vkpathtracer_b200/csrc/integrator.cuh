@@ -406,15 +406,15 @@ struct ShadeOut {
 // sheen and toon branches and the environment-map lookup (for launches whose
 // scenes have none: the host classifies the material tables with the same
 // tests), which keeps the shading kernel's hot code compact.
-// sdf_staged: a load-balanced stage has already folded the SDF hits into
-// (ht, prim) and tests the shadow queries itself (the loop driver).
-template <bool kParity, bool kEffects = true, bool kSdf = true, bool kExotic = true>
+// kStaged: load-balanced stages have already folded the SDF hits into (ht, prim)
+// and test the shadow queries (the wavefront and the loop driver); the marches
+// are then compiled out too.
+template <bool kParity, bool kEffects = true, bool kSdf = true, bool kExotic = true, bool kStaged = false>
 __device__ __forceinline__ ShadeOut shade_bounce(const DevScene& s, const DevSettings& st, const float* lights,
-                                               uint32_t depth, PathRegs& P, float ht, uint32_t prim,
-                                               bool sdf_staged = false) {
+                                               uint32_t depth, PathRegs& P, float ht, uint32_t prim) {
   ShadeOut R;
-  if constexpr (kSdf) {
-    if (s.sdf_count != 0u && !sdf_staged) sdf_closest(s.sdf, s.sdf_count, P.o, P.d, ht, prim, R.sdf);
+  if constexpr (kSdf && !kStaged) {
+    if (s.sdf_count != 0u) sdf_closest(s.sdf, s.sdf_count, P.o, P.d, ht, prim, R.sdf);
   }
   R.next = false;
   R.shadow = false;
@@ -478,7 +478,7 @@ __device__ __forceinline__ ShadeOut shade_bounce(const DevScene& s, const DevSet
           c = mulv(thr, nq.radiance);
         }
         if (nq.remain > 0.004f) {
-          R.shadow = !(kSdf && s.sdf_count != 0u && !s.has_transmissive && !sdf_staged &&
+          R.shadow = !(kSdf && !kStaged && s.sdf_count != 0u && !s.has_transmissive &&
                        sdf_any(s.sdf, s.sdf_count, nq.origin, nq.dir, nq.remain, R.sdf));
           R.sh_o = nq.origin;
           R.sh_d = nq.dir;

@@ -146,9 +146,25 @@ __device__ __forceinline__ float sdf_distance(const SdfPrim& p, V3 world) {
 // sdf_normal: central differences with e = 5e-4, normalised.
 static __device__ __noinline__ V3 sdf_march_normal(const SdfPrim& p, V3 w) {
   const float e = 0.0005f;
-  const float dx = sdf_distance(p, add(w, mk(e, 0.0f, 0.0f))) - sdf_distance(p, sub(w, mk(e, 0.0f, 0.0f)));
-  const float dy = sdf_distance(p, add(w, mk(0.0f, e, 0.0f))) - sdf_distance(p, sub(w, mk(0.0f, e, 0.0f)));
-  const float dz = sdf_distance(p, add(w, mk(0.0f, 0.0f, e))) - sdf_distance(p, sub(w, mk(0.0f, 0.0f, e)));
+  // One copy of the distance code for the six evaluations: with six, the shading
+  // stage of an SDF scene waited on instruction fetch for 19 of every 26 cycles
+  // (frame 4.67 -> 4.28 ms).  -1 * 0 keeps the zero signs of a subtraction.
+  float dx = 0.0f, dy = 0.0f, dz = 0.0f, plus = 0.0f;
+#pragma unroll 1
+  for (int k = 0; k < 6; ++k) {
+    const int a = k >> 1;
+    const float sg = (k & 1) ? -1.0f : 1.0f;
+    const float dist = sdf_distance(p, add(w, mk(sg * (a == 0 ? e : 0.0f), sg * (a == 1 ? e : 0.0f),
+                                                 sg * (a == 2 ? e : 0.0f))));
+    if (k & 1) {
+      const float g = plus - dist;
+      if (a == 0) dx = g;
+      else if (a == 1) dy = g;
+      else dz = g;
+    } else {
+      plus = dist;
+    }
+  }
   return unit(mul(mk(dx, dy, dz), 0.5f));
 }
 
