@@ -147,3 +147,21 @@ def test_sah_trees_at_subtree_and_chunk_edges(n_lat, n_lon):
             rec = t.read_accel(native.ACCEL_TRIANGLES).reshape(-1, 12)
         assert np.array_equal(np.sort(rec[:, 9]), np.arange(sc.indices.shape[0]))
         assert np.array_equal(p, rp) and np.array_equal(tt.view(np.uint32), rt.view(np.uint32))
+
+
+@pytest.mark.parametrize("block_size", [0, 32, 256])
+@pytest.mark.parametrize("extra", [-1, 0, 1, 33])
+def test_ray_counts_around_one_per_thread(extra, block_size):
+    """Calls of at most one ray per resident thread are spread over the warps
+    without a query counter; the count where that ends depends on the device, so
+    counts around every multiple of its threads per block and SM are tried."""
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    sc = scenes.cornell_box(seed=4)
+    n = sms * 1024 + extra
+    rays = probe_rays(sc, n, 9)
+    rp, rt, _, _ = oracle.load("port").intersect(sc, rays, threads=8)
+    with tracer(sc, block_size=block_size) as t:
+        for k in (n, sms * 32 + extra, 5 * sms + extra):
+            p, tt = t.trace_rays(rays[:k])
+            assert np.array_equal(p, rp[:k]) and np.array_equal(tt.view(np.uint32), rt[:k].view(np.uint32))

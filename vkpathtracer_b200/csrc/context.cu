@@ -221,6 +221,9 @@ struct vkptc_ctx {
   DevBuf<uint32_t> w_q0, w_q1, w_sh_path, w_counts;
   uint32_t wave_capacity = 0;
   size_t smem_configured = 48 * 1024;
+  int max_smem_optin = 0;                 // the device's shared-memory limit per block
+  int shape_block = 0, shape_per_sm = 0;  // resident blocks per SM of the last launch shape
+  size_t shape_smem = 0;
 
   // counters, error word, fetch counter of the ray-query kernel, stack spill
   DevBuf<DevCounters> d_ctr;
@@ -368,8 +371,12 @@ int32_t launch_shape(vkptc_ctx* c, cudaStream_t stream, LaunchShape& ls, bool al
   const int32_t rc = ensure_stack_smem(c, ls);
   if (rc != VKPTC_OK) return rc;
   const size_t smem = StackSmemBytes(ls.block, ls.smem_entries);
-  const int per_sm = ExtendBlocksPerSm(ls.block, smem, c->config.triangle_test == VKPTC_TRIANGLE_WATERTIGHT);
-  ls.grid = c->sm_count * per_sm;
+  if (c->shape_block != ls.block || c->shape_smem != smem) {   // the occupancy query, once per shape
+    c->shape_per_sm = ExtendBlocksPerSm(ls.block, smem, c->config.triangle_test == VKPTC_TRIANGLE_WATERTIGHT);
+    c->shape_block = ls.block;
+    c->shape_smem = smem;
+  }
+  ls.grid = c->sm_count * c->shape_per_sm;
   const size_t spill = SpillEntries(ls);
   if (spill > 0) {
     if (c->d_spill.count < spill) VKPTC_CUDA(c, c->d_spill.alloc(spill), "stack spill alloc");
@@ -383,9 +390,7 @@ int32_t ensure_stack_smem(vkptc_ctx* c, const LaunchShape& ls) {
   // The transmissive shadow kernel keeps its whole stack in shared memory.
   const size_t smem_full = c->has_transmissive ? StackSmemBytes(ls.block, ls.stack_cap) : smem;
   const size_t need = std::max(smem, smem_full);
-  int max_optin = 0;
-  cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
-  if (need > static_cast<size_t>(max_optin)) {
+  if (need > static_cast<size_t>(c->max_smem_optin)) {
     return fail(c, VKPTC_UNSUPPORTED, "traversal stack does not fit in shared memory (BVH too deep for this block size)");
   }
   if (need > c->smem_configured) {
@@ -629,6 +634,7 @@ int32_t vkptc_create(const vkptc_config* config, vkptc_ctx** out_ctx) {
     c->timer.capacity = 4096;
   }
   cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, c->device);
+  cudaDeviceGetAttribute(&c->max_smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
   if (c->d_ctr.alloc(1) != cudaSuccess || c->d_err.alloc(1) != cudaSuccess || c->d_fetch.alloc(1) != cudaSuccess ||
       cudaMemset(c->d_ctr.ptr, 0, sizeof(DevCounters)) != cudaSuccess ||
       cudaMemset(c->d_err.ptr, 0, sizeof(uint32_t)) != cudaSuccess) {
@@ -1569,11 +1575,10 @@ int32_t vkptc_resolve_hdr(vkptc_ctx* ctx, float* rgb) {
   if (!rgb) return fail(ctx, VKPTC_INVALID_ARGUMENT, "rgb is null");
   cudaSetDevice(ctx->device);
   const size_t px = static_cast<size_t>(ctx->settings.width) * ctx->settings.height;
-  float* d_rgb = nullptr;
-  VKPTC_CUDA(ctx, cudaMallocAsync(reinterpret_cast<void**>(&d_rgb), std::max<size_t>(1, 3 * px) * sizeof(float), ctx->stream), "resolve alloc");
-  cudaError_t e = LaunchResolveHdr(film_of(ctx), d_rgb, ctx->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(rgb, d_rgb, 3 * px * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream);
-  cudaFreeAsync(d_rgb, ctx->stream);
+  VKPTC_CUDA(ctx, ctx->d_pack.alloc(std::max<size_t>(1, 3 * px)), "resolve alloc");
+  cudaError_t e = LaunchResolveHdr(film_of(ctx), ctx->d_pack.ptr, ctx->stream);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(rgb, ctx->d_pack.ptr, 3 * px * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "resolve");
   return VKPTC_OK;

@@ -195,8 +195,9 @@ __device__ __forceinline__ TwoLevelStack launch_stack(int2* smem_stack, int scap
 // grid took 37.2 ms instead of 30.7.
 // =============================================================== ray queries
 template <bool kAny, bool kStats, bool kWt>
-__global__ void __launch_bounds__(256, 4) k_trace_rays(DevScene s, RaysSource src, uint32_t n, uint32_t* fetch, int scap,
-                                                    int2* spill, int total, int steps, DevCounters* ctr, uint32_t* err) {
+__global__ void __launch_bounds__(256, 4) k_trace_rays(DevScene s, RaysSource src, uint32_t n, uint32_t* fetch,
+                                                       int scap, int2* spill, int total, int steps, DevCounters* ctr,
+                                                       uint32_t* err) {
   extern __shared__ int2 smem_stack[];
   TraceStats st;
   uint32_t lerr = 0u;
@@ -216,12 +217,22 @@ cudaError_t LaunchTraceRays(const DevScene& s, const float* rays, const float* t
                             uint32_t* err, uint32_t* fetch) {
   if (n == 0) return cudaSuccess;
   const size_t smem = StackSmemBytes(ls.block, ls.smem_entries);
-  cudaError_t e = cudaMemsetAsync(fetch, 0, sizeof(uint32_t), ls.stream);
-  if (e != cudaSuccess) return e;
   const RaysSource src{geo_of(s), rays, tmax, prim_out, t_out, any_hit};
   const uint32_t n32 = static_cast<uint32_t>(n);
+  // At most one ray per resident thread: the kernel spreads them over its warps
+  // without the query counter, so there is none to clear, and warps that would
+  // get nothing are not launched.
+  const uint32_t per_block = static_cast<uint32_t>(ls.block) / 32u;
+  uint32_t grid = static_cast<uint32_t>(ls.grid);
+  if (n <= 32ull * grid * per_block) {
+    const uint32_t share = (n32 + grid * per_block - 1u) / (grid * per_block);
+    grid = ((n32 + share - 1u) / share + per_block - 1u) / per_block;
+  } else {
+    const cudaError_t e = cudaMemsetAsync(fetch, 0, sizeof(uint32_t), ls.stream);
+    if (e != cudaSuccess) return e;
+  }
 #define VKPTC_TR(A, S, W) \
-  k_trace_rays<A, S, W><<<ls.grid, ls.block, smem, ls.stream>>>(s, src, n32, fetch, ls.smem_entries, ls.spill, ls.stack_cap, ls.steps, ctr, err)
+  k_trace_rays<A, S, W><<<grid, ls.block, smem, ls.stream>>>(s, src, n32, fetch, ls.smem_entries, ls.spill, ls.stack_cap, ls.steps, ctr, err)
 #define VKPTC_TR2(A, S) \
   if (s.watertight) VKPTC_TR(A, S, true); \
   else VKPTC_TR(A, S, false)

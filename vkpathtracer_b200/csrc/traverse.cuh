@@ -571,7 +571,12 @@ __device__ __forceinline__ bool trace_any(const DevScene& s, V3 o, V3 d, float t
 // refills; the high bits, when non-zero, a refill threshold -- the warp
 // leaves the step loop for a refill as soon as that many lanes are idle
 // (checked after every step).  Without a threshold the lanes run the full
-// number of steps between refills.  st: the work of closest-hit queries, st_any
+// number of steps between refills.  At most one query per thread of the launch:
+// no counter is needed (fetch may be null); the queries are spread evenly over
+// all warps, because a warp takes as long as its lanes' divergent steps together
+// (1,000 rays on the 130k-triangle field, queries and clearing of the counter:
+// 46 us in full warps with the counter, 38 us in full warps without, 18.5 us
+// spread).  st: the work of closest-hit queries, st_any
 // that of any-hit queries (the same object where a launch has one kind).
 template <class Src, int kMode, bool kStats, bool kWt = false>
 __device__ __forceinline__ void persistent_traverse(const Src& src, uint32_t n, uint32_t* fetch, TwoLevelStack stk,
@@ -579,6 +584,8 @@ __device__ __forceinline__ void persistent_traverse(const Src& src, uint32_t n, 
   const unsigned lane_id = threadIdx.x & 31u;
   const int max_steps = steps & 0xFFFF;
   const int refill_min = steps >> 16;
+  const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+  const bool spread = n <= 32u * warps;
   LaneState L;
   const float4* nodes = nullptr;
   const float4* tris = nullptr;
@@ -619,13 +626,20 @@ __device__ __forceinline__ void persistent_traverse(const Src& src, uint32_t n, 
   while (true) {
     const unsigned idle = __ballot_sync(0xffffffffu, !active);
     if (idle != 0u && !exhausted) {
-      uint32_t base = 0u;
-      if (lane_id == 0u) base = atomicAdd(fetch, static_cast<uint32_t>(__popc(idle)));
-      base = __shfl_sync(0xffffffffu, base, 0);
-      if (base >= n) exhausted = true;
+      uint32_t base = 0u, limit = n;
+      if (!spread) {
+        if (lane_id == 0u) base = atomicAdd(fetch, static_cast<uint32_t>(__popc(idle)));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (base >= n) exhausted = true;
+      } else {
+        const uint32_t share = (n + warps - 1u) / warps;
+        base = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * share;
+        limit = min(n, base + share);
+        exhausted = true;
+      }
       if (!active) {
         const uint32_t j = base + static_cast<uint32_t>(__popc(idle & ((1u << lane_id) - 1u)));
-        if (j < n && j >= base) {
+        if (j < limit && j >= base) {
           V3 o, d;
           float tmax;
           GeoView g;
