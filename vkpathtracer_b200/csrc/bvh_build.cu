@@ -20,9 +20,9 @@
 //      internal-node count of the left subtree when coming from the right;
 //   3. optionally a binned-SAH traversal tree (32 bins per axis) with the same
 //      machinery;
-//   4. the wide collapse of the traversal tree (CollapseToWide's greedy
-//      largest-area opening, wide nodes in depth-first pre-order, found the
-//      same way), triangle records in leaf order and the tie records of the
+//   4. the wide collapse of the traversal tree (CollapseToWide's choice of the
+//      cheapest four subtrees per wide node, wide nodes in depth-first pre-order,
+//      found the same way), triangle records in leaf order and the tie records of the
 //      reference tree.
 // Every array equals the host path's bit for bit (tested).  A non-finite
 // vertex, edge or bound sends the build back to the host path (min/max of NaN
@@ -368,19 +368,15 @@ __device__ __forceinline__ uint32_t level_active(const BuildArrays& A) { return 
 __device__ __forceinline__ uint32_t grid_thread() { return blockIdx.x * blockDim.x + threadIdx.x; }
 __device__ __forceinline__ uint32_t grid_threads() { return gridDim.x * blockDim.x; }
 
-__global__ void k_level_init(BuildArrays A, const uint32_t* __restrict__ act) {
-  const uint32_t n_act = level_active(A);
-  for (uint32_t s = grid_thread(); s < n_act; s += grid_threads()) {
-    A.slot_of[act[s]] = static_cast<int32_t>(s);
-    uint32_t* k = A.cb + 6 * s;
-    k[0] = k[1] = k[2] = 0xffffffffu;   // min keys
-    k[3] = k[4] = k[5] = 0u;            // max keys
-  }
+// A node becomes active in slot s of a level.
+__device__ __forceinline__ void activate(const BuildArrays& A, uint32_t nd, uint32_t s) {
+  A.slot_of[nd] = static_cast<int32_t>(s);
+  uint32_t* k = A.cb + 6 * s;
+  k[0] = k[1] = k[2] = 0xffffffffu;   // min keys
+  k[3] = k[4] = k[5] = 0u;            // max keys
 }
-
-__global__ void k_level_done(BuildArrays A, const uint32_t* __restrict__ act) {
-  const uint32_t n_act = level_active(A);
-  for (uint32_t s = grid_thread(); s < n_act; s += grid_threads()) A.slot_of[act[s]] = -1;
+__global__ void k_level_init(BuildArrays A, const uint32_t* __restrict__ act) {   // the first level: the root or nothing
+  if (level_active(A) != 0u) activate(A, act[0], 0u);
 }
 
 // End of a level: the children ids advance past this level's children, the
@@ -389,13 +385,6 @@ __global__ void k_level_advance(BuildArrays A) {
   A.counter[5] += 2u * A.counter[4];
   A.counter[4] = A.counter[1];
   A.counter[1] = 0u;
-}
-
-// The scattered order of a level becomes the current one (skipped when the
-// level had no active node: its scatter wrote nothing).
-__global__ void k_copy_level(BuildArrays A, uint32_t* __restrict__ dst, const uint32_t* __restrict__ src, uint32_t n) {
-  if (level_active(A) == 0u) return;
-  for (uint32_t i = grid_thread(); i < n; i += grid_threads()) dst[i] = src[i];
 }
 
 // After the last level: temporary ids of the small subtrees start after the levels' nodes.
@@ -506,25 +495,91 @@ __device__ __forceinline__ bool goes_left(const BuildArrays& A, uint32_t p, int3
   return bin <= static_cast<int>(__float_as_uint(A.split[s]));
 }
 
-__global__ void k_flags(BuildArrays A, const uint32_t* __restrict__ idx, const uint32_t* __restrict__ node_of,
-                        uint32_t n, uint32_t* __restrict__ flag, bool sah) {
+// Left flags of a level and their exclusive scan within blocks of kScanBlock
+// positions: loc[pos] = rank in the block, the flag in the top bit; sums[block] =
+// the block's count.  n + 1 entries, so the rank at n exists.
+__global__ void __launch_bounds__(kScanThreads) k_flag_scan(BuildArrays A, const uint32_t* __restrict__ idx,
+                                                            const uint32_t* __restrict__ node_of, uint32_t n, bool sah,
+                                                            uint32_t* __restrict__ loc, uint32_t* __restrict__ sums) {
   if (level_active(A) == 0u) return;
-  const uint32_t pos = blockIdx.x * blockDim.x + threadIdx.x;
-  if (pos >= n) return;
-  const int32_t s = A.slot_of[node_of[pos]];
-  flag[pos] = (s >= 0 && goes_left(A, idx[pos], s, sah)) ? 1u : 0u;
+  __shared__ uint32_t warp_tot[kScanThreads / 32];
+  const uint32_t i0 = blockIdx.x * kScanBlock + 2u * threadIdx.x;
+  uint32_t f[2];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const uint32_t pos = i0 + static_cast<uint32_t>(k);
+    f[k] = 0u;
+    if (pos < n) {
+      const int32_t s = A.slot_of[node_of[pos]];
+      f[k] = s >= 0 && goes_left(A, idx[pos], s, sah) ? 1u : 0u;
+    }
+  }
+  const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  uint32_t x = f[0] + f[1];
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (static_cast<int>(lane) >= o) x += y;
+  }
+  if (lane == 31u) warp_tot[warp] = x;
+  __syncthreads();
+  uint32_t off = 0u;
+  for (unsigned w = 0; w < warp; ++w) off += warp_tot[w];
+  const uint32_t excl = off + x - f[0] - f[1];
+  if (i0 <= n) loc[i0] = excl | (f[0] << 31);
+  if (i0 + 1u <= n) loc[i0 + 1u] = (excl + f[0]) | (f[1] << 31);
+  if (threadIdx.x == kScanThreads - 1) sums[blockIdx.x] = off + x;
 }
+
+// Exclusive scan of the block counts, in place, by one block.
+__global__ void __launch_bounds__(1024) k_scan_sums(BuildArrays A, uint32_t* __restrict__ sums, uint32_t blocks) {
+  if (level_active(A) == 0u) return;
+  __shared__ uint32_t warp_tot[32];
+  const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  uint32_t carry = 0u;
+  for (uint32_t base = 0u; base < blocks; base += 1024u) {
+    const uint32_t i = base + threadIdx.x;
+    const uint32_t v = i < blocks ? sums[i] : 0u;
+    uint32_t x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+      if (static_cast<int>(lane) >= o) x += y;
+    }
+    if (lane == 31u) warp_tot[warp] = x;
+    __syncthreads();
+    uint32_t t = warp_tot[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, t, o);
+      if (static_cast<int>(lane) >= o) t += y;
+    }
+    const uint32_t off = warp ? __shfl_sync(0xffffffffu, t, static_cast<int>(warp) - 1) : 0u;
+    if (i < blocks) sums[i] = carry + off + x - v;
+    carry += __shfl_sync(0xffffffffu, t, 31);
+    __syncthreads();   // warp_tot is rewritten
+  }
+}
+
+struct LevelRank {   // left flags before a position
+  const uint32_t* loc;
+  const uint32_t* sums;
+  __device__ __forceinline__ uint32_t at(uint32_t pos) const {
+    return (loc[pos] & 0x7fffffffu) + sums[pos / kScanBlock];
+  }
+  __device__ __forceinline__ bool flag(uint32_t pos) const { return (loc[pos] >> 31) != 0u; }
+};
 
 // Children of every active node; big ones go to the next level's list, small
 // ones to the subtree list, leaves nowhere.
-__global__ void k_children(BuildArrays A, const uint32_t* __restrict__ act, const uint32_t* __restrict__ excl,
+__global__ void k_children(BuildArrays A, const uint32_t* __restrict__ act, LevelRank rank,
                            uint32_t* __restrict__ next_act, uint32_t* __restrict__ small) {
   const uint32_t n_act = level_active(A), base = A.counter[5];
   for (uint32_t s = grid_thread(); s < n_act; s += grid_threads()) {
   const uint32_t nd = act[s];
   TNode& t = A.nodes[nd];
   const uint32_t b = static_cast<uint32_t>(t.begin), n = static_cast<uint32_t>(t.count);
-  uint32_t nl = excl[b + n] - excl[b];
+  uint32_t nl = rank.at(b + n) - rank.at(b);
   const bool ident = nl == 0u || nl == n;
   if (ident) nl = n / 2u;
   A.nl[s] = nl;
@@ -538,16 +593,17 @@ __global__ void k_children(BuildArrays A, const uint32_t* __restrict__ act, cons
     A.nodes[id[c]] = TNode{static_cast<int32_t>(c == 0 ? b : b + nl), static_cast<int32_t>(cnt[c]), -1, -1,
                            static_cast<int32_t>(nd)};
     A.slot_of[id[c]] = -1;
-    if (cnt[c] > kSmallNode) next_act[atomicAdd(&A.counter[1], 1u)] = id[c];
-    else if (cnt[c] > A.leaf_max) small[atomicAdd(&A.counter[2], 1u)] = id[c];
+    if (cnt[c] > kSmallNode) {
+      const uint32_t ns = atomicAdd(&A.counter[1], 1u);
+      next_act[ns] = id[c];
+      activate(A, id[c], ns);   // this level's bounds have been used
+    } else if (cnt[c] > A.leaf_max) small[atomicAdd(&A.counter[2], 1u)] = id[c];
   }
   }
 }
 
 __global__ void k_scatter(BuildArrays A, const uint32_t* __restrict__ idx, const uint32_t* __restrict__ node_of,
-                          uint32_t n, const uint32_t* __restrict__ excl, uint32_t* __restrict__ idx2,
-                          uint32_t* __restrict__ node2) {
-  if (level_active(A) == 0u) return;
+                          uint32_t n, LevelRank rank, uint32_t* __restrict__ idx2, uint32_t* __restrict__ node2) {
   const uint32_t pos = blockIdx.x * blockDim.x + threadIdx.x;
   if (pos >= n) return;
   const uint32_t nd = node_of[pos];
@@ -567,8 +623,8 @@ __global__ void k_scatter(BuildArrays A, const uint32_t* __restrict__ idx, const
     dst = pos;
     left = i < nl;
   } else {
-    const uint32_t rk = excl[pos] - excl[b];
-    left = excl[pos + 1] != excl[pos];
+    const uint32_t rk = rank.at(pos) - rank.at(b);
+    left = rank.flag(pos);
     dst = left ? b + rk : b + nl + (i - rk);
   }
   idx2[dst] = idx[pos];
@@ -773,9 +829,11 @@ __global__ void k_sah_bin_init(BuildArrays A, uint32_t* __restrict__ bins) {
 // primitives and its positions are contiguous, so a chunk meets at most
 // kBinSegs nodes.  Global atomics from every warp (one leader per bin and warp)
 // took up to 447 us for a level of the 2,064,386-triangle grid, where all of
-// them meet in one node's 96 bins, and 3.07 ms for its 19 levels; this takes
-// 1.75 ms.
+// them meet in one node's 96 bins, and 3.07 ms for its 19 levels; shared-memory
+// atomics alone take 1.75 ms, with the warp's lanes combined where they share one
+// or two bins 0.95 ms.
 constexpr uint32_t kBinChunk = 512;
+constexpr int kBinGroups = 2;   // bins of a warp up to which it combines its lanes first
 constexpr uint32_t kBinSegs = (kBinChunk - 2u) / (kSmallNode + 1u) + 2u;
 __global__ void __launch_bounds__(kThreads) k_sah_bin(BuildArrays A, const uint32_t* __restrict__ idx,
                                                       const uint32_t* __restrict__ node_of, uint32_t n,
@@ -821,6 +879,7 @@ __global__ void __launch_bounds__(kThreads) k_sah_bin(BuildArrays A, const uint3
   __syncthreads();
 #pragma unroll
   for (uint32_t r = 0; r < kRounds; ++r) {
+    const unsigned in = __ballot_sync(0xffffffffu, slot[r] >= 0);
     if (slot[r] < 0) continue;
     const uint32_t p = idx[start + r * kThreads + threadIdx.x];
     const uint32_t* k = A.cb + 6 * slot[r];
@@ -836,14 +895,35 @@ __global__ void __launch_bounds__(kThreads) k_sah_bin(BuildArrays A, const uint3
         bin = static_cast<int>((c[a] - c0) * (static_cast<float>(kSahBins) / ext));
         bin = bin < 0 ? 0 : (bin > kSahBins - 1 ? kSahBins - 1 : bin);
       }
-      uint32_t* w = s_bin + kBinWords * ((seg[r] * 3u + a) * kSahBins + static_cast<uint32_t>(bin));
-      atomicAdd(w, 1u);
-      atomicMin(w + 1, klo[0]);
-      atomicMin(w + 2, klo[1]);
-      atomicMin(w + 3, klo[2]);
-      atomicMax(w + 4, khi[0]);
-      atomicMax(w + 5, khi[1]);
-      atomicMax(w + 6, khi[2]);
+      const uint32_t at = (seg[r] * 3u + a) * kSahBins + static_cast<uint32_t>(bin);
+      uint32_t* w = s_bin + kBinWords * at;
+      // Neighbours fall into few bins where nodes are large against them: one
+      // atomic per bin and warp then, one per primitive where they spread.
+      const unsigned grp = __match_any_sync(in, at);
+      const bool leader = static_cast<int>(lane) == __ffs(grp) - 1;
+      if (__popc(__ballot_sync(in, leader)) <= kBinGroups) {
+        const uint32_t m0 = __reduce_min_sync(grp, klo[0]), m1 = __reduce_min_sync(grp, klo[1]),
+                       m2 = __reduce_min_sync(grp, klo[2]);
+        const uint32_t x0 = __reduce_max_sync(grp, khi[0]), x1 = __reduce_max_sync(grp, khi[1]),
+                       x2 = __reduce_max_sync(grp, khi[2]);
+        if (leader) {
+          atomicAdd(w, static_cast<uint32_t>(__popc(grp)));
+          atomicMin(w + 1, m0);
+          atomicMin(w + 2, m1);
+          atomicMin(w + 3, m2);
+          atomicMax(w + 4, x0);
+          atomicMax(w + 5, x1);
+          atomicMax(w + 6, x2);
+        }
+      } else {
+        atomicAdd(w, 1u);
+        atomicMin(w + 1, klo[0]);
+        atomicMin(w + 2, klo[1]);
+        atomicMin(w + 3, klo[2]);
+        atomicMax(w + 4, khi[0]);
+        atomicMax(w + 5, khi[1]);
+        atomicMax(w + 6, khi[2]);
+      }
     }
   }
   __syncthreads();
@@ -1088,11 +1168,42 @@ struct WideArrays {
   uint32_t* visits;
   int32_t* final_id;
   int32_t* slot_bin;    // optional: binary node per wide slot (refit)
+  const uint2* range;   // per binary node: first position and count of its triangles
+  const uint8_t* choice;   // per internal binary node: CollapseNode's choices
 };
 
-__device__ __forceinline__ float bin_area(const BinNode& n) {
-  const float dx = n.hi[0] - n.lo[0], dy = n.hi[1] - n.lo[1], dz = n.hi[2] - n.lo[2];
-  return dx * dy + dy * dz + dz * dx;
+// Costs and choices of every subtree (CollapseNode), bottom-up: one thread per
+// leaf walks up, the second child to arrive does the parent.
+__global__ void k_collapse_cost(const BinNode* __restrict__ bin, uint32_t n, const int32_t* __restrict__ parent,
+                                uint32_t* __restrict__ visits, float4* __restrict__ cost, uint2* __restrict__ range,
+                                uint8_t* __restrict__ choice) {
+  uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
+  if (x >= n || bin[x].count == 0) return;
+  {
+    const BinNode b = bin[x];
+    const float c = HalfArea(b.lo, b.hi) * (kTriangleCost * static_cast<float>(b.count));
+    cost[x] = make_float4(c, c, c, c);
+    range[x] = make_uint2(static_cast<uint32_t>(b.first), static_cast<uint32_t>(b.count));
+  }
+  while (true) {
+    __threadfence();
+    const int32_t p = parent[x];
+    if (p < 0) break;
+    if (atomicAdd(&visits[p], 1u) == 0u) break;   // the sibling finishes the parent
+    const BinNode b = bin[p];
+    const float4 l = __ldcg(cost + b.left), r = __ldcg(cost + b.right);
+    const uint2 rl = __ldcg(range + b.left), rr = __ldcg(range + b.right);
+    const float lc[4] = {l.x, l.y, l.z, l.w}, rc[4] = {r.x, r.y, r.z, r.w};
+    float o[4];
+    choice[p] = static_cast<uint8_t>(CollapseNode(lc, rc, HalfArea(b.lo, b.hi), static_cast<int32_t>(rl.y + rr.y), o));
+    cost[p] = make_float4(o[0], o[1], o[2], o[3]);
+    range[p] = make_uint2(rl.x, rl.y + rr.y);
+    x = static_cast<uint32_t>(p);
+  }
+}
+
+__device__ __forceinline__ bool wide_leaf(const WideArrays& W, int32_t id) {
+  return W.bin[id].count > 0 || CollapseLeaf(W.choice[id]);
 }
 
 // One level of the collapse; the level's count is read from counter[4] (0
@@ -1110,26 +1221,32 @@ __global__ void k_wide_expand(WideArrays W, const uint32_t* __restrict__ cur, ui
   if (r.count > 0) {
     slots[ns++] = root;
   } else {
-    slots[ns++] = r.left;
-    slots[ns++] = r.right;
-    while (ns < 4) {
-      int best = -1;
-      float best_area = -1.0f;
-      for (int s = 0; s < ns; ++s) {
-        const BinNode c = W.bin[slots[s]];
-        if (c.count > 0) continue;
-        const float a = bin_area(c);
-        if (a > best_area) {
-          best_area = a;
-          best = s;
-        }
+    // the best four roots, left to right
+    int32_t todo[4];
+    uint32_t take[4];
+    const uint32_t k0 = CollapseSplit(W.choice[root], 4u);
+    todo[0] = r.right;
+    take[0] = 4u - k0;
+    todo[1] = r.left;
+    take[1] = k0;
+    int left = 2;
+    while (left > 0) {
+      --left;
+      const int32_t id = todo[left];
+      uint32_t i2 = take[left];
+      const bool leaf = W.bin[id].count > 0;
+      const uint32_t bits = leaf ? 0u : W.choice[id];
+      if (leaf) i2 = 1u;
+      while (i2 > 1u && CollapseFewer(bits, i2)) --i2;
+      if (i2 == 1u) {
+        slots[ns++] = id;
+      } else {
+        const uint32_t k = CollapseSplit(bits, i2);
+        todo[left] = W.bin[id].right;
+        take[left++] = i2 - k;
+        todo[left] = W.bin[id].left;
+        take[left++] = k;
       }
-      if (best < 0) break;
-      const BinNode c = W.bin[slots[best]];
-      for (int s = ns; s > best + 1; --s) slots[s] = slots[s - 1];
-      slots[best] = c.left;
-      slots[best + 1] = c.right;
-      ++ns;
     }
   }
   const int32_t stack_here = w.stack_here + ns - 1;
@@ -1140,7 +1257,7 @@ __global__ void k_wide_expand(WideArrays W, const uint32_t* __restrict__ cur, ui
   for (int s = 0; s < 4; ++s) {
     w.slot[s] = s < ns ? slots[s] : -1;
     w.child[s] = -1;
-    if (s < ns && W.bin[slots[s]].count == 0) {
+    if (s < ns && !wide_leaf(W, slots[s])) {
       const uint32_t c = atomicAdd(&W.counter[0], 1u);
       W.w[c].slot[0] = slots[s];
       W.w[c].parent = static_cast<int32_t>(wid);
@@ -1212,9 +1329,8 @@ __global__ void k_wide_write(WideArrays W, uint32_t n_wide, WideNode* __restrict
   for (int k = 0; k < w.nslots; ++k) {
     const BinNode c = W.bin[w.slot[k]];
     SetWideSlot(n, k, c.lo, c.hi);
-    n.child[k] = c.count > 0 ? ~static_cast<int32_t>((static_cast<uint32_t>(c.first) << 3) |
-                                                     static_cast<uint32_t>(c.count - 1))
-                             : W.final_id[w.child[k]];
+    const uint2 g = W.range[w.slot[k]];
+    n.child[k] = w.child[k] < 0 ? ~static_cast<int32_t>((g.x << 3) | (g.y - 1u)) : W.final_id[w.child[k]];
   }
   out[W.final_id[x]] = n;
 }
@@ -1278,8 +1394,9 @@ cudaError_t build_tree(const float4* blo, const float4* bhi, uint32_t n, bool sa
   uint32_t* node_of = sc.get<uint32_t>(n);
   uint32_t* idx2 = sc.get<uint32_t>(n);
   uint32_t* node2 = sc.get<uint32_t>(n);
-  uint32_t* flag = sc.get<uint32_t>(n);
-  uint32_t* excl = sc.get<uint32_t>(n + 1u);
+  uint32_t* loc = sc.get<uint32_t>(n + 1u);
+  const uint32_t scan_blocks = n / kScanBlock + 1u;   // n + 1 entries
+  uint32_t* sums = sc.get<uint32_t>(scan_blocks);
   // Nodes of one level above kSmallNode primitives are disjoint: at most n / 65 of them;
   // small subtree roots (leaf_max + 1..64 primitives) are disjoint too.
   const uint32_t max_act = n / (kSmallNode + 1u) + 2u;
@@ -1322,8 +1439,9 @@ cudaError_t build_tree(const float4* blo, const float4* bhi, uint32_t n, bool sa
   uint32_t first_check = 1u;
   for (uint64_t m = n / (kSmallNode + 1u); m > 1u; m >>= 1) ++first_check;
   bool more = init[4] != 0u;
+  const LevelRank rank{loc, sums};
+  k_level_init<<<1, 1, 0, s>>>(A, act);
   for (uint32_t level = 1u; more; ++level) {
-    k_level_init<<<act_grid, kThreads, 0, s>>>(A, act);
     k_centroid_bounds<<<grid_for(n), kThreads, 0, s>>>(A, idx, node_of, n);
     if (sah) {
       k_sah_bin_init<<<bin_grid, kThreads, 0, s>>>(A, bins);
@@ -1332,15 +1450,14 @@ cudaError_t build_tree(const float4* blo, const float4* bhi, uint32_t n, bool sa
     } else {
       k_midpoint_split<<<act_grid, kThreads, 0, s>>>(A);
     }
-    k_flags<<<grid_for(n), kThreads, 0, s>>>(A, idx, node_of, n, flag, sah);
-    BB_TRY(exclusive_scan(flag, n, excl, sc));
-    k_children<<<act_grid, kThreads, 0, s>>>(A, act, excl, next, small);
-    k_scatter<<<grid_for(n), kThreads, 0, s>>>(A, idx, node_of, n, excl, idx2, node2);
-    k_level_done<<<act_grid, kThreads, 0, s>>>(A, act);
-    // the scattered order becomes the current one (the caller's buffer keeps the final order)
-    k_copy_level<<<std::min(grid_for(n), 148u * 8u), kThreads, 0, s>>>(A, idx, idx2, n);
+    k_flag_scan<<<scan_blocks, kScanThreads, 0, s>>>(A, idx, node_of, n, sah, loc, sums);
+    k_scan_sums<<<1, 1024, 0, s>>>(A, sums, scan_blocks);
+    k_children<<<act_grid, kThreads, 0, s>>>(A, act, rank, next, small);
+    // (a level queued past the last copies the order unchanged)
+    k_scatter<<<grid_for(n), kThreads, 0, s>>>(A, idx, node_of, n, rank, idx2, node2);
     k_level_advance<<<1, 1, 0, s>>>(A);
     BB_TRY(cudaGetLastError());
+    std::swap(idx, idx2);
     std::swap(node_of, node2);
     std::swap(act, next);
     if (level >= first_check && (level - first_check) % 2u == 0u) {
@@ -1348,6 +1465,10 @@ cudaError_t build_tree(const float4* blo, const float4* bhi, uint32_t n, bool sa
       BB_TRY(read_scalar(counter + 4, cur, s));
       more = cur != 0u;
     }
+  }
+  if (idx != order) {   // the caller's buffer keeps the final order
+    BB_TRY(cudaMemcpyAsync(order, idx, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
+    idx = order;
   }
   uint32_t n_small = 0u;
   BB_TRY(read_scalar(counter + 2, n_small, s));
@@ -1378,6 +1499,17 @@ cudaError_t finish_tree(const float4* blo, const float4* bhi, const uint32_t* or
   return cudaGetLastError();
 }
 
+__global__ void k_parents(const BinNode* __restrict__ nodes, uint32_t n, int32_t* __restrict__ parent) {
+  const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
+  if (x >= n) return;
+  if (x == 0u) parent[0] = -1;
+  const BinNode b = nodes[x];
+  if (b.count == 0) {
+    parent[b.left] = static_cast<int32_t>(x);
+    parent[b.right] = static_cast<int32_t>(x);
+  }
+}
+
 // Each wide node starts at a binary internal node of its own (at a leaf only
 // when that is the root).
 uint32_t wide_capacity(uint32_t n_bin) { return n_bin / 2u + 1u; }
@@ -1386,11 +1518,19 @@ cudaError_t collapse(const BinNode* bin, uint32_t n_bin, WideNode* out, uint32_t
                      uint32_t& stack_required, Scratch& sc, int32_t* slot_bin = nullptr) {
   cudaStream_t s = sc.s;
   const uint32_t cap = wide_capacity(n_bin);
+  int32_t* parent = sc.get<int32_t>(n_bin);
+  uint32_t* visits = sc.get<uint32_t>(n_bin);
+  float4* cost = sc.get<float4>(n_bin);
+  uint2* range = sc.get<uint2>(n_bin);
+  uint8_t* choice = sc.get<uint8_t>(n_bin);
   WideArrays W{bin, sc.get<WTemp>(cap), sc.get<uint32_t>(8), sc.get<uint32_t>(cap), sc.get<uint32_t>(cap),
-               sc.get<int32_t>(cap), slot_bin};
+               sc.get<int32_t>(cap), slot_bin, range, choice};
   uint32_t* cur = sc.get<uint32_t>(cap);
   uint32_t* next = sc.get<uint32_t>(cap);
   if (sc.err != cudaSuccess) return sc.err;
+  k_parents<<<grid_for(n_bin), kThreads, 0, s>>>(bin, n_bin, parent);
+  BB_TRY(cudaMemsetAsync(visits, 0, n_bin * sizeof(uint32_t), s));
+  k_collapse_cost<<<grid_for(n_bin), kThreads, 0, s>>>(bin, n_bin, parent, visits, cost, range, choice);
   WTemp root{};
   root.slot[0] = 0;
   root.parent = -1;
@@ -1453,17 +1593,6 @@ __global__ void k_inst_first(const uint32_t* __restrict__ pos, const unsigned lo
 __global__ void k_tri_pos(const uint32_t* __restrict__ order, uint32_t n, uint32_t* __restrict__ tri_pos) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) tri_pos[order[i]] = i;
-}
-
-__global__ void k_parents(const BinNode* __restrict__ nodes, uint32_t n, int32_t* __restrict__ parent) {
-  const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= n) return;
-  if (x == 0u) parent[0] = -1;
-  const BinNode b = nodes[x];
-  if (b.count == 0) {
-    parent[b.left] = static_cast<int32_t>(x);
-    parent[b.right] = static_cast<int32_t>(x);
-  }
 }
 
 // ---------------------------------------------------------------- refit after transform updates

@@ -12,6 +12,7 @@
 #include "bvh_host.h"
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstring>
 #include <functional>
@@ -92,11 +93,6 @@ struct Builder {
     build(r, idx + left_n, n - left_n);
   }
 };
-
-float surface_area(const BinNode& n) {
-  const float dx = n.hi[0] - n.lo[0], dy = n.hi[1] - n.lo[1], dz = n.hi[2] - n.lo[2];
-  return dx * dy + dy * dz + dz * dx;
-}
 
 }  // namespace
 
@@ -465,28 +461,69 @@ void CollapseToWide(const SceneGeometry& geo, const std::vector<BinNode>& bin,
     t.depth = depth[i];
   }
 
-  auto emit_leaf = [&](int32_t leaf_id) -> int32_t {
-    const BinNode& lf = bin[static_cast<size_t>(leaf_id)];
-    const uint32_t first = static_cast<uint32_t>(out.tris.size());
-    for (int32_t i = 0; i < lf.count; ++i) {
-      const uint32_t p = prim_indices[static_cast<size_t>(lf.first + i)];
-      const HostPrim& hp = geo.prims[p];
-      TriRecord r;
-      r.v0x = hp.v0[0];
-      r.v0y = hp.v0[1];
-      r.v0z = hp.v0[2];
-      r.e1x = hp.e1[0];
-      r.e1y = hp.e1[1];
-      r.e1z = hp.e1[2];
-      r.e2x = hp.e2[0];
-      r.e2y = hp.e2[1];
-      r.e2z = hp.e2[2];
-      r.prim = p;
-      r.leaf = ref_leaf[p];
-      r.lane = ref_lane[p];
-      out.tris.push_back(r);
+  // Bottom-up costs and choices of the collapse (children after their parents in `post` reversed).
+  std::vector<std::array<float, 4>> cost(bin.size());
+  std::vector<int32_t> count(bin.size(), 0);
+  std::vector<uint8_t> choice(bin.size(), 0);
+  {
+    std::vector<int32_t> post, st{0};
+    while (!st.empty()) {
+      const int32_t id = st.back();
+      st.pop_back();
+      post.push_back(id);
+      const BinNode& nd = bin[static_cast<size_t>(id)];
+      if (nd.count > 0) continue;
+      st.push_back(nd.left);
+      st.push_back(nd.right);
     }
-    return ~static_cast<int32_t>((first << 3) | static_cast<uint32_t>(lf.count - 1));
+    for (size_t k = post.size(); k-- > 0;) {
+      const size_t id = static_cast<size_t>(post[k]);
+      const BinNode& nd = bin[id];
+      const float area = HalfArea(nd.lo, nd.hi);
+      if (nd.count > 0) {
+        count[id] = nd.count;
+        cost[id].fill(area * (kTriangleCost * static_cast<float>(nd.count)));
+      } else {
+        const size_t l = static_cast<size_t>(nd.left), r = static_cast<size_t>(nd.right);
+        count[id] = count[l] + count[r];
+        choice[id] = static_cast<uint8_t>(CollapseNode(cost[l].data(), cost[r].data(), area, count[id], cost[id].data()));
+      }
+    }
+  }
+  auto is_leaf = [&](int32_t id) { return bin[static_cast<size_t>(id)].count > 0 || CollapseLeaf(choice[static_cast<size_t>(id)]); };
+
+  // The triangles of a subtree, left to right, as one leaf.
+  auto emit_leaf = [&](int32_t root_id) -> int32_t {
+    const uint32_t first = static_cast<uint32_t>(out.tris.size());
+    std::vector<int32_t> st{root_id};
+    while (!st.empty()) {
+      const BinNode& lf = bin[static_cast<size_t>(st.back())];
+      st.pop_back();
+      if (lf.count == 0) {
+        st.push_back(lf.right);
+        st.push_back(lf.left);
+        continue;
+      }
+      for (int32_t i = 0; i < lf.count; ++i) {
+        const uint32_t p = prim_indices[static_cast<size_t>(lf.first + i)];
+        const HostPrim& hp = geo.prims[p];
+        TriRecord r;
+        r.v0x = hp.v0[0];
+        r.v0y = hp.v0[1];
+        r.v0z = hp.v0[2];
+        r.e1x = hp.e1[0];
+        r.e1y = hp.e1[1];
+        r.e1z = hp.e1[2];
+        r.e2x = hp.e2[0];
+        r.e2y = hp.e2[1];
+        r.e2z = hp.e2[2];
+        r.prim = p;
+        r.leaf = ref_leaf[p];
+        r.lane = ref_lane[p];
+        out.tris.push_back(r);
+      }
+    }
+    return ~static_cast<int32_t>((first << 3) | (static_cast<uint32_t>(out.tris.size()) - first - 1u));
   };
 
   // Depth-first, pre-order allocation of wide nodes.
@@ -499,23 +536,23 @@ void CollapseToWide(const SceneGeometry& geo, const std::vector<BinNode>& bin,
     if (root.count > 0) {
       slots.push_back(bin_id);
     } else {
-      slots = {root.left, root.right};
-      while (slots.size() < 4) {
-        int best = -1;
-        float best_area = -1.0f;
-        for (size_t s = 0; s < slots.size(); ++s) {
-          const BinNode& c = bin[static_cast<size_t>(slots[s])];
-          if (c.count > 0) continue;
-          const float a = surface_area(c);
-          if (a > best_area) {
-            best_area = a;
-            best = static_cast<int>(s);
-          }
+      const uint32_t k0 = CollapseSplit(choice[static_cast<size_t>(bin_id)], 4u);
+      std::vector<std::pair<int32_t, uint32_t>> st{{root.right, 4u - k0}, {root.left, k0}};
+      while (!st.empty()) {
+        const int32_t id = st.back().first;
+        uint32_t i = st.back().second;
+        st.pop_back();
+        const BinNode& nd = bin[static_cast<size_t>(id)];
+        const uint32_t bits = choice[static_cast<size_t>(id)];
+        if (nd.count > 0) i = 1u;
+        while (i > 1u && CollapseFewer(bits, i)) --i;
+        if (i == 1u) {
+          slots.push_back(id);
+        } else {
+          const uint32_t k = CollapseSplit(bits, i);
+          st.push_back({nd.right, i - k});
+          st.push_back({nd.left, k});
         }
-        if (best < 0) break;
-        const BinNode& c = bin[static_cast<size_t>(slots[static_cast<size_t>(best)])];
-        slots[static_cast<size_t>(best)] = c.left;
-        slots.insert(slots.begin() + best + 1, c.right);
       }
     }
     const uint32_t stack_here = stack_so_far + static_cast<uint32_t>(slots.size()) - 1u;
@@ -528,10 +565,8 @@ void CollapseToWide(const SceneGeometry& geo, const std::vector<BinNode>& bin,
       const BinNode& c = bin[static_cast<size_t>(slots[s])];
       SetWideSlot(wn, static_cast<int>(s), c.lo, c.hi);
     }
-    for (size_t s = 0; s < slots.size(); ++s) {
-      const BinNode& c = bin[static_cast<size_t>(slots[s])];
-      wn.child[s] = (c.count > 0) ? emit_leaf(slots[s]) : make(slots[s], level + 1u, stack_here);
-    }
+    for (size_t s = 0; s < slots.size(); ++s)
+      wn.child[s] = is_leaf(slots[s]) ? emit_leaf(slots[s]) : make(slots[s], level + 1u, stack_here);
     out.nodes[static_cast<size_t>(wide_id)] = wn;
     return wide_id;
   };
