@@ -127,10 +127,11 @@ __device__ __forceinline__ float4 adj_primal(const DevScene& s, const DevSetting
   return make_float4(rad.x, rad.y, rad.z, __uint_as_float(static_cast<uint32_t>(sig ^ (sig >> 32))));
 }
 
-// 102 registers (5 blocks of 128 threads per SM): 1.98 -> 1.87 ms per forward pass.
-// kRecord: the forward also writes every path's vertex records (recs, the
-// backward's layout with all paths as one chunk) and their count (nrec), so
-// a backward over the same paths needs no replay.
+// One path per thread from start to end: the forward without records, and the
+// recording forward of few paths.  102 registers (5 blocks of 128 threads per
+// SM): 1.98 -> 1.87 ms per 524,288-path forward.  kRecord: every path's vertex
+// records (recs, the backward's layout with all paths as one chunk) and their
+// count (nrec), so a backward over the same paths needs no replay.
 template <bool kParity, bool kRecord>
 __global__ void __launch_bounds__(128, 5) k_adj_forward(DevScene s, DevSettings st, const float* mat0, uint32_t spp,
                                                      uint32_t first_sample, int cap, float4* rad, AdjRec* recs,
@@ -154,6 +155,203 @@ __global__ void __launch_bounds__(128, 5) k_adj_forward(DevScene s, DevSettings 
     }
   }
   if (local_err) atomicOr(err, local_err);
+}
+
+// ------------------------------------------------------------ recording forward
+// The recording forward of many paths runs as a wavefront, as the renderer's frames do
+// (kernels.cu): per depth one trace launch (the closest hits of this depth's
+// paths and the previous depth's next-event queries) and one shading launch,
+// which writes the vertex records.  Walking a whole path per thread leaves a warp
+// waiting for its longest path, with the traversal and the shading code in one
+// kernel at 96 registers: 1.38 ms per 524,288-path forward, this takes 0.84 ms.
+// Words of AdjWave::counts: 0, 1 extension queue sizes, 2, 3 query counts by the
+// depth that fills them (even, odd), 4 the trace's fetch counter.
+struct AdjTraceSource {
+  GeoView geo;
+  const uint32_t* q;
+  AdjWave w;
+  float4* rad;
+  AdjRec* rec_prev;     // the previous depth's vertex of every path
+  uint32_t n_ext;
+  static constexpr bool kUniform = true;
+  __device__ __forceinline__ const GeoView& geo_at(uint32_t) const { return geo; }
+  __device__ __forceinline__ bool any(uint32_t j) const { return j >= n_ext; }
+  __device__ __forceinline__ void load(uint32_t j, V3& o, V3& d, float& tm, GeoView& g) const {
+    g = geo;
+    const bool sh = j >= n_ext;
+    const uint32_t k = sh ? j - n_ext : q[j];
+    const float4 a = (sh ? w.sh_o : w.ray_o)[k], b = (sh ? w.sh_d : w.ray_d)[k];
+    o = mk(a.x, a.y, a.z);
+    d = mk(b.x, b.y, b.z);
+    tm = sh ? a.w : kInf;
+  }
+  __device__ __forceinline__ bool finish(uint32_t j, float t, uint32_t prim, V3&, V3, float&) const {
+    if (j < n_ext) {
+      w.hit[q[j]] = make_float2(t, __uint_as_float(prim));
+      return false;
+    }
+    if (prim) return false;   // occluded
+    const uint32_t p = w.sh_path[j - n_ext];
+    const float4 c = w.sh_c[j - n_ext];
+    float4 r = rad[p];
+    r.x = r.x + c.x;
+    r.y = r.y + c.y;
+    r.z = r.z + c.z;
+    rad[p] = r;
+    rec_prev[p].e.z |= kVfNeeVis;
+    return false;
+  }
+};
+
+template <bool kParity>
+__global__ void __launch_bounds__(256) k_adj_raygen(DevScene s, DevSettings st, uint32_t n, uint32_t first_sample,
+                                                    AdjWave w, float4* rad) {
+  const uint32_t npx = st.width * st.height;
+  for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
+    const uint32_t sl = j / npx, p = j - sl * npx;
+    V3 o, d;
+    uint64_t rng;
+    camera_path<kParity>(s, st, p % st.width, p / st.width, first_sample + sl, o, d, rng);
+    w.rng[j] = rng;
+    w.ray_o[j] = make_float4(o.x, o.y, o.z, 0.0f);
+    w.ray_d[j] = make_float4(d.x, d.y, d.z, 0.0f);
+    w.thr[j] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
+    w.thr0[j] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
+    rad[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    w.q[0][j] = j;
+  }
+  if (blockIdx.x == 0 && threadIdx.x < 8u) w.counts[threadIdx.x] = threadIdx.x == 0u ? n : 0u;
+}
+
+__global__ void __launch_bounds__(256, 4) k_adj_trace(DevScene s, AdjWave w, const uint32_t* q, uint32_t depth,
+                                                      float4* rad, AdjRec* rec_prev, int scap, int2* spill, int total,
+                                                      int steps, uint32_t* err) {
+  extern __shared__ int2 smem_stack[];
+  const uint32_t cur = depth & 1u;
+  const uint32_t n_ext = w.counts[cur], n_sh = depth > 0u ? w.counts[2u + (cur ^ 1u)] : 0u;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    w.counts[cur ^ 1u] = 0u;
+    w.counts[2u + cur] = 0u;
+  }
+  const AdjTraceSource src{geo_of(s), q, w, rad, rec_prev, n_ext};
+  const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x;
+  const TwoLevelStack stk{smem_stack + threadIdx.x, static_cast<int>(blockDim.x), scap, spill ? spill + gtid : nullptr,
+                          static_cast<int>(gridDim.x * blockDim.x), total};
+  TraceStats st;
+  uint32_t lerr = 0u;
+  persistent_traverse<AdjTraceSource, kQueryMixed, false>(src, n_ext + n_sh, &w.counts[4], stk, steps, st, st, lerr);
+  if (lerr) atomicOr(err, lerr);
+}
+
+// One vertex per queued path: adj_primal's bounce with the visibility test left
+// to the next trace, the record written, survivors and queries appended.
+template <bool kParity>
+__global__ void __launch_bounds__(128, 5) k_adj_shade(DevScene s, DevSettings st, const float* mat0, AdjWave w,
+                                                      const uint32_t* q, uint32_t* qn, uint32_t depth, float4* rad,
+                                                      AdjRec* rec, uint32_t* nrec) {
+  const uint32_t cur = depth & 1u;
+  const uint32_t n = w.counts[cur];
+  if (blockIdx.x == 0 && threadIdx.x == 0) w.counts[4] = 0u;
+  for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
+    const uint32_t j = base + threadIdx.x;
+    bool next = false, shadow = false;
+    uint32_t p = 0u;
+    V3 sh_c = mk(0.0f, 0.0f, 0.0f);
+    AdjVertex<float, V3> R;
+    R.nee = false;
+    if (j < n) {
+      p = q[j];
+      const float4 o4 = w.ray_o[p], d4 = w.ray_d[p], t4 = w.thr[p], u4 = w.thr0[p], r4 = rad[p];
+      const float2 h2 = w.hit[p];
+      const V3 o = mk(o4.x, o4.y, o4.z), d = mk(d4.x, d4.y, d4.z);
+      V3 thr = mk(t4.x, t4.y, t4.z), thr0 = mk(u4.x, u4.y, u4.z), r = mk(r4.x, r4.y, r4.z);
+      const uint32_t prim = __float_as_uint(h2.y);
+      AdjRec v;
+      v.a = make_float4(o.x, o.y, o.z, prim == kMiss ? 0.0f : h2.x);
+      v.b = make_float4(d.x, d.y, d.z, h2.y);
+      if (prim == kMiss) {
+        r = add(r, mulv(thr, s.env));
+        v.c = make_float4(thr.x, thr.y, thr.z, 1.0f);
+        v.e = make_uint4(0u, 0u, kVfMiss, 0u);
+      } else {
+        uint64_t rng = w.rng[p];
+        const uint64_t rng_at = rng;
+        const float4 sh = __ldg(s.shade + prim);
+        const V3 gn = mk(sh.x, sh.y, sh.z);
+        const uint32_t mi = mat_slot(s, __float_as_uint(sh.w));
+        const MaterialRec m = load_material(s.materials + 16u * mi);
+        uint32_t flags = 0u;
+        adj_vertex<float, V3, kParity, false>(s, st, s.lights, depth, o, d, h2.x, gn, m, clamp01(m.roughness), rng, flags,
+                                              R);
+        const bool emissive_model = m.model == 1u || m.emissive.x > 0.0f || m.emissive.y > 0.0f || m.emissive.z > 0.0f;
+        if (!st.enable_nee || depth == 0u) r = add(r, mulv(thr, m.emissive));
+        else if (st.enable_mis && emissive_model) r = add(r, mul(mulv(thr, m.emissive), R.w_e));
+        if (R.nee) {
+          sh_c = st.enable_mis ? mul(mulv(thr, R.q.radiance), R.w_n) : mulv(thr, R.q.radiance);
+          shadow = R.q.remain > 0.004f;
+          if (!shadow) {   // no visibility test runs for so short a segment
+            r = add(r, sh_c);
+            flags |= kVfNeeVis;
+          }
+        }
+        v.c = make_float4(thr.x, thr.y, thr.z, 1.0f);
+        if (R.scattered) {
+          thr = mulv(thr, albedo_effect0(m));
+          thr0 = mulv(thr0, albedo_effect0(load_material(mat0 + 16u * mi)));
+          const float tmx = smax(thr0.x, smax(thr0.y, thr0.z));
+          if (!(tmx < 0.001f)) {
+            const float rr = smin(st.rr_max, smax(st.rr_min, tmx));
+            v.c.w = rr;
+            if (!(depth >= st.rr_start && next01(rng) > rr)) {
+              thr = divs(thr, rr);
+              thr0 = divs(thr0, rr);
+              next = depth + 1u < st.max_depth;
+            }
+          }
+        }
+        v.e = make_uint4(static_cast<uint32_t>(rng_at), static_cast<uint32_t>(rng_at >> 32), flags | (next ? kVfCont : 0u),
+                         mi);
+        if (next) {
+          const V3 no = add(R.hp, mul(R.out, 0.002f));
+          w.ray_o[p] = make_float4(no.x, no.y, no.z, 0.0f);
+          w.ray_d[p] = make_float4(R.out.x, R.out.y, R.out.z, 0.0f);
+          w.thr[p] = make_float4(thr.x, thr.y, thr.z, 0.0f);
+          w.thr0[p] = make_float4(thr0.x, thr0.y, thr0.z, 0.0f);
+          w.rng[p] = rng;
+        }
+      }
+      rec[p] = v;
+      if (!next) nrec[p] = depth + 1u;
+      rad[p] = make_float4(r.x, r.y, r.z, 0.0f);
+    }
+    const uint32_t slot_n = warp_append(&w.counts[cur ^ 1u], next);
+    if (next) qn[slot_n] = p;
+    const uint32_t slot_s = warp_append(&w.counts[2u + cur], shadow);
+    if (shadow) {
+      w.sh_path[slot_s] = p;
+      w.sh_o[slot_s] = make_float4(R.q.origin.x, R.q.origin.y, R.q.origin.z, R.q.remain);
+      w.sh_d[slot_s] = make_float4(R.q.dir.x, R.q.dir.y, R.q.dir.z, 0.0f);
+      w.sh_c[slot_s] = make_float4(sh_c.x, sh_c.y, sh_c.z, 0.0f);
+    }
+  }
+}
+
+// adj_primal's hash of a path's decisions, from its records, into rad's w.
+__global__ void __launch_bounds__(256) k_adj_sign(uint32_t n, const AdjRec* __restrict__ recs,
+                                                  const uint32_t* __restrict__ nrec, float4* rad) {
+  for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
+    uint64_t sig = 0u;
+    const uint32_t k = nrec[j];
+    for (uint32_t v = 0; v < k; ++v) {
+      const AdjRec& r = recs[static_cast<size_t>(v) * n + j];
+      const uint32_t flags = r.e.z;
+      const uint64_t word = (flags & kVfMiss) ? 0xFFFFFFFFull
+                                              : (static_cast<uint64_t>(__float_as_uint(r.b.w) + 1u) |
+                                                 static_cast<uint64_t>(flags) << 32);
+      sig = mix64(sig ^ word);
+    }
+    reinterpret_cast<float*>(rad + j)[3] = __uint_as_float(static_cast<uint32_t>(sig ^ (sig >> 32)));
+  }
 }
 
 // Per pixel: film accumulation in sample order (non-finite samples dropped,
@@ -510,18 +708,39 @@ cudaError_t LaunchAdjForward(const DevScene& s, const DevSettings& st, const flo
   const size_t smem = AdjForwardSmem(l.block, l.stack_cap);
   AdjRec* r = reinterpret_cast<AdjRec*>(recs);
   const bool rec = recs != nullptr && nrec != nullptr;
-  if (l.parity && rec)
-    k_adj_forward<true, true><<<l.grid, l.block, smem, l.stream>>>(s, st, mat0, l.spp, l.first_sample, l.stack_cap, rad,
-                                                                   r, nrec, err);
-  else if (l.parity)
-    k_adj_forward<true, false><<<l.grid, l.block, smem, l.stream>>>(s, st, mat0, l.spp, l.first_sample, l.stack_cap,
-                                                                    rad, nullptr, nullptr, err);
-  else if (rec)
-    k_adj_forward<false, true><<<l.grid, l.block, smem, l.stream>>>(s, st, mat0, l.spp, l.first_sample, l.stack_cap,
-                                                                    rad, r, nrec, err);
-  else
-    k_adj_forward<false, false><<<l.grid, l.block, smem, l.stream>>>(s, st, mat0, l.spp, l.first_sample, l.stack_cap,
-                                                                     rad, nullptr, nullptr, err);
+#define VKPTC_FWD(P, R) \
+  k_adj_forward<P, R><<<l.grid, l.block, smem, l.stream>>>(s, st, mat0, l.spp, l.first_sample, l.stack_cap, rad, r, nrec, err)
+  if (l.parity && rec) VKPTC_FWD(true, true);
+  else if (l.parity) VKPTC_FWD(true, false);
+  else if (rec) VKPTC_FWD(false, true);
+  else VKPTC_FWD(false, false);
+#undef VKPTC_FWD
+  return cudaGetLastError();
+}
+
+cudaError_t ConfigureAdjTraceSmem(size_t bytes) {
+  return cudaFuncSetAttribute(k_adj_trace, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+}
+
+cudaError_t LaunchAdjRecord(const DevScene& s, const DevSettings& st, const float* mat0, const AdjWaveLaunch& l,
+                            const AdjWave& w, float4* rad, float4* recs, uint32_t* nrec, uint32_t* err) {
+  const uint32_t n = st.width * st.height * l.spp;
+  AdjRec* r = reinterpret_cast<AdjRec*>(recs);
+  const size_t smem = static_cast<size_t>(l.block) * l.smem_entries * sizeof(int2);
+  constexpr int kShadeBlock = 128;   // k_adj_shade's bound
+  const int shade_grid = std::max(1, l.grid * l.block / kShadeBlock);
+  if (l.parity) k_adj_raygen<true><<<l.grid, l.block, 0, l.stream>>>(s, st, n, l.first_sample, w, rad);
+  else k_adj_raygen<false><<<l.grid, l.block, 0, l.stream>>>(s, st, n, l.first_sample, w, rad);
+  for (uint32_t depth = 0; depth < st.max_depth; ++depth) {
+    const uint32_t* q = w.q[depth & 1u];
+    uint32_t* qn = w.q[(depth & 1u) ^ 1u];
+    AdjRec* rec = r + static_cast<size_t>(depth) * n;
+    k_adj_trace<<<l.grid, l.block, smem, l.stream>>>(s, w, q, depth, rad, depth > 0u ? rec - n : rec, l.smem_entries,
+                                                     l.spill, l.stack_cap, l.steps, err);
+    if (l.parity) k_adj_shade<true><<<shade_grid, kShadeBlock, 0, l.stream>>>(s, st, mat0, w, q, qn, depth, rad, rec, nrec);
+    else k_adj_shade<false><<<shade_grid, kShadeBlock, 0, l.stream>>>(s, st, mat0, w, q, qn, depth, rad, rec, nrec);
+  }
+  k_adj_sign<<<l.grid, l.block, 0, l.stream>>>(n, r, nrec, rad);
   return cudaGetLastError();
 }
 

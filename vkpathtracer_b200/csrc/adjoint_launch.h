@@ -1,6 +1,6 @@
 // adjoint_launch.h -- launch interface of the differentiable-rendering kernels
-// (adjoint.cu).  One forward renders `spp` samples of every pixel with one
-// path per thread and keeps each sample's radiance; the loss kernel forms the
+// (adjoint.cu).  One forward renders `spp` samples of every pixel and keeps
+// each sample's radiance; the loss kernel forms the
 // image, the mean-squared-error loss (FP64 reduction) and the per-pixel
 // adjoint; the backward replays every path from its RNG key and runs the
 // reverse sweep over its vertices.
@@ -30,6 +30,26 @@ struct AdjLaunch {
 // that a backward over the same paths skips its replay.
 cudaError_t LaunchAdjForward(const DevScene& s, const DevSettings& st, const float* mat0, const AdjLaunch& l,
                              float4* rad, uint32_t* err, float4* recs = nullptr, uint32_t* nrec = nullptr);
+
+// The recording forward as a wavefront, for many paths.
+struct AdjWave {
+  float4 *ray_o, *ray_d, *thr, *thr0, *sh_o, *sh_d, *sh_c;
+  uint64_t* rng;
+  float2* hit;
+  uint32_t *q[2], *sh_path;
+  uint32_t* counts;       // 8 words
+};
+struct AdjWaveLaunch {
+  int grid, block, smem_entries, stack_cap, steps;
+  int2* spill;
+  uint32_t spp, first_sample;
+  bool parity;
+  cudaStream_t stream;
+};
+cudaError_t LaunchAdjRecord(const DevScene& s, const DevSettings& st, const float* mat0, const AdjWaveLaunch& l,
+                            const AdjWave& w, float4* rad, float4* recs, uint32_t* nrec, uint32_t* err);
+// Raises its trace kernel's dynamic shared-memory limit (stacks above 48 KB per block).
+cudaError_t ConfigureAdjTraceSmem(size_t bytes);
 
 // Image (sample-order accumulation exactly as the film does), loss partials
 // per block, and the per-pixel adjoint dL/d(sample radiance) (0 without a target).
