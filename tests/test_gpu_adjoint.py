@@ -287,3 +287,61 @@ def test_backward_before_forward_is_not_ready():
         t.backward()
     assert e.value.code == native.NOT_READY
     t.close()
+
+
+@pytest.mark.parametrize("max_depth,nee", [(1, True), (2, False), (8, True)])
+@pytest.mark.parametrize("width,height,spp", [(7, 3, 1), (148, 160, 4), (149, 160, 4), (128, 96, 16)])
+def test_recording_wavefront_equals_the_per_path_forward(width, height, spp, max_depth, nee):
+    """An ordinary forward of more paths than the per-path kernel has resident
+    threads runs as a recording wavefront; a decorrelated setup always runs
+    one path per thread without records and its backward replays.  Loss,
+    samples, decision hashes and gradient are bit-identical, below, at and
+    above the line (94,720 paths on 148 SMs) and for queues that empty after
+    the first depth."""
+    sc = scenes.inverse_box_scene()
+    st = scenes.inverse_settings(width, height, spp)
+    st.max_depth, st.enable_nee = max_depth, nee
+    t = CudaPathTracer(bvh="reference")
+    assert t.configure(st).ok and t.load_scene_snapshot(sc).ok and t.build_or_update_acceleration().ok
+    target = np.full((height, width, 3), 0.25, np.float32)
+    out = []
+    for kw in ({}, dict(frame=0, decorrelated=True, backward_frame=0)):
+        t.adjoint_setup(spp, target, **kw)
+        loss, img = t.forward(start_params(sc, 2), image=True)
+        rgb, sig = t.adjoint_samples()
+        out.append((loss, img.copy(), rgb.copy(), sig.copy(), t.backward().copy()))
+    assert out[0][0] == out[1][0]
+    for a, b in zip(out[0][1:], out[1][1:]):
+        assert np.array_equal(np.ascontiguousarray(a).view(np.uint32), np.ascontiguousarray(b).view(np.uint32))
+    t.close()
+
+
+@pytest.mark.parametrize("case", ["mis_off", "nee_off", "depth_2", "depth_8", "spot"])
+def test_vertex_vjp_matches_fp64_adjoint(case):
+    """The options the vertex's vector-Jacobian product branches on: no MIS
+    weights, no next event, the shallowest and deepest paths with a gradient,
+    a spot light's falloff."""
+    sc = scenes.inverse_box_scene()
+    st = scenes.inverse_settings(48, 48, 8)
+    p = start_params(sc, 4)
+    if case == "mis_off":
+        st.enable_mis = False
+    elif case == "nee_off":
+        st.enable_nee = False
+    elif case.startswith("depth"):
+        st.max_depth = int(case[-1])
+    else:
+        sc.lights[:, 8:13] = (0.1, -1.0, 0.05, 0.95, 0.3)   # axis, inner and outer cosine
+    t = CudaPathTracer(bvh="reference")
+    assert t.configure(st).ok and t.load_scene_snapshot(sc).ok and t.build_or_update_acceleration().ok
+    t.adjoint_setup(8)
+    _, target = t.forward(material_params(sc.materials), image=True)
+    t.adjoint_setup(8, target)
+    loss = t.forward(p)
+    g = t.backward().reshape(-1)[param_index()]
+    o_loss, o_grad, _ = oracle.load_adjoint().run(sc, st, p, target, 8, param_index(), threads=8)
+    print(f"{case}: loss {loss:.6e} (fp64 {o_loss:.6e}), gradient rel err {rel_err(g, o_grad):.2e}")
+    assert abs(loss - o_loss) <= 1e-3 * o_loss
+    assert np.linalg.norm(o_grad) > 0
+    assert rel_err(g, o_grad) <= GRAD_REL_TOL
+    t.close()

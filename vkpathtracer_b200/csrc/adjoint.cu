@@ -1,20 +1,20 @@
 // adjoint.cu -- forward / loss / backward kernels of differentiable rendering.
 //
-// Forward: one thread per (sample, pixel) path, inline closest-hit and
-// any-hit traversal, the float instantiation of the vertex math (adjoint.cuh)
-// in the reference's operation order, so each sample's radiance equals the
-// renderer's (the film test pins this bit-for-bit).
+// Forward: the renderer's trace and next-event arithmetic (adjoint.cuh) in the
+// reference's operation order, so each sample's radiance equals the renderer's
+// (the film test pins this bit-for-bit).  Up to one path per resident thread
+// it is one thread per (sample, pixel) path with inline traversal; above, a
+// wavefront that writes the vertex records (AdjTraceSource below).
 //
-// Backward ("re-trace from the seed"): the same path is replayed from its RNG
-// key, recording per vertex the ray, hit, throughput, roulette divisor, RNG
-// state and decision flags (64 bytes, at most 8 vertices), then swept in
-// reverse.  Each vertex's local Jacobian with respect to (ray origin, ray
-// direction, roughness) comes from the dual-number instantiation of the same
-// vertex math; albedo and emission enter affinely and are handled in closed
-// form.  Per-vertex parameter gradients are combined across the warp (lanes
-// grouped by material, butterfly sums) into per-warp shared-memory slots,
-// then per-block partials, then a fixed-order FP64 reduction: the gradient is
-// deterministic for a given launch shape.
+// Backward: from those records, or, where the forward did not write them,
+// "re-trace from the seed": the same path is replayed from its RNG key,
+// recording per vertex the ray, hit, throughput, roulette divisor, RNG state
+// and decision flags (64 bytes, at most 8 vertices).  The records are swept in
+// reverse with each vertex's vector-Jacobian product (adj_vertex_vjp); albedo
+// and emission enter affinely.  Per-vertex parameter gradients are added in a
+// fixed order to per-warp shared-memory slots, then per-block partials, then a
+// fixed-order FP64 reduction: the gradient is deterministic for a given launch
+// shape.
 #define VKPTC_INLINE_UNIT 1   // common.cuh
 #include "adjoint.cuh"
 #include <algorithm>
@@ -78,8 +78,8 @@ __device__ __forceinline__ float4 adj_primal(const DevScene& s, const DevSetting
     const uint32_t mi = mat_slot(s, __float_as_uint(sh.w));
     const MaterialRec m = load_material(s.materials + 16u * mi);
     uint32_t flags = 0u;
-    AdjVertex<float, V3> R;
-    adj_vertex<float, V3, kParity, false>(s, st, lights, depth, o, d, t, gn, m, clamp01(m.roughness), rng, flags, R);
+    AdjVertex R;
+    adj_vertex<kParity>(s, st, lights, depth, o, d, t, gn, m, clamp01(m.roughness), rng, flags, R);
     // emission, then the next-event term, in the renderer's order
     const bool emissive_model = m.model == 1u || m.emissive.x > 0.0f || m.emissive.y > 0.0f || m.emissive.z > 0.0f;
     if (!st.enable_nee || depth == 0u) rad = add(rad, mulv(thr, m.emissive));
@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(128, 5) k_adj_shade(DevScene s, DevSettings st
     bool next = false, shadow = false;
     uint32_t p = 0u;
     V3 sh_c = mk(0.0f, 0.0f, 0.0f);
-    AdjVertex<float, V3> R;
+    AdjVertex R;
     R.nee = false;
     if (j < n) {
       p = q[j];
@@ -281,8 +281,7 @@ __global__ void __launch_bounds__(128, 5) k_adj_shade(DevScene s, DevSettings st
         const uint32_t mi = mat_slot(s, __float_as_uint(sh.w));
         const MaterialRec m = load_material(s.materials + 16u * mi);
         uint32_t flags = 0u;
-        adj_vertex<float, V3, kParity, false>(s, st, s.lights, depth, o, d, h2.x, gn, m, clamp01(m.roughness), rng, flags,
-                                              R);
+        adj_vertex<kParity>(s, st, s.lights, depth, o, d, h2.x, gn, m, clamp01(m.roughness), rng, flags, R);
         const bool emissive_model = m.model == 1u || m.emissive.x > 0.0f || m.emissive.y > 0.0f || m.emissive.z > 0.0f;
         if (!st.enable_nee || depth == 0u) r = add(r, mulv(thr, m.emissive));
         else if (st.enable_mis && emissive_model) r = add(r, mul(mulv(thr, m.emissive), R.w_e));
@@ -415,19 +414,8 @@ __global__ void k_adj_loss_final(const double* part, int n, double scale, double
   if (threadIdx.x == 0) *loss = red[0] * scale;
 }
 
-__device__ __forceinline__ DV3 seed3(V3 v, int first) {
-  DV3 r = lift<DV3>(v);
-  r.x.g[first] = 1.0f;
-  r.y.g[first + 1] = 1.0f;
-  r.z.g[first + 2] = 1.0f;
-  return r;
-}
-
-__device__ __forceinline__ float warp_sum(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
+// Gradient slots (sum, rounding error) per warp: a set for each group of eight lanes.
+constexpr int kGradCopies = 4;
 
 // Reverse sweep of one path.  `g` is dL/d(path radiance).  The warp runs the
 // vertex loop in lockstep (k from the longest path's last vertex down) so the
@@ -435,7 +423,7 @@ __device__ __forceinline__ float warp_sum(float v) {
 template <bool kParity>
 __device__ __forceinline__ void adj_reverse(const DevScene& s, const DevSettings& st, const AdjRec* rec,
                                             uint32_t rec_stride, uint32_t nrec, bool lane_on, V3 g,
-                                            float* warp_grad) {
+                                            float* stage, float2* warp_grad, uint32_t grad_stride) {
   const uint32_t kmax = __reduce_max_sync(0xffffffffu, lane_on ? nrec : 0u);
   const int lane = threadIdx.x & 31;
   V3 aT = mk(0.0f, 0.0f, 0.0f), aO = aT, aD = aT;
@@ -456,102 +444,47 @@ __device__ __forceinline__ void adj_reverse(const DevScene& s, const DevSettings
         const V3 gn = mk(sh.x, sh.y, sh.z);
         mat = r.e.w;
         const MaterialRec m = load_material(s.materials + 16u * mat);
-        const V3 ov = mk(r.a.x, r.a.y, r.a.z), dv = mk(r.b.x, r.b.y, r.b.z);
-        const float th = r.a.w;
-        // Seeds: origin (0..2), direction (3..5), roughness (6).
-        const DV3 od = seed3(ov, 0), dd = seed3(dv, 3);
-        Dual rough = dconst(clamp01(m.roughness));
-        rough.g[6] = (m.roughness > 0.0f && m.roughness < 1.0f) ? 1.0f : 0.0f;
-        // Hit distance on the hit triangle's plane: t = (v0 - o).n / (d.n).
-        Dual tt = dconst(th);
-        const float dn = dot(dv, gn);
-        if (dn != 0.0f) {
-          tt.g[0] = -gn.x / dn;
-          tt.g[1] = -gn.y / dn;
-          tt.g[2] = -gn.z / dn;
-          tt.g[3] = -th * gn.x / dn;
-          tt.g[4] = -th * gn.y / dn;
-          tt.g[5] = -th * gn.z / dn;
-        }
-        uint64_t rng = static_cast<uint64_t>(r.e.x) | (static_cast<uint64_t>(r.e.y) << 32);
-        uint32_t fl = flags;
-        AdjVertex<Dual, DV3> R;
-        adj_vertex<Dual, DV3, kParity, true>(s, st, s.lights, static_cast<uint32_t>(k), od, dd, tt, gn, m, rough,
-                                             rng, fl, R);
-        float xb[kAdjN];
-#pragma unroll
-        for (int i = 0; i < kAdjN; ++i) xb[i] = 0.0f;
-        V3 aTk = mk(0.0f, 0.0f, 0.0f);
-        const V3 amask = mk((m.albedo.x > 0.0f && m.albedo.x < 1.5f) ? 1.0f : 0.0f,
-                            (m.albedo.y > 0.0f && m.albedo.y < 1.5f) ? 1.0f : 0.0f,
-                            (m.albedo.z > 0.0f && m.albedo.z < 1.5f) ? 1.0f : 0.0f);
-        // emission: (T * Le) * w_e
-        {
-          const float we = R.w_e.v;
-          const float se = g.x * T.x * m.emissive.x + g.y * T.y * m.emissive.y + g.z * T.z * m.emissive.z;
-#pragma unroll
-          for (int i = 0; i < kAdjN; ++i) xb[i] += se * R.w_e.g[i];
-          gv[4] = g.x * T.x * we;
-          gv[5] = g.y * T.y * we;
-          gv[6] = g.z * T.z * we;
-          aTk = mk(g.x * m.emissive.x * we, g.y * m.emissive.y * we, g.z * m.emissive.z * we);
-        }
-        // next-event term: (T * R) * w_n when it was added
-        if (R.nee && (flags & kVfNeeVis)) {
-          const float wn = R.w_n.v;
-          const V3 q = mk(g.x * T.x, g.y * T.y, g.z * T.z);
-          const float sr = q.x * R.q.radiance.x.v + q.y * R.q.radiance.y.v + q.z * R.q.radiance.z.v;
-#pragma unroll
-          for (int i = 0; i < kAdjN; ++i)
-            xb[i] += wn * (q.x * R.q.radiance.x.g[i] + q.y * R.q.radiance.y.g[i] + q.z * R.q.radiance.z.g[i]) +
-                     sr * R.w_n.g[i];
-          gv[0] += q.x * wn * R.q.p_alb.x * amask.x;
-          gv[1] += q.y * wn * R.q.p_alb.y * amask.y;
-          gv[2] += q.z * wn * R.q.p_alb.z * amask.z;
-          aTk = add(aTk, mk(g.x * R.q.radiance.x.v * wn, g.y * R.q.radiance.y.v * wn, g.z * R.q.radiance.z.v * wn));
-        }
-        // throughput T' = T * albedo / rr (rr held constant) and the next ray
-        if (flags & kVfCont) {
-          const float inv_rr = 1.0f / r.c.w;
-          const V3 W = albedo_effect0(m);
-          aTk = add(aTk, mk(aT.x * W.x * inv_rr, aT.y * W.y * inv_rr, aT.z * W.z * inv_rr));
-          gv[0] += aT.x * T.x * inv_rr * amask.x;
-          gv[1] += aT.y * T.y * inv_rr * amask.y;
-          gv[2] += aT.z * T.z * inv_rr * amask.z;
-          const DV3 o2 = add(R.hp, mul(R.out, 0.002f));
-#pragma unroll
-          for (int i = 0; i < kAdjN; ++i)
-            xb[i] += aO.x * o2.x.g[i] + aO.y * o2.y.g[i] + aO.z * o2.z.g[i] + aD.x * R.out.x.g[i] +
-                     aD.y * R.out.y.g[i] + aD.z * R.out.z.g[i];
-        }
-        gv[3] = xb[6];
-        aT = aTk;
-        aO = mk(xb[0], xb[1], xb[2]);
-        aD = mk(xb[3], xb[4], xb[5]);
+        adj_vertex_vjp<kParity>(s, st, s.lights, static_cast<uint32_t>(k), mk(r.a.x, r.a.y, r.a.z),
+                                mk(r.b.x, r.b.y, r.b.z), r.a.w, gn, m, T, r.c.w, flags,
+                                static_cast<uint64_t>(r.e.x) | (static_cast<uint64_t>(r.e.y) << 32), g, aT, aO, aD, gv);
       }
     }
-    // Combine lanes that hit the same material, one group at a time.
-    unsigned pending = __ballot_sync(0xffffffffu, mat != kMiss);
-    while (pending) {
-      const int leader = __ffs(pending) - 1;
-      const uint32_t gm = __shfl_sync(0xffffffffu, mat, leader);
-      const bool mine = mat == gm;
+    // Add the lanes' gradients to the warp's slots: eight lanes (seven at work,
+    // one per parameter) take every fourth source lane, each group of eight its
+    // own copy of the slots, in a fixed order.  A tree over the lanes of one
+    // material at a time cost 35 shuffles for each material of the warp
+    // (0.41 ms a sweep of 524,288 paths against 0.36).  The slots carry their
+    // rounding error along (Kahan): they take lanes one by one, so their
+    // chains are longer than a tree's.
+    __syncwarp();
+    float4* mine = reinterpret_cast<float4*>(stage) + 2 * lane;
+    mine[0] = make_float4(gv[0], gv[1], gv[2], gv[3]);
+    mine[1] = make_float4(gv[4], gv[5], gv[6], __uint_as_float(mat));
+    __syncwarp();
+    const int copy = lane >> 3, param = lane & 7;
+    if (param < static_cast<int>(kAdjParams)) {
+      float2* slots = warp_grad + copy * grad_stride + param;
 #pragma unroll
-      for (int i = 0; i < static_cast<int>(kAdjParams); ++i) {
-        const float v = warp_sum(mine ? gv[i] : 0.0f);
-        if (lane == leader) warp_grad[gm * kAdjParams + i] += v;
+      for (int j = 0; j < 32; j += kGradCopies) {
+        const float* src = stage + 8 * (j + copy);
+        const uint32_t mj = __float_as_uint(src[7]);
+        if (mj != kMiss) {
+          float2& c = slots[mj * kAdjParams];
+          const float y = src[param] - c.y, sum = c.x + y;
+          c.y = (sum - c.x) - y;
+          c.x = sum;
+        }
       }
-      pending &= ~__ballot_sync(0xffffffffu, mine);
     }
   }
 }
 
 // The backward runs as two kernels per chunk of paths: the replay (the
 // primal path again, with the traversal) writes every path's vertex records
-// and its radiance adjoint to device memory, and the reverse sweep (the dual-
-// number vertex code) reads them.  Split, each kernel's code is small enough
-// for the instruction cache -- the fused kernel's warps waited on instruction
-// fetch more than on anything else -- and each gets its own register budget.
+// and its radiance adjoint to device memory, and the reverse sweep reads them.
+// Split, each kernel's code is small enough for the instruction cache -- the
+// fused kernel's warps waited on instruction fetch more than on anything else
+// -- and each gets its own register budget.
 // Records: vertex k of chunk path i at recs[k * count + i] (lanes of a warp
 // touch consecutive records).
 template <bool kParity>
@@ -618,19 +551,28 @@ __global__ void __launch_bounds__(256) k_adj_gout(DevSettings st, const float4* 
 // The reverse sweep of one chunk: per-warp gradient slots in shared memory,
 // then one partial per block, added to the partials of the earlier chunks
 // (accumulate) in a fixed order, so the gradient is deterministic.
-#ifndef VKPTC_ADJ_REVERSE_BLOCKS
-#define VKPTC_ADJ_REVERSE_BLOCKS 4
-#endif
+//
+// Bound by instruction issue and fetch: a vertex is several hundred scalar
+// instructions on about 14 of 32 lanes, its record 64 bytes.  Differentiating
+// with seven-tangent dual numbers instead took 1.20 ms for 524,288 paths, two
+// thirds of its stalls waiting for instructions; the vector-Jacobian product
+// 0.41 ms, with the slots added through shared memory 0.36 and with their
+// rounding errors carried along 0.38.  Four blocks (128 registers) 0.36 ms,
+// five (96) 0.40, six (80) 0.42.
 template <bool kParity>
-__global__ void __launch_bounds__(128, VKPTC_ADJ_REVERSE_BLOCKS) k_adj_reverse(DevScene s, DevSettings st, uint32_t count,
+__global__ void __launch_bounds__(128, 4) k_adj_reverse(DevScene s, DevSettings st, uint32_t count,
                                                      const AdjRec* recs, const float4* gout, float* grad_part,
                                                      int accumulate) {
-  extern __shared__ float grads[];
+  extern __shared__ float4 smem_reverse[];   // per warp 32 x 8 floats of staging, then the slots
+  float* smem = reinterpret_cast<float*>(smem_reverse);
   const int warps = blockDim.x >> 5;
   const uint32_t stride = s.material_count * kAdjParams;
-  for (uint32_t i = threadIdx.x; i < stride * warps; i += blockDim.x) grads[i] = 0.0f;
+  float* stage = smem + (threadIdx.x >> 5) * 256;
+  float2* grads = reinterpret_cast<float2*>(smem + warps * 256);
+  const int slots = warps * kGradCopies;
+  for (uint32_t i = threadIdx.x; i < stride * slots; i += blockDim.x) grads[i] = make_float2(0.0f, 0.0f);
   __syncthreads();
-  float* warp_grad = grads + (threadIdx.x >> 5) * stride;
+  float2* warp_grad = grads + (threadIdx.x >> 5) * kGradCopies * stride;
   for (uint32_t base = blockIdx.x * blockDim.x; base < count; base += gridDim.x * blockDim.x) {
     const uint32_t i = base + threadIdx.x;
     V3 g = mk(0.0f, 0.0f, 0.0f);
@@ -640,12 +582,17 @@ __global__ void __launch_bounds__(128, VKPTC_ADJ_REVERSE_BLOCKS) k_adj_reverse(D
       g = mk(gv.x, gv.y, gv.z);
       nrec = __float_as_uint(gv.w);
     }
-    adj_reverse<kParity>(s, st, recs + (i < count ? i : 0u), count, nrec, nrec != 0u, g, warp_grad);
+    adj_reverse<kParity>(s, st, recs + (i < count ? i : 0u), count, nrec, nrec != 0u, g, stage,
+                         warp_grad, stride);
   }
   __syncthreads();
   for (uint32_t i = threadIdx.x; i < stride; i += blockDim.x) {
-    float v = 0.0f;
-    for (int w = 0; w < warps; ++w) v += grads[w * stride + i];
+    double sum = 0.0;
+    for (int w = 0; w < slots; ++w) {
+      const float2 c = grads[w * stride + i];
+      sum += static_cast<double>(c.x) - c.y;
+    }
+    const float v = static_cast<float>(sum);
     float* dst = grad_part + static_cast<size_t>(blockIdx.x) * stride + i;
     *dst = accumulate ? *dst + v : v;
   }
@@ -668,7 +615,7 @@ size_t AdjBackwardSmem(int block, int stack_cap, uint32_t materials) {
 }
 
 size_t AdjReverseSmem(int block, uint32_t materials) {
-  return static_cast<size_t>(block / 32) * materials * kAdjParams * sizeof(float);
+  return static_cast<size_t>(block / 32) * (256 + 2 * kGradCopies * materials * kAdjParams) * sizeof(float);
 }
 
 int AdjBlocksPerSm(AdjKernel k, int block, size_t smem, bool parity) {

@@ -2658,8 +2658,9 @@ int32_t vkptc_forward(vkptc_ctx* ctx, const float* params, uint32_t param_count,
   // skips the replay (the same records, so the same gradient).
   const bool record = !(a.desc.flags & VKPTC_ADJ_DECORRELATED) && a.stats.paths <= kAdjChunkPaths;
   // More paths than the per-path kernel has resident threads take the
-  // wavefront: 65,536 paths 0.23 ms per path against 0.27 as a wavefront, 98,304
-  // 0.35 against 0.31, 524,288 1.38 against 0.84 (94,720 resident threads).
+  // wavefront: 65,536 paths 0.23 ms with a path per thread against 0.27 as a
+  // wavefront, 98,304 0.35 against 0.31, 524,288 1.38 against 0.84 (94,720
+  // resident threads).
   const bool wavefront = record && a.stats.paths > static_cast<uint64_t>(l.grid) * l.block;
   a.recorded = false;
   AdjWaveLaunch wl{};
