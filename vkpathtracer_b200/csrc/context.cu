@@ -215,10 +215,7 @@ struct vkptc_ctx {
   DevBuf<float> d_film_invalid;
 
   // wave state
-  DevBuf<uint64_t> w_rng;
-  DevBuf<float4> w_ray_o, w_ray_d, w_thr, w_rad, w_sh_o, w_sh_d, w_sh_c;
-  DevBuf<float2> w_hit;
-  DevBuf<uint32_t> w_q0, w_q1, w_sh_path, w_counts;
+  DevBuf<uint8_t> w_arena;
   uint32_t wave_capacity = 0;
   size_t smem_configured = 48 * 1024;
   int max_smem_optin = 0;                 // the device's shared-memory limit per block
@@ -400,41 +397,40 @@ int32_t ensure_stack_smem(vkptc_ctx* c, const LaunchShape& ls) {
   return VKPTC_OK;
 }
 
+constexpr size_t kWaveBytesPerPath = 7u * sizeof(float4) + sizeof(uint64_t) + sizeof(float2) + 3u * sizeof(uint32_t);
+
 int32_t ensure_wave(vkptc_ctx* c, uint32_t paths) {
   if (paths <= c->wave_capacity) return VKPTC_OK;
-  const size_t n = paths;
-  VKPTC_CUDA(c, c->w_rng.alloc(n), "wave alloc");
-  VKPTC_CUDA(c, c->w_ray_o.alloc(n), "wave alloc");
-  VKPTC_CUDA(c, c->w_ray_d.alloc(n), "wave alloc");
-  VKPTC_CUDA(c, c->w_thr.alloc(n), "wave alloc");
-  VKPTC_CUDA(c, c->w_rad.alloc(n), "wave alloc");
-  VKPTC_CUDA(c, c->w_hit.alloc(n), "wave alloc");
-  VKPTC_CUDA(c, c->w_q0.alloc(n), "wave alloc");
-  VKPTC_CUDA(c, c->w_q1.alloc(n), "wave alloc");
-  VKPTC_CUDA(c, c->w_sh_path.alloc(n), "wave alloc");
-  VKPTC_CUDA(c, c->w_sh_o.alloc(n), "wave alloc");
-  VKPTC_CUDA(c, c->w_sh_d.alloc(n), "wave alloc");
-  VKPTC_CUDA(c, c->w_sh_c.alloc(n), "wave alloc");
-  VKPTC_CUDA(c, c->w_counts.alloc(8), "wave alloc");
-  c->wave_capacity = paths;
+  // One allocation for all of a wave's arrays: an allocation and its release
+  // cost 0.5 ms between them whatever their size, and the arrays number 13.
+  const size_t n = (static_cast<size_t>(paths) + 31u) & ~static_cast<size_t>(31);
+  c->wave_capacity = 0u;
+  VKPTC_CUDA(c, c->w_arena.alloc(n * kWaveBytesPerPath + 8u * sizeof(uint32_t)), "wave alloc");
+  c->wave_capacity = static_cast<uint32_t>(n);
   return VKPTC_OK;
 }
 
 WaveState wave_state(vkptc_ctx* c) {
   WaveState w{};
-  w.rng = c->w_rng.ptr;
-  w.ray_o = c->w_ray_o.ptr;
-  w.ray_d = c->w_ray_d.ptr;
-  w.thr = c->w_thr.ptr;
-  w.rad = c->w_rad.ptr;
-  w.hit = c->w_hit.ptr;
-  w.sh_path = c->w_sh_path.ptr;
-  w.sh_o = c->w_sh_o.ptr;
-  w.sh_d = c->w_sh_d.ptr;
-  w.sh_c = c->w_sh_c.ptr;
-  w.q[0] = c->w_q0.ptr;
-  w.q[1] = c->w_q1.ptr;
-  w.counts = c->w_counts.ptr;
+  uint8_t* at = c->w_arena.ptr;
+  const size_t n = c->wave_capacity;   // a multiple of 32: every array starts on 128 bytes
+  const auto take = [&at, n](auto*& array) {
+    array = reinterpret_cast<std::remove_reference_t<decltype(array)>>(at);
+    at += n * sizeof(*array);
+  };
+  take(w.ray_o);
+  take(w.ray_d);
+  take(w.thr);
+  take(w.rad);
+  take(w.sh_o);
+  take(w.sh_d);
+  take(w.sh_c);
+  take(w.rng);
+  take(w.hit);
+  take(w.q[0]);
+  take(w.q[1]);
+  take(w.sh_path);
+  take(w.counts);   // 8 words
   w.capacity = c->wave_capacity;
   return w;
 }
