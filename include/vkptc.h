@@ -508,7 +508,8 @@ typedef struct vkptc_batch_tuning {
   uint32_t use_graph;        /* persistent/loop modes: 1 = capture once, replay the CUDA graph
                                 (loop mode without a graph runs one host round trip per iteration) */
   uint32_t occupancy;        /* traversal kernels' register variant: 0..3 = at least 1..4 resident
-                                256-thread blocks per SM (fewer registers, more warps); 4 (loop
+                                256-thread blocks per SM (fewer registers, more warps; the loop
+                                driver's kernels run four for each of them); 4 (loop
                                 driver; the persistent driver takes it as 3) = at least 7 resident
                                 128-thread blocks per SM (72 registers), and the launch's block
                                 size becomes 128 */

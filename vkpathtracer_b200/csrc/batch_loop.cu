@@ -3,8 +3,8 @@
 // The persistent driver (batch.cu) runs the five stages of an iteration in
 // one cooperative kernel with grid barriers between them.  This driver runs
 // each stage as its own kernel, so a stage gets the register budget and
-// occupancy it needs (the traversal stages run at 64-80 registers, shading at
-// ~94), and the iterations are driven by the device: the stages form the body
+// occupancy it needs (the traversal stages run at 64-72 registers, shading at
+// 80), and the iterations are driven by the device: the stages form the body
 // of a CUDA graph while-node whose condition the last stage sets.  One
 // graph launch renders every job; no kernel ever waits on another.
 //
@@ -430,34 +430,28 @@ cudaError_t set_smem_attr(K kernel, int bytes) {
 }
 
 // Traversal stage variants: [triangle test][stats][register variant].
-// Variants 0..3: at least 1..4 resident 256-thread blocks per SM (at most
-// 255, 128, 80 and 64 registers); variant 4: at least 7 resident 128-thread
-// blocks (at most 72 registers, 28 warps; launched with 128 threads only).  Stats runs use
-// the unconstrained variant at the launch's block size.
+// Variants 0..3: four resident 256-thread blocks per SM (64 registers).  The
+// 64-job workload at 256 threads takes 519 ms with it, 537 with three blocks
+// (80 registers) and 10 % more with the 86-90 registers the compiler takes
+// when fewer are asked for.  Variant 4: at least 7 resident 128-thread blocks
+// (72 registers, 28 warps; launched with at most 128 threads), 513 ms.  Stats
+// runs use the unconstrained variant at the launch's block size.
 using LoopTraceFn = void (*)(const DevJob*, LoopPool, int, int2*, int, int, DevCounters*, uint32_t*);
 LoopTraceFn extend_fn(bool stats, int occ, bool wt) {
-  static const LoopTraceFn t[2][2][5] = {
-      {{k_lp_extend<false, 256, 1, false>, k_lp_extend<false, 256, 2, false>, k_lp_extend<false, 256, 3, false>,
-        k_lp_extend<false, 256, 4, false>, k_lp_extend<false, 128, 7, false>},
-       {k_lp_extend<true, 256, 1, false>, k_lp_extend<true, 256, 1, false>, k_lp_extend<true, 256, 1, false>,
-        k_lp_extend<true, 256, 1, false>, k_lp_extend<true, 128, 1, false>}},
-      {{k_lp_extend<false, 256, 1, true>, k_lp_extend<false, 256, 2, true>, k_lp_extend<false, 256, 3, true>,
-        k_lp_extend<false, 256, 4, true>, k_lp_extend<false, 128, 7, true>},
-       {k_lp_extend<true, 256, 1, true>, k_lp_extend<true, 256, 1, true>, k_lp_extend<true, 256, 1, true>,
-        k_lp_extend<true, 256, 1, true>, k_lp_extend<true, 128, 1, true>}}};
-  return t[wt ? 1 : 0][stats ? 1 : 0][occ < 0 ? 0 : (occ > 4 ? 4 : occ)];
+  static const LoopTraceFn t[2][2][2] = {
+      {{k_lp_extend<false, 256, 4, false>, k_lp_extend<false, 128, 7, false>},
+       {k_lp_extend<true, 256, 1, false>, k_lp_extend<true, 128, 1, false>}},
+      {{k_lp_extend<false, 256, 4, true>, k_lp_extend<false, 128, 7, true>},
+       {k_lp_extend<true, 256, 1, true>, k_lp_extend<true, 128, 1, true>}}};
+  return t[wt ? 1 : 0][stats ? 1 : 0][occ >= 4 ? 1 : 0];
 }
 LoopTraceFn shadow_fn(bool stats, int occ, bool wt) {
-  static const LoopTraceFn t[2][2][5] = {
-      {{k_lp_shadow<false, 256, 1, false>, k_lp_shadow<false, 256, 2, false>, k_lp_shadow<false, 256, 3, false>,
-        k_lp_shadow<false, 256, 4, false>, k_lp_shadow<false, 128, 7, false>},
-       {k_lp_shadow<true, 256, 1, false>, k_lp_shadow<true, 256, 1, false>, k_lp_shadow<true, 256, 1, false>,
-        k_lp_shadow<true, 256, 1, false>, k_lp_shadow<true, 128, 1, false>}},
-      {{k_lp_shadow<false, 256, 1, true>, k_lp_shadow<false, 256, 2, true>, k_lp_shadow<false, 256, 3, true>,
-        k_lp_shadow<false, 256, 4, true>, k_lp_shadow<false, 128, 7, true>},
-       {k_lp_shadow<true, 256, 1, true>, k_lp_shadow<true, 256, 1, true>, k_lp_shadow<true, 256, 1, true>,
-        k_lp_shadow<true, 256, 1, true>, k_lp_shadow<true, 128, 1, true>}}};
-  return t[wt ? 1 : 0][stats ? 1 : 0][occ < 0 ? 0 : (occ > 4 ? 4 : occ)];
+  static const LoopTraceFn t[2][2][2] = {
+      {{k_lp_shadow<false, 256, 4, false>, k_lp_shadow<false, 128, 7, false>},
+       {k_lp_shadow<true, 256, 1, false>, k_lp_shadow<true, 128, 1, false>}},
+      {{k_lp_shadow<false, 256, 4, true>, k_lp_shadow<false, 128, 7, true>},
+       {k_lp_shadow<true, 256, 1, true>, k_lp_shadow<true, 128, 1, true>}}};
+  return t[wt ? 1 : 0][stats ? 1 : 0][occ >= 4 ? 1 : 0];
 }
 
 // Shading stage variants: [parity][effects][sdf][exotic].
@@ -492,7 +486,7 @@ cudaError_t ConfigureBatchLoopSmem(size_t bytes) {
   cudaError_t e = cudaSuccess;
   for (int wt = 0; wt < 2 && e == cudaSuccess; ++wt)
     for (int st = 0; st < 2 && e == cudaSuccess; ++st)
-      for (int o = 0; o < 5 && e == cudaSuccess; ++o) {
+      for (int o = 3; o < 5 && e == cudaSuccess; ++o) {
         e = set_smem_attr(extend_fn(st != 0, o, wt != 0), b);
         if (e == cudaSuccess) e = set_smem_attr(shadow_fn(st != 0, o, wt != 0), b);
       }

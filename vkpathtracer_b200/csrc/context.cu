@@ -397,13 +397,26 @@ int32_t ensure_stack_smem(vkptc_ctx* c, const LaunchShape& ls) {
   return VKPTC_OK;
 }
 
+// Arrays of n elements one after the other in one allocation (n a multiple of
+// 32, so each starts on 128 bytes).  An allocation and its release cost 0.5 ms
+// between them whatever their size; a wave has 13 arrays, the loop driver's
+// pool 25.
+struct Carve {
+  uint8_t* at;
+  size_t n;
+  template <class T>
+  void take(T*& array) {
+    array = reinterpret_cast<T*>(at);
+    at += n * sizeof(T);
+  }
+};
+size_t carve_count(size_t n) { return (n + 31u) & ~static_cast<size_t>(31); }
+
 constexpr size_t kWaveBytesPerPath = 7u * sizeof(float4) + sizeof(uint64_t) + sizeof(float2) + 3u * sizeof(uint32_t);
 
 int32_t ensure_wave(vkptc_ctx* c, uint32_t paths) {
   if (paths <= c->wave_capacity) return VKPTC_OK;
-  // One allocation for all of a wave's arrays: an allocation and its release
-  // cost 0.5 ms between them whatever their size, and the arrays number 13.
-  const size_t n = (static_cast<size_t>(paths) + 31u) & ~static_cast<size_t>(31);
+  const size_t n = carve_count(paths);
   c->wave_capacity = 0u;
   VKPTC_CUDA(c, c->w_arena.alloc(n * kWaveBytesPerPath + 8u * sizeof(uint32_t)), "wave alloc");
   c->wave_capacity = static_cast<uint32_t>(n);
@@ -412,25 +425,20 @@ int32_t ensure_wave(vkptc_ctx* c, uint32_t paths) {
 
 WaveState wave_state(vkptc_ctx* c) {
   WaveState w{};
-  uint8_t* at = c->w_arena.ptr;
-  const size_t n = c->wave_capacity;   // a multiple of 32: every array starts on 128 bytes
-  const auto take = [&at, n](auto*& array) {
-    array = reinterpret_cast<std::remove_reference_t<decltype(array)>>(at);
-    at += n * sizeof(*array);
-  };
-  take(w.ray_o);
-  take(w.ray_d);
-  take(w.thr);
-  take(w.rad);
-  take(w.sh_o);
-  take(w.sh_d);
-  take(w.sh_c);
-  take(w.rng);
-  take(w.hit);
-  take(w.q[0]);
-  take(w.q[1]);
-  take(w.sh_path);
-  take(w.counts);   // 8 words
+  Carve carve{c->w_arena.ptr, c->wave_capacity};
+  carve.take(w.ray_o);
+  carve.take(w.ray_d);
+  carve.take(w.thr);
+  carve.take(w.rad);
+  carve.take(w.sh_o);
+  carve.take(w.sh_d);
+  carve.take(w.sh_c);
+  carve.take(w.rng);
+  carve.take(w.hit);
+  carve.take(w.q[0]);
+  carve.take(w.q[1]);
+  carve.take(w.sh_path);
+  carve.take(w.counts);   // 8 words
   w.capacity = c->wave_capacity;
   return w;
 }
@@ -1801,12 +1809,7 @@ struct vkptc_batch {
   DevBuf<float2> p_hit;
   DevBuf<int2> spill;
   // loop-driver state: two compacted path generations, shadow queue, finished list
-  DevBuf<uint32_t> l_job[2], l_local[2], l_depth[2];
-  DevBuf<uint64_t> l_rng[2];
-  DevBuf<float4> l_o[2], l_d[2], l_thr[2], l_rad[2];
-  DevBuf<float2> l_hit;
-  DevBuf<float4> l_sh_o, l_sh_d, l_sh_c, l_fin_rad;
-  DevBuf<uint32_t> l_sh_dst, l_fin_job, l_fin_local, l_ctl;
+  DevBuf<uint8_t> l_arena;
   DevBuf<DevCounters> d_ctr;
   DevBuf<uint32_t> d_err;
   size_t smem_configured = 48 * 1024;
@@ -1839,6 +1842,14 @@ int32_t bcuda(vkptc_batch* b, cudaError_t e, const char* what) {
   } while (0)
 
 constexpr uint32_t kDefaultPoolPaths = 1u << 21;
+// The loop driver's launches each have a tail, so it gains from a larger pool:
+// the 64-job workload takes 540 ms at 2^21 paths, 523 at 2^22, 514 at 2^23 and
+// 511 at 2^24 (252 bytes a path), eight small jobs 11.46, 11.34, 11.34 and 12.04.
+constexpr uint32_t kDefaultLoopPoolPaths = 1u << 23;
+constexpr size_t kLoopBytesPerPath = 2u * (4u * sizeof(float4) + sizeof(uint64_t) + 3u * sizeof(uint32_t)) +
+                                     4u * sizeof(float4) + sizeof(float2) + 3u * sizeof(uint32_t);
+// Steps between its refills: 540 ms at 16, 549 at 8.
+constexpr int kDefaultLoopSteps = 16;
 
 uint32_t job_samples(const vkptc_ctx* c, uint32_t limit) {
   const uint32_t spp = std::max(1u, c->settings.spp);
@@ -1947,7 +1958,7 @@ int32_t batch_run_pool(vkptc_batch* b, const vkptc_batch_tuning& t, uint32_t mod
   bl.block = t.block_size ? static_cast<int>(std::min(256u, std::max(32u, (t.block_size + 31u) / 32u * 32u))) : 128;
   bl.stack_cap = stack_cap;
   bl.smem_entries = std::min(stack_cap, t.stack_depth ? static_cast<int>(t.stack_depth) : kDefaultSmemEntries);
-  bl.steps = steps_word(t.steps, kDefaultSteps);
+  bl.steps = steps_word(t.steps, loop ? kDefaultLoopSteps : kDefaultSteps);
   bl.stream = b->stream;
   bl.parity = parity;
   bl.stats = b->config.collect_stats != 0u;
@@ -1961,9 +1972,12 @@ int32_t batch_run_pool(vkptc_batch* b, const vkptc_batch_tuning& t, uint32_t mod
     bl.exotic = bl.exotic || c->has_exotic || c->env_w != 0u;
   }
   // Register variant of the traversal kernels: 0..3 for both drivers; the loop
-  // driver's variant 4 runs its stages in 128-thread blocks.
+  // driver's variant 4 runs its stages in 128-thread blocks.  Variant 0 leaves
+  // the number of registers open: blocks that variant 4 can run take its 72
+  // (the 64-job workload 513 ms, 520 at 64 registers).
   bl.occupancy = static_cast<int>(std::min(loop ? 4u : 3u, t.occupancy));
   if (loop && bl.occupancy == 4) bl.block = 128;
+  if (loop && bl.occupancy == 0 && bl.block <= 128) bl.occupancy = 4;
   const size_t smem = StackSmemBytes(bl.block, bl.smem_entries);
   int max_optin = 0;
   cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device);
@@ -1996,42 +2010,35 @@ int32_t batch_run_pool(vkptc_batch* b, const vkptc_batch_tuning& t, uint32_t mod
   bl.spill = spill_entries ? b->spill.ptr : nullptr;
   bl.spill_shadow = spill_entries && loop ? b->spill.ptr + spill_entries : bl.spill;
   // ---- pool
-  const uint32_t cap = std::max<uint32_t>(1024u, t.pool_paths ? t.pool_paths : kDefaultPoolPaths);
+  const uint32_t by_default =
+      loop ? static_cast<uint32_t>(std::min<unsigned long long>(kDefaultLoopPoolPaths, total)) : kDefaultPoolPaths;
+  const uint32_t cap = std::max<uint32_t>(1024u, t.pool_paths ? t.pool_paths : by_default);
   const size_t n = cap;
   BatchPool P{};
   LoopPool LP{};
   if (loop) {
-    for (int g = 0; g < 2; ++g) {
-      VKPTC_BCUDA(b, b->l_job[g].alloc(n), "pool alloc");
-      VKPTC_BCUDA(b, b->l_local[g].alloc(n), "pool alloc");
-      VKPTC_BCUDA(b, b->l_depth[g].alloc(n), "pool alloc");
-      VKPTC_BCUDA(b, b->l_rng[g].alloc(n), "pool alloc");
-      VKPTC_BCUDA(b, b->l_o[g].alloc(n), "pool alloc");
-      VKPTC_BCUDA(b, b->l_d[g].alloc(n), "pool alloc");
-      VKPTC_BCUDA(b, b->l_thr[g].alloc(n), "pool alloc");
-      VKPTC_BCUDA(b, b->l_rad[g].alloc(n), "pool alloc");
-      LP.gen[g] = PathSoA{b->l_job[g].ptr, b->l_local[g].ptr, b->l_depth[g].ptr, b->l_rng[g].ptr,
-                          b->l_o[g].ptr,   b->l_d[g].ptr,     b->l_thr[g].ptr,   b->l_rad[g].ptr};
+    VKPTC_BCUDA(b, b->l_arena.alloc(carve_count(n) * kLoopBytesPerPath + kLoopCtlWords * sizeof(uint32_t)), "pool alloc");
+    Carve carve{b->l_arena.ptr, carve_count(n)};
+    for (PathSoA& gen : LP.gen) {
+      carve.take(gen.o);
+      carve.take(gen.d);
+      carve.take(gen.thr);
+      carve.take(gen.rad);
+      carve.take(gen.rng);
+      carve.take(gen.job);
+      carve.take(gen.local);
+      carve.take(gen.depth);
     }
-    VKPTC_BCUDA(b, b->l_hit.alloc(n), "pool alloc");
-    VKPTC_BCUDA(b, b->l_sh_o.alloc(n), "pool alloc");
-    VKPTC_BCUDA(b, b->l_sh_d.alloc(n), "pool alloc");
-    VKPTC_BCUDA(b, b->l_sh_c.alloc(n), "pool alloc");
-    VKPTC_BCUDA(b, b->l_sh_dst.alloc(n), "pool alloc");
-    VKPTC_BCUDA(b, b->l_fin_rad.alloc(n), "pool alloc");
-    VKPTC_BCUDA(b, b->l_fin_job.alloc(n), "pool alloc");
-    VKPTC_BCUDA(b, b->l_fin_local.alloc(n), "pool alloc");
-    VKPTC_BCUDA(b, b->l_ctl.alloc(kLoopCtlWords), "pool alloc");
+    carve.take(LP.hit);
+    carve.take(LP.sh_o);
+    carve.take(LP.sh_d);
+    carve.take(LP.sh_c);
+    carve.take(LP.sh_dst);
+    carve.take(LP.fin_rad);
+    carve.take(LP.fin_job);
+    carve.take(LP.fin_local);
+    LP.ctl = reinterpret_cast<uint32_t*>(carve.at);
     LP.capacity = cap;
-    LP.hit = b->l_hit.ptr;
-    LP.sh_o = b->l_sh_o.ptr;
-    LP.sh_d = b->l_sh_d.ptr;
-    LP.sh_c = b->l_sh_c.ptr;
-    LP.sh_dst = b->l_sh_dst.ptr;
-    LP.fin_rad = b->l_fin_rad.ptr;
-    LP.fin_job = b->l_fin_job.ptr;
-    LP.fin_local = b->l_fin_local.ptr;
-    LP.ctl = b->l_ctl.ptr;
   } else {
   VKPTC_BCUDA(b, b->p_job.alloc(n), "pool alloc");
   VKPTC_BCUDA(b, b->p_local.alloc(n), "pool alloc");
@@ -2146,7 +2153,7 @@ int32_t batch_run_pool(vkptc_batch* b, const vkptc_batch_tuning& t, uint32_t mod
                             "/" + std::to_string(bl.steps) + "/" + std::to_string(t.sample_limit) + "/" +
                             std::to_string(b->jobs.size()) + "/" +
                             std::to_string(reinterpret_cast<uintptr_t>(b->staging.ptr)) + "/" +
-                            std::to_string(reinterpret_cast<uintptr_t>(loop ? b->l_job[0].ptr : b->p_job.ptr));
+                            std::to_string(reinterpret_cast<uintptr_t>(loop ? static_cast<void*>(b->l_arena.ptr) : static_cast<void*>(b->p_job.ptr)));
     if (!b->graph || b->graph_key != key) {
       release_graph(b);
       VKPTC_BCUDA(b, cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal), "graph capture");
