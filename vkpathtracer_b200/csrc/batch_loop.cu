@@ -144,8 +144,6 @@ struct LoopSdfShadowSource {
   }
 };
 
-constexpr int kSdfStepsPerRefill = 8;
-
 __device__ __forceinline__ void flush_sdf(DevCounters* ctr, const SdfCount& c) {
   warp_count(&ctr->sdf_tests, c.tests);
   warp_count(&ctr->sdf_steps, c.steps);
@@ -283,7 +281,7 @@ __global__ void __launch_bounds__(256) k_lp_sdf(const DevJob* __restrict__ jobs,
   if (n == 0u) return;
   SdfCount c;
   const LoopSdfExtSource src{jobs, P.gen[cur], P.hit};
-  sdf_persistent<LoopSdfExtSource, false>(src, n, &P.ctl[kLFetchSdf], kSdfStepsPerRefill, c);
+  sdf_persistent<LoopSdfExtSource, false>(src, n, &P.ctl[kLFetchSdf], kSdfSteps, c);
   flush_sdf(ctr, c);
 }
 
@@ -292,7 +290,7 @@ __global__ void __launch_bounds__(256) k_lp_sdf_shadow(const DevJob* __restrict_
   if (n == 0u) return;
   SdfCount c;
   const LoopSdfShadowSource src{jobs, P};
-  sdf_persistent<LoopSdfShadowSource, true>(src, n, &P.ctl[kLFetchSdfShadow], kSdfStepsPerRefill, c);
+  sdf_persistent<LoopSdfShadowSource, true>(src, n, &P.ctl[kLFetchSdfShadow], kSdfSteps, c);
   flush_sdf(ctr, c);
 }
 

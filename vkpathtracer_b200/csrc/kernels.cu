@@ -339,7 +339,6 @@ __global__ void __launch_bounds__(256, 4) k_trace(DevScene s, WaveState w, const
 // One sphere-tracing step per lane and call, lanes refilled as their queries
 // finish, so a warp is not held by its longest march (inside the shading stage
 // the marches took nine tenths of a frame of the SDF gallery).
-constexpr int kWaveSdfSteps = 8;   // march steps between refills
 
 __device__ __forceinline__ void flush_sdf(DevCounters* ctr, const SdfCount& c) {
   warp_count(&ctr->sdf_tests, c.tests);
@@ -352,7 +351,7 @@ __global__ void __launch_bounds__(256) k_sdf(DevScene s, WaveState w, const uint
   const uint32_t n = w.counts[kWaveExt + (depth & 1u)];
   SdfCount c;
   const WaveSdfExtSource src{s.sdf, s.sdf_count, q, w.ray_o, w.ray_d, w.hit};
-  sdf_persistent<WaveSdfExtSource, false>(src, n, &w.counts[kWaveFetchSdf], kWaveSdfSteps, c);
+  sdf_persistent<WaveSdfExtSource, false>(src, n, &w.counts[kWaveFetchSdf], kSdfSteps, c);
   flush_sdf(ctr, c);
 }
 
@@ -360,7 +359,7 @@ __global__ void __launch_bounds__(256) k_sdf_shadow(DevScene s, WaveState w, uin
   const uint32_t n = w.counts[kWaveShadow + (depth & 1u)];
   SdfCount c;
   const WaveSdfShadowSource src{s.sdf, s.sdf_count, w.sh_o, w.sh_d, w.sh_path};
-  sdf_persistent<WaveSdfShadowSource, true>(src, n, &w.counts[kWaveFetchSdfShadow], kWaveSdfSteps, c);
+  sdf_persistent<WaveSdfShadowSource, true>(src, n, &w.counts[kWaveFetchSdfShadow], kSdfSteps, c);
   flush_sdf(ctr, c);
 }
 
