@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(256) k_adj_raygen(DevScene s, DevSettings st, 
     rad[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     w.q[0][j] = j;
   }
-  if (blockIdx.x == 0 && threadIdx.x < 8u) w.counts[threadIdx.x] = threadIdx.x == 0u ? n : 0u;
+  if (blockIdx.x == 0 && threadIdx.x < 8u) ctl_word(w.counts, threadIdx.x) = threadIdx.x == 0u ? n : 0u;
 }
 
 __global__ void __launch_bounds__(256, 4) k_adj_trace(DevScene s, AdjWave w, const uint32_t* q, uint32_t depth,
@@ -228,10 +228,10 @@ __global__ void __launch_bounds__(256, 4) k_adj_trace(DevScene s, AdjWave w, con
                                                       int steps, uint32_t* err) {
   extern __shared__ int2 smem_stack[];
   const uint32_t cur = depth & 1u;
-  const uint32_t n_ext = w.counts[cur], n_sh = depth > 0u ? w.counts[2u + (cur ^ 1u)] : 0u;
+  const uint32_t n_ext = ctl_word(w.counts, cur), n_sh = depth > 0u ? ctl_word(w.counts, 2u + (cur ^ 1u)) : 0u;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
-    w.counts[cur ^ 1u] = 0u;
-    w.counts[2u + cur] = 0u;
+    ctl_word(w.counts, cur ^ 1u) = 0u;
+    ctl_word(w.counts, 2u + cur) = 0u;
   }
   const AdjTraceSource src{geo_of(s), q, w, rad, rec_prev, n_ext};
   const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(256, 4) k_adj_trace(DevScene s, AdjWave w, con
                           static_cast<int>(gridDim.x * blockDim.x), total};
   TraceStats st;
   uint32_t lerr = 0u;
-  persistent_traverse<AdjTraceSource, kQueryMixed, false>(src, n_ext + n_sh, &w.counts[4], stk, steps, st, st, lerr);
+  persistent_traverse<AdjTraceSource, kQueryMixed, false>(src, n_ext + n_sh, &ctl_word(w.counts, 4), stk, steps, st, st, lerr);
   if (lerr) atomicOr(err, lerr);
 }
 
@@ -250,8 +250,8 @@ __global__ void __launch_bounds__(128, 5) k_adj_shade(DevScene s, DevSettings st
                                                       const uint32_t* q, uint32_t* qn, uint32_t depth, float4* rad,
                                                       AdjRec* rec, uint32_t* nrec) {
   const uint32_t cur = depth & 1u;
-  const uint32_t n = w.counts[cur];
-  if (blockIdx.x == 0 && threadIdx.x == 0) w.counts[4] = 0u;
+  const uint32_t n = ctl_word(w.counts, cur);
+  if (blockIdx.x == 0 && threadIdx.x == 0) ctl_word(w.counts, 4) = 0u;
   for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
     const uint32_t j = base + threadIdx.x;
     bool next = false, shadow = false;
@@ -323,9 +323,9 @@ __global__ void __launch_bounds__(128, 5) k_adj_shade(DevScene s, DevSettings st
       if (!next) nrec[p] = depth + 1u;
       rad[p] = make_float4(r.x, r.y, r.z, 0.0f);
     }
-    const uint32_t slot_n = warp_append(&w.counts[cur ^ 1u], next);
+    const uint32_t slot_n = warp_append(&ctl_word(w.counts, cur ^ 1u), next);
     if (next) qn[slot_n] = p;
-    const uint32_t slot_s = warp_append(&w.counts[2u + cur], shadow);
+    const uint32_t slot_s = warp_append(&ctl_word(w.counts, 2u + cur), shadow);
     if (shadow) {
       w.sh_path[slot_s] = p;
       w.sh_o[slot_s] = make_float4(R.q.origin.x, R.q.origin.y, R.q.origin.z, R.q.remain);

@@ -37,7 +37,7 @@ struct AdjWave {
   uint64_t* rng;
   float2* hit;
   uint32_t *q[2], *sh_path;
-  uint32_t* counts;       // 8 words
+  uint32_t* counts;       // control words (ctl_word)
 };
 struct AdjWaveLaunch {
   int grid, block, smem_entries, stack_cap, steps;

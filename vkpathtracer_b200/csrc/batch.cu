@@ -331,9 +331,9 @@ __global__ void __launch_bounds__(256, kMinBlocks) k_batch(const DevJob* __restr
 __global__ void __launch_bounds__(256) k_staging_accumulate(const DevJob* jobs, uint32_t jb, DevCounters* ctr) {
   const DevJob& J = jobs[jb];
   const float clampv = J.settings.firefly_clamp;
+  uint32_t samples = 0u, segs = 0u, dropped = 0u;
   for (uint32_t base = blockIdx.x * blockDim.x; base < J.pixels; base += gridDim.x * blockDim.x) {
     const uint32_t px = base + threadIdx.x;
-    uint32_t samples = 0u, segs = 0u, dropped = 0u;
     if (px < J.pixels) {
       float4 acc = J.film.sum[px];
       uint32_t cnt = J.film.count[px];
@@ -359,10 +359,8 @@ __global__ void __launch_bounds__(256) k_staging_accumulate(const DevJob* jobs, 
       J.film.sum[px] = acc;
       J.film.count[px] = cnt;
     }
-    warp_count(&ctr->samples, samples);
-    warp_count(&ctr->rays, segs);
-    warp_count(&ctr->dropped, dropped);
   }
+  block_count3(&ctr->samples, samples, &ctr->rays, segs, &ctr->dropped, dropped);
 }
 
 // Pool reset before a run: every slot free, all queues and counters zero.

@@ -175,8 +175,7 @@ __device__ __forceinline__ void flush_stats(DevCounters* ctr, const TraceStats& 
 
 // ---------------------------------------------------------------- stages
 __global__ void k_lp_init(uint32_t* ctl) {
-  const uint32_t i = threadIdx.x;
-  if (i < static_cast<uint32_t>(kLoopCtlWords)) ctl[i] = 0u;
+  for (uint32_t i = threadIdx.x; i < kCtlStride * kLoopCtlWords; i += blockDim.x) ctl[i] = 0u;
 }
 
 // 1: REGEN claims work items and queue slots once per block and iteration;
@@ -187,17 +186,17 @@ __global__ void k_lp_init(uint32_t* ctl) {
 template <bool kParity>
 __global__ void __launch_bounds__(256) k_lp_regen(const DevJob* __restrict__ jobs, uint32_t job_count,
                                                   unsigned long long total, LoopPool P) {
-  const uint32_t cur = P.ctl[kLCur];
-  uint32_t* count = P.ctl + kLCount0 + cur;
+  const uint32_t cur = ctl_word(P.ctl, kLCur);
+  uint32_t* count = &ctl_word(P.ctl, kLCount0 + cur);
   // The count itself grows while this kernel appends; every block sizes its
   // share from the value the previous finish stage recorded.
-  const uint32_t room = P.capacity - P.ctl[kLBase];
+  const uint32_t room = P.capacity - ctl_word(P.ctl, kLBase);
   if (block_leader()) {
-    P.ctl[kLFetchExt] = 0u;
-    P.ctl[kLFetchSdf] = 0u;
+    ctl_word(P.ctl, kLFetchExt) = 0u;
+    ctl_word(P.ctl, kLFetchSdf) = 0u;
   }
   const PathSoA A = P.gen[cur];
-  unsigned long long* work_next = reinterpret_cast<unsigned long long*>(P.ctl + kLWork);
+  unsigned long long* work_next = reinterpret_cast<unsigned long long*>(&ctl_word(P.ctl, kLWork));
   const uint32_t gthreads = gridDim.x * blockDim.x;
 #if VKPTC_REGEN_BLOCK
   // One claim per block and iteration: the threads that take a path are a
@@ -263,34 +262,34 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_lp_extend(const DevJob
                                                                int2* spill, int total_cap, int steps, DevCounters* ctr,
                                                                uint32_t* err) {
   extern __shared__ int2 smem_stack[];
-  const uint32_t cur = P.ctl[kLCur];
-  const uint32_t n = P.ctl[kLCount0 + cur];
+  const uint32_t cur = ctl_word(P.ctl, kLCur);
+  const uint32_t n = ctl_word(P.ctl, kLCount0 + cur);
   if (n == 0u) return;
   const TwoLevelStack stk = loop_stack(smem_stack, scap, spill, total_cap);
   TraceStats st;
   uint32_t lerr = 0u;
   const LoopExtendSource src{jobs, P.gen[cur], P.hit};
-  persistent_traverse<LoopExtendSource, false, kStats, kWt>(src, n, &P.ctl[kLFetchExt], stk, steps, st, st, lerr);
+  persistent_traverse<LoopExtendSource, false, kStats, kWt>(src, n, &ctl_word(P.ctl, kLFetchExt), stk, steps, st, st, lerr);
   flush_stats<kStats>(ctr, st, false);
   if (lerr) atomicOr(err, lerr);
 }
 
 __global__ void __launch_bounds__(256) k_lp_sdf(const DevJob* __restrict__ jobs, LoopPool P, DevCounters* ctr) {
-  const uint32_t cur = P.ctl[kLCur];
-  const uint32_t n = P.ctl[kLCount0 + cur];
+  const uint32_t cur = ctl_word(P.ctl, kLCur);
+  const uint32_t n = ctl_word(P.ctl, kLCount0 + cur);
   if (n == 0u) return;
   SdfCount c;
   const LoopSdfExtSource src{jobs, P.gen[cur], P.hit};
-  sdf_persistent<LoopSdfExtSource, false>(src, n, &P.ctl[kLFetchSdf], kSdfSteps, c);
+  sdf_persistent<LoopSdfExtSource, false>(src, n, &ctl_word(P.ctl, kLFetchSdf), kSdfSteps, c);
   flush_sdf(ctr, c);
 }
 
 __global__ void __launch_bounds__(256) k_lp_sdf_shadow(const DevJob* __restrict__ jobs, LoopPool P, DevCounters* ctr) {
-  const uint32_t n = P.ctl[kLShadow];
+  const uint32_t n = ctl_word(P.ctl, kLShadow);
   if (n == 0u) return;
   SdfCount c;
   const LoopSdfShadowSource src{jobs, P};
-  sdf_persistent<LoopSdfShadowSource, true>(src, n, &P.ctl[kLFetchSdfShadow], kSdfSteps, c);
+  sdf_persistent<LoopSdfShadowSource, true>(src, n, &ctl_word(P.ctl, kLFetchSdfShadow), kSdfSteps, c);
   flush_sdf(ctr, c);
 }
 
@@ -302,8 +301,8 @@ __global__ void __launch_bounds__(256) k_lp_sdf_shadow(const DevJob* __restrict_
 template <bool kParity, bool kEffects, bool kSdf, bool kExotic>
 __global__ void __launch_bounds__(256, 3) k_lp_shade(const DevJob* __restrict__ jobs, LoopPool P,
                                                      DevCounters* ctr) {
-  const uint32_t cur = P.ctl[kLCur];
-  const uint32_t n = P.ctl[kLCount0 + cur];
+  const uint32_t cur = ctl_word(P.ctl, kLCur);
+  const uint32_t n = ctl_word(P.ctl, kLCount0 + cur);
   const PathSoA A = P.gen[cur], B = P.gen[cur ^ 1u];
   const uint32_t gthreads = gridDim.x * blockDim.x;
   uint32_t shadow_tests = 0u;
@@ -333,7 +332,7 @@ __global__ void __launch_bounds__(256, 3) k_lp_shade(const DevJob* __restrict__ 
       shadow = R.shadow;
       shadow_tests += R.shadow_tests;
     }
-    const uint32_t qn = warp_append(&P.ctl[kLCount0 + (cur ^ 1u)], next);
+    const uint32_t qn = warp_append(&ctl_word(P.ctl, kLCount0 + (cur ^ 1u)), next);
     if (next) {
       B.job[qn] = jb;
       B.local[qn] = local;
@@ -344,13 +343,13 @@ __global__ void __launch_bounds__(256, 3) k_lp_shade(const DevJob* __restrict__ 
       B.thr[qn] = make_float4(pr.thr.x, pr.thr.y, pr.thr.z, 0.0f);
       B.rad[qn] = make_float4(pr.rad.x, pr.rad.y, pr.rad.z, pr.segs);
     }
-    const uint32_t qf = warp_append(&P.ctl[kLFin0 + cur], fin);
+    const uint32_t qf = warp_append(&ctl_word(P.ctl, kLFin0 + cur), fin);
     if (fin) {
       P.fin_rad[qf] = make_float4(pr.rad.x, pr.rad.y, pr.rad.z, pr.segs);
       P.fin_job[qf] = jb;
       P.fin_local[qf] = local;
     }
-    const uint32_t qs = warp_append(&P.ctl[kLShadow], shadow);
+    const uint32_t qs = warp_append(&ctl_word(P.ctl, kLShadow), shadow);
     if (shadow) {
       P.sh_o[qs] = make_float4(R.sh_o.x, R.sh_o.y, R.sh_o.z, R.sh_t);
       P.sh_d[qs] = make_float4(R.sh_d.x, R.sh_d.y, R.sh_d.z, __uint_as_float(jb));
@@ -366,15 +365,15 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_lp_shadow(const DevJob
                                                                int2* spill, int total_cap, int steps, DevCounters* ctr,
                                                                uint32_t* err) {
   extern __shared__ int2 smem_stack[];
-  const uint32_t n = P.ctl[kLShadow];
+  const uint32_t n = ctl_word(P.ctl, kLShadow);
   if (n == 0u) return;
-  const uint32_t cur = P.ctl[kLCur];
+  const uint32_t cur = ctl_word(P.ctl, kLCur);
   const TwoLevelStack stk = loop_stack(smem_stack, scap, spill, total_cap);
   TraceStats st;
   uint32_t lerr = 0u;
   // The queries of the previous shading stage; their survivors are generation `cur` now.
   const LoopShadowSource src{jobs, P, P.gen[cur]};
-  persistent_traverse<LoopShadowSource, true, kStats, kWt>(src, n, &P.ctl[kLFetchShadow], stk, steps, st, st, lerr);
+  persistent_traverse<LoopShadowSource, true, kStats, kWt>(src, n, &ctl_word(P.ctl, kLFetchShadow), stk, steps, st, st, lerr);
   flush_stats<kStats>(ctr, st, true);
   if (lerr) atomicOr(err, lerr);
 }
@@ -383,15 +382,15 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_lp_shadow(const DevJob
 // added by the shadow stage) to their jobs' staging slots; then the words the
 // coming shading stage appends to start from zero.
 __global__ void __launch_bounds__(256) k_lp_drain(const DevJob* __restrict__ jobs, LoopPool P) {
-  const uint32_t cur = P.ctl[kLCur];
+  const uint32_t cur = ctl_word(P.ctl, kLCur);
   if (block_leader()) {
-    P.ctl[kLCount0 + (cur ^ 1u)] = 0u;
-    P.ctl[kLFin0 + cur] = 0u;
-    P.ctl[kLShadow] = 0u;
-    P.ctl[kLFetchShadow] = 0u;
-    P.ctl[kLFetchSdfShadow] = 0u;
+    ctl_word(P.ctl, kLCount0 + (cur ^ 1u)) = 0u;
+    ctl_word(P.ctl, kLFin0 + cur) = 0u;
+    ctl_word(P.ctl, kLShadow) = 0u;
+    ctl_word(P.ctl, kLFetchShadow) = 0u;
+    ctl_word(P.ctl, kLFetchSdfShadow) = 0u;
   }
-  const uint32_t n = P.ctl[kLFin0 + (cur ^ 1u)];
+  const uint32_t n = ctl_word(P.ctl, kLFin0 + (cur ^ 1u));
   for (uint32_t f = blockIdx.x * blockDim.x + threadIdx.x; f < n; f += gridDim.x * blockDim.x) {
     const DevJob& J = jobs[P.fin_job[f]];
     J.staging[P.fin_local[f]] = P.fin_rad[f];
@@ -403,15 +402,15 @@ __global__ void __launch_bounds__(256) k_lp_drain(const DevJob* __restrict__ job
 // finished paths for the next iteration's shadow and drain stages.
 __global__ void k_lp_decide(unsigned long long total, LoopPool P, cudaGraphConditionalHandle handle) {
   if (threadIdx.x != 0u) return;
-  const uint32_t cur = P.ctl[kLCur];
-  const unsigned long long work = *reinterpret_cast<const unsigned long long*>(P.ctl + kLWork);
-  const uint32_t survivors = P.ctl[kLCount0 + (cur ^ 1u)];
+  const uint32_t cur = ctl_word(P.ctl, kLCur);
+  const unsigned long long work = *reinterpret_cast<const unsigned long long*>(&ctl_word(P.ctl, kLWork));
+  const uint32_t survivors = ctl_word(P.ctl, kLCount0 + (cur ^ 1u));
   const uint32_t more =
-      (survivors > 0u || work < total || P.ctl[kLShadow] > 0u || P.ctl[kLFin0 + cur] > 0u) ? 1u : 0u;
-  P.ctl[kLMore] = more;
-  P.ctl[kLBase] = survivors;
-  P.ctl[kLCur] = cur ^ 1u;
-  P.ctl[kLIter] += 1u;
+      (survivors > 0u || work < total || ctl_word(P.ctl, kLShadow) > 0u || ctl_word(P.ctl, kLFin0 + cur) > 0u) ? 1u : 0u;
+  ctl_word(P.ctl, kLMore) = more;
+  ctl_word(P.ctl, kLBase) = survivors;
+  ctl_word(P.ctl, kLCur) = cur ^ 1u;
+  ctl_word(P.ctl, kLIter) += 1u;
   if (handle) cudaGraphSetConditional(handle, more);
 }
 
@@ -492,7 +491,7 @@ cudaError_t ConfigureBatchLoopSmem(size_t bytes) {
 }
 
 cudaError_t LaunchBatchLoopInit(const LoopPool& pool, cudaStream_t stream) {
-  k_lp_init<<<1, kLoopCtlWords, 0, stream>>>(pool.ctl);
+  k_lp_init<<<1, 256, 0, stream>>>(pool.ctl);
   return cudaGetLastError();
 }
 

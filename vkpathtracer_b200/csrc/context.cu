@@ -113,7 +113,8 @@ struct AdjointState {
 // a 256-byte boundary.
 constexpr size_t kNoAllocPathBytes = 8 + 7 * 16 + 8 + 3 * 4;
 constexpr size_t kNoAllocArrays = 12;
-constexpr size_t kNoAllocBytes = VKPTC_NOALLOC_MAX_PATHS * kNoAllocPathBytes + (kNoAllocArrays + 1) * 256;
+constexpr size_t kNoAllocBytes = VKPTC_NOALLOC_MAX_PATHS * kNoAllocPathBytes + (kNoAllocArrays + 1) * 256 +
+                                 kCtlStride * kWaveCtlWords * sizeof(uint32_t);
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
 
 // Live contexts per device (a batch's jobs are contexts too): when the last
@@ -418,7 +419,7 @@ int32_t ensure_wave(vkptc_ctx* c, uint32_t paths) {
   if (paths <= c->wave_capacity) return VKPTC_OK;
   const size_t n = carve_count(paths);
   c->wave_capacity = 0u;
-  VKPTC_CUDA(c, c->w_arena.alloc(n * kWaveBytesPerPath + 8u * sizeof(uint32_t)), "wave alloc");
+  VKPTC_CUDA(c, c->w_arena.alloc(n * kWaveBytesPerPath + kCtlStride * kWaveCtlWords * sizeof(uint32_t)), "wave alloc");
   c->wave_capacity = static_cast<uint32_t>(n);
   return VKPTC_OK;
 }
@@ -438,7 +439,7 @@ WaveState wave_state(vkptc_ctx* c) {
   carve.take(w.q[0]);
   carve.take(w.q[1]);
   carve.take(w.sh_path);
-  carve.take(w.counts);   // 8 words
+  carve.take(w.counts);   // kWaveCtlWords of them
   w.capacity = c->wave_capacity;
   return w;
 }
@@ -2017,7 +2018,7 @@ int32_t batch_run_pool(vkptc_batch* b, const vkptc_batch_tuning& t, uint32_t mod
   BatchPool P{};
   LoopPool LP{};
   if (loop) {
-    VKPTC_BCUDA(b, b->l_arena.alloc(carve_count(n) * kLoopBytesPerPath + kLoopCtlWords * sizeof(uint32_t)), "pool alloc");
+    VKPTC_BCUDA(b, b->l_arena.alloc(carve_count(n) * kLoopBytesPerPath + kCtlStride * kLoopCtlWords * sizeof(uint32_t)), "pool alloc");
     Carve carve{b->l_arena.ptr, carve_count(n)};
     for (PathSoA& gen : LP.gen) {
       carve.take(gen.o);
@@ -2198,7 +2199,7 @@ int32_t batch_run_pool(vkptc_batch* b, const vkptc_batch_tuning& t, uint32_t mod
                                               timing ? b->marks : nullptr),
                   "loop iteration");
       uint32_t more = 0;
-      VKPTC_BCUDA(b, cudaMemcpyAsync(&more, LP.ctl + kLoopCtlMore, sizeof(more), cudaMemcpyDeviceToHost, b->stream),
+      VKPTC_BCUDA(b, cudaMemcpyAsync(&more, LP.ctl + kCtlStride * kLoopCtlMore, sizeof(more), cudaMemcpyDeviceToHost, b->stream),
                   "loop condition");
       VKPTC_BCUDA(b, cudaStreamSynchronize(b->stream), "loop sync");
       if (timing) {
@@ -2225,7 +2226,7 @@ int32_t batch_run_pool(vkptc_batch* b, const vkptc_batch_tuning& t, uint32_t mod
   DevCounters dc{};
   VKPTC_BCUDA(b, cudaMemcpy(&dc, b->d_ctr.ptr, sizeof(dc), cudaMemcpyDeviceToHost), "counters");
   uint32_t iterations = 0;
-  VKPTC_BCUDA(b, cudaMemcpy(&iterations, loop ? LP.ctl + kLoopCtlIterations : P.ctl + kBatchCtlIterations,
+  VKPTC_BCUDA(b, cudaMemcpy(&iterations, loop ? LP.ctl + kCtlStride * kLoopCtlIterations : P.ctl + kBatchCtlIterations,
                             sizeof(iterations), cudaMemcpyDeviceToHost),
               "iterations");
   b->stats.segments = dc.rays;
@@ -2444,7 +2445,7 @@ extern "C" int32_t vkptc_render_tile_noalloc(vkptc_ctx* ctx, const vkptc_tile* t
   w.q[0] = carve<uint32_t>(cur, n);
   w.q[1] = carve<uint32_t>(cur, n);
   w.sh_path = carve<uint32_t>(cur, n);
-  w.counts = carve<uint32_t>(cur, 8);   // set by the raygen stage of every call
+  w.counts = carve<uint32_t>(cur, kCtlStride * kWaveCtlWords);   // set by the raygen stage of every call
   w.capacity = VKPTC_NOALLOC_MAX_PATHS;
   if (static_cast<size_t>(cur - base) > kNoAllocBytes) return fail(ctx, VKPTC_INTERNAL_ERROR, "scratch layout overflow");
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;

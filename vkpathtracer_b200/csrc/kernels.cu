@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(256) k_raygen(DevScene s, DevSettings st, Wave
     w.rad[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     w.q[0][i] = i;
   }
-  if (blockIdx.x == 0 && threadIdx.x < 8u) w.counts[threadIdx.x] = threadIdx.x == kWaveExt ? n : 0u;
+  if (blockIdx.x == 0 && threadIdx.x < 8u) ctl_word(w.counts, threadIdx.x) = threadIdx.x == kWaveExt ? n : 0u;
 }
 
 // ===================================================================== trace
@@ -307,20 +307,20 @@ __global__ void __launch_bounds__(256, 4) k_trace(DevScene s, WaveState w, const
                                                   DevCounters* ctr, uint32_t* err) {
   extern __shared__ int2 smem_stack[];
   const uint32_t cur = depth & 1u;
-  const uint32_t n_ext = (parts & 1u) ? w.counts[kWaveExt + cur] : 0u;
-  const uint32_t n_sh = (parts & 2u) ? w.counts[kWaveShadow + (cur ^ 1u)] : 0u;
+  const uint32_t n_ext = (parts & 1u) ? ctl_word(w.counts, kWaveExt + cur) : 0u;
+  const uint32_t n_sh = (parts & 2u) ? ctl_word(w.counts, kWaveShadow + (cur ^ 1u)) : 0u;
   if (blockIdx.x == 0 && threadIdx.x == 0 && (parts & 1u)) {
-    w.counts[kWaveExt + (cur ^ 1u)] = 0u;
-    w.counts[kWaveShadow + cur] = 0u;
-    w.counts[kWaveFetchSdf] = 0u;
-    w.counts[kWaveFetchSdfShadow] = 0u;
+    ctl_word(w.counts, kWaveExt + (cur ^ 1u)) = 0u;
+    ctl_word(w.counts, kWaveShadow + cur) = 0u;
+    ctl_word(w.counts, kWaveFetchSdf) = 0u;
+    ctl_word(w.counts, kWaveFetchSdfShadow) = 0u;
   }
   const WaveTraceSource<kTrans> src{geo_of(s), q, w.ray_o, w.ray_d, w.hit, w.sh_o, w.sh_d, w.sh_c, w.sh_path, w.rad,
                                     n_ext, s.shade, s.materials, s.material_count};
   TraceStats st, st_sh;
   uint32_t lerr = 0u;
   persistent_traverse<WaveTraceSource<kTrans>, kQueryMixed, kStats, kWt>(
-      src, n_ext + n_sh, &w.counts[kWaveFetch + ((parts & 1u) ? 0 : 1)], launch_stack(smem_stack, scap, spill, total),
+      src, n_ext + n_sh, &ctl_word(w.counts, kWaveFetch + ((parts & 1u) ? 0 : 1)), launch_stack(smem_stack, scap, spill, total),
       steps, st, st_sh, lerr);
   if (kStats) {
     warp_count(&ctr->nodes, st.nodes);
@@ -348,18 +348,18 @@ __device__ __forceinline__ void flush_sdf(DevCounters* ctr, const SdfCount& c) {
 
 __global__ void __launch_bounds__(256) k_sdf(DevScene s, WaveState w, const uint32_t* q, uint32_t depth,
                                              DevCounters* ctr) {
-  const uint32_t n = w.counts[kWaveExt + (depth & 1u)];
+  const uint32_t n = ctl_word(w.counts, kWaveExt + (depth & 1u));
   SdfCount c;
   const WaveSdfExtSource src{s.sdf, s.sdf_count, q, w.ray_o, w.ray_d, w.hit};
-  sdf_persistent<WaveSdfExtSource, false>(src, n, &w.counts[kWaveFetchSdf], kSdfSteps, c);
+  sdf_persistent<WaveSdfExtSource, false>(src, n, &ctl_word(w.counts, kWaveFetchSdf), kSdfSteps, c);
   flush_sdf(ctr, c);
 }
 
 __global__ void __launch_bounds__(256) k_sdf_shadow(DevScene s, WaveState w, uint32_t depth, DevCounters* ctr) {
-  const uint32_t n = w.counts[kWaveShadow + (depth & 1u)];
+  const uint32_t n = ctl_word(w.counts, kWaveShadow + (depth & 1u));
   SdfCount c;
   const WaveSdfShadowSource src{s.sdf, s.sdf_count, w.sh_o, w.sh_d, w.sh_path};
-  sdf_persistent<WaveSdfShadowSource, true>(src, n, &w.counts[kWaveFetchSdfShadow], kSdfSteps, c);
+  sdf_persistent<WaveSdfShadowSource, true>(src, n, &ctl_word(w.counts, kWaveFetchSdfShadow), kSdfSteps, c);
   flush_sdf(ctr, c);
 }
 
@@ -374,10 +374,10 @@ template <bool kParity, bool kEffects, bool kSdf, bool kExotic>
 __global__ void __launch_bounds__(256, 4) k_shade(DevScene s, DevSettings st, WaveState w, const uint32_t* q,
                                                   uint32_t* qn, uint32_t depth, DevCounters* ctr) {
   const uint32_t cur = depth & 1u;
-  const uint32_t n = w.counts[kWaveExt + cur];
+  const uint32_t n = ctl_word(w.counts, kWaveExt + cur);
   if (blockIdx.x == 0 && threadIdx.x == 0) {   // the next trace stage claims from 0
-    w.counts[kWaveFetch] = 0u;
-    w.counts[kWaveFetch + 1] = 0u;
+    ctl_word(w.counts, kWaveFetch) = 0u;
+    ctl_word(w.counts, kWaveFetch + 1) = 0u;
   }
   uint32_t shadow_tests = 0u;
   for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
@@ -407,9 +407,9 @@ __global__ void __launch_bounds__(256, 4) k_shade(DevScene s, DevSettings st, Wa
       shadow_tests += R.shadow_tests;
     }
     // Warp-aggregated appends (the whole warp reaches these together).
-    const uint32_t slot_n = warp_append(&w.counts[kWaveExt + (cur ^ 1u)], R.next);
+    const uint32_t slot_n = warp_append(&ctl_word(w.counts, kWaveExt + (cur ^ 1u)), R.next);
     if (R.next) qn[slot_n] = p;
-    const uint32_t slot_s = warp_append(&w.counts[kWaveShadow + cur], R.shadow);
+    const uint32_t slot_s = warp_append(&ctl_word(w.counts, kWaveShadow + cur), R.shadow);
     if (R.shadow) {
       w.sh_path[slot_s] = p;
       w.sh_o[slot_s] = make_float4(R.sh_o.x, R.sh_o.y, R.sh_o.z, R.sh_t);
@@ -428,7 +428,7 @@ __global__ void __launch_bounds__(256) k_shadow_transmissive(DevScene s, WaveSta
                                                              DevCounters* ctr, uint32_t* err) {
   extern __shared__ int2 smem_stack[];
   const TwoLevelStack stk = smem_stack_of(smem_stack + threadIdx.x, static_cast<int>(blockDim.x), cap);
-  const uint32_t n = w.counts[kWaveShadow + (depth & 1u)];
+  const uint32_t n = ctl_word(w.counts, kWaveShadow + (depth & 1u));
   uint32_t local_err = 0u;
   for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
     const uint32_t j = base + threadIdx.x;
@@ -490,9 +490,9 @@ __global__ void __launch_bounds__(256) k_shadow_transmissive(DevScene s, WaveSta
 __global__ void __launch_bounds__(256) k_accumulate(DevSettings st, WaveState w, WaveTile tile, Film film,
                                                     DevCounters* ctr) {
   const uint32_t tile_px = tile.w * tile.h;
+  uint32_t samples = 0u, segs = 0u, dropped = 0u;
   for (uint32_t base = blockIdx.x * blockDim.x; base < tile_px; base += gridDim.x * blockDim.x) {
     const uint32_t k = base + threadIdx.x;
-    uint32_t samples = 0u, segs = 0u, dropped = 0u;
     if (k < tile_px) {
       const uint32_t pl = tile_order_pixel(k, tile.w, tile.h);
       const uint32_t x = tile.x + pl % tile.w, y = tile.y + pl / tile.w;
@@ -521,10 +521,8 @@ __global__ void __launch_bounds__(256) k_accumulate(DevSettings st, WaveState w,
       film.sum[px] = acc;
       film.count[px] = cnt;
     }
-    warp_count(&ctr->samples, samples);
-    warp_count(&ctr->rays, segs);
-    warp_count(&ctr->dropped, dropped);
   }
+  block_count3(&ctr->samples, samples, &ctr->rays, segs, &ctr->dropped, dropped);
 }
 
 namespace {

@@ -24,7 +24,7 @@ struct WaveState {
   float4* sh_d;       // direction xyz
   float4* sh_c;       // contribution to add when visible
   // queues: q[0], q[1] ping-pong extension queues; counts: their sizes, the
-  // shadow queue's and the stages' fetch counters (8 words, kernels.cu)
+  // shadow queue's and the stages' fetch counters (ctl_word, kernels.cu)
   uint32_t* q[2];
   uint32_t* counts;
   uint32_t capacity;
