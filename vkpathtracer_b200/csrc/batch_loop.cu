@@ -245,14 +245,14 @@ __global__ void __launch_bounds__(256) k_lp_regen(const DevJob* __restrict__ job
       V3 o, d;
       uint64_t rng;
       camera_path<kParity>(J.scene, J.settings, px % W, px / W, J.first_sample + sl, o, d, rng);
-      A.job[q] = jb;
-      A.local[q] = local;
-      A.depth[q] = 0u;
-      A.rng[q] = rng;
-      A.o[q] = make_float4(o.x, o.y, o.z, 0.0f);
-      A.d[q] = make_float4(d.x, d.y, d.z, 0.0f);
-      A.thr[q] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
-      A.rad[q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      __stcs(A.job + q, jb);
+      __stcs(A.local + q, local);
+      __stcs(A.depth + q, 0u);
+      __stcs(reinterpret_cast<unsigned long long*>(A.rng + q), static_cast<unsigned long long>(rng));
+      __stcs(A.o + q, make_float4(o.x, o.y, o.z, 0.0f));
+      __stcs(A.d + q, make_float4(d.x, d.y, d.z, 0.0f));
+      __stcs(A.thr + q, make_float4(1.0f, 1.0f, 1.0f, 0.0f));
+      __stcs(A.rad + q, make_float4(0.0f, 0.0f, 0.0f, 0.0f));
     }
   }
 }
@@ -298,6 +298,9 @@ __global__ void __launch_bounds__(256) k_lp_sdf_shadow(const DevJob* __restrict_
 // kExotic: some job has a transmissive, clear-coat, sheen or toon material or
 // an environment map; without, those branches are compiled out.
 // 80 registers: the 64-job step takes 522 ms, 526 at 64 registers, 538 at 48.
+// Path state is read once and written once per iteration and far larger than
+// L2: streaming loads and stores leave the caches to the scenes (the step 509.2
+// -> 506.6 ms, eight small jobs 11.29 -> 11.25).
 template <bool kParity, bool kEffects, bool kSdf, bool kExotic>
 __global__ void __launch_bounds__(256, 3) k_lp_shade(const DevJob* __restrict__ jobs, LoopPool P,
                                                      DevCounters* ctr) {
@@ -313,18 +316,18 @@ __global__ void __launch_bounds__(256, 3) k_lp_shade(const DevJob* __restrict__ 
     PathRegs pr;
     ShadeOut R;
     if (j < n) {
-      jb = A.job[j];
-      local = A.local[j];
-      depth = A.depth[j];
+      jb = __ldcs(A.job + j);
+      local = __ldcs(A.local + j);
+      depth = __ldcs(A.depth + j);
       const DevJob& J = jobs[jb];
-      const float4 o4 = A.o[j], d4 = A.d[j], t4 = A.thr[j], r4 = A.rad[j];
-      const float2 h2 = P.hit[j];
+      const float4 o4 = __ldcs(A.o + j), d4 = __ldcs(A.d + j), t4 = __ldcs(A.thr + j), r4 = __ldcs(A.rad + j);
+      const float2 h2 = __ldcs(P.hit + j);
       pr.o = mk(o4.x, o4.y, o4.z);
       pr.d = mk(d4.x, d4.y, d4.z);
       pr.thr = mk(t4.x, t4.y, t4.z);
       pr.rad = mk(r4.x, r4.y, r4.z);
       pr.segs = r4.w;
-      pr.rng = A.rng[j];
+      pr.rng = __ldcs(reinterpret_cast<const unsigned long long*>(A.rng + j));
       R = shade_bounce<kParity, kEffects, kSdf, kExotic, true>(J.scene, J.settings, J.scene.lights, depth, pr, h2.x,
                                                                __float_as_uint(h2.y));
       next = R.next;
@@ -334,27 +337,27 @@ __global__ void __launch_bounds__(256, 3) k_lp_shade(const DevJob* __restrict__ 
     }
     const uint32_t qn = warp_append(&ctl_word(P.ctl, kLCount0 + (cur ^ 1u)), next);
     if (next) {
-      B.job[qn] = jb;
-      B.local[qn] = local;
-      B.depth[qn] = depth + 1u;
-      B.rng[qn] = pr.rng;
-      B.o[qn] = make_float4(pr.o.x, pr.o.y, pr.o.z, 0.0f);
-      B.d[qn] = make_float4(pr.d.x, pr.d.y, pr.d.z, 0.0f);
-      B.thr[qn] = make_float4(pr.thr.x, pr.thr.y, pr.thr.z, 0.0f);
-      B.rad[qn] = make_float4(pr.rad.x, pr.rad.y, pr.rad.z, pr.segs);
+      __stcs(B.job + qn, jb);
+      __stcs(B.local + qn, local);
+      __stcs(B.depth + qn, depth + 1u);
+      __stcs(reinterpret_cast<unsigned long long*>(B.rng + qn), static_cast<unsigned long long>(pr.rng));
+      __stcs(B.o + qn, make_float4(pr.o.x, pr.o.y, pr.o.z, 0.0f));
+      __stcs(B.d + qn, make_float4(pr.d.x, pr.d.y, pr.d.z, 0.0f));
+      __stcs(B.thr + qn, make_float4(pr.thr.x, pr.thr.y, pr.thr.z, 0.0f));
+      __stcs(B.rad + qn, make_float4(pr.rad.x, pr.rad.y, pr.rad.z, pr.segs));
     }
     const uint32_t qf = warp_append(&ctl_word(P.ctl, kLFin0 + cur), fin);
     if (fin) {
-      P.fin_rad[qf] = make_float4(pr.rad.x, pr.rad.y, pr.rad.z, pr.segs);
-      P.fin_job[qf] = jb;
-      P.fin_local[qf] = local;
+      __stcs(P.fin_rad + qf, make_float4(pr.rad.x, pr.rad.y, pr.rad.z, pr.segs));
+      __stcs(P.fin_job + qf, jb);
+      __stcs(P.fin_local + qf, local);
     }
     const uint32_t qs = warp_append(&ctl_word(P.ctl, kLShadow), shadow);
     if (shadow) {
-      P.sh_o[qs] = make_float4(R.sh_o.x, R.sh_o.y, R.sh_o.z, R.sh_t);
-      P.sh_d[qs] = make_float4(R.sh_d.x, R.sh_d.y, R.sh_d.z, __uint_as_float(jb));
-      P.sh_c[qs] = make_float4(R.sh_c.x, R.sh_c.y, R.sh_c.z, 0.0f);
-      P.sh_dst[qs] = next ? qn : (qf | kLoopFinBit);
+      __stcs(P.sh_o + qs, make_float4(R.sh_o.x, R.sh_o.y, R.sh_o.z, R.sh_t));
+      __stcs(P.sh_d + qs, make_float4(R.sh_d.x, R.sh_d.y, R.sh_d.z, __uint_as_float(jb)));
+      __stcs(P.sh_c + qs, make_float4(R.sh_c.x, R.sh_c.y, R.sh_c.z, 0.0f));
+      __stcs(P.sh_dst + qs, next ? qn : (qf | kLoopFinBit));
     }
   }
   warp_count(&ctr->shadow_tests, shadow_tests);
