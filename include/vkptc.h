@@ -345,7 +345,7 @@ int32_t vkptc_update_scene_delta(vkptc_ctx* ctx, const vkptc_scene_delta* delta)
 /* Extension (no reference counterpart): copies one device array of the built
  * accelerator to host memory, for inspection and for checking the device
  * build against the host build.  what: VKPTC_ACCEL_WIDE_NODES (128 B each: the children's
- * boxes as centre and half extent, then their refs),
+ * boxes, lo and hi of the four per axis, then their refs),
  * VKPTC_ACCEL_TRIANGLES (48 B each, leaf order), VKPTC_ACCEL_TIE_NODES (32 B
  * each, the reference binary tree), VKPTC_ACCEL_SHADING (16 B per primitive).
  * *bytes receives the array's size; out may be NULL to query it. */
@@ -510,8 +510,8 @@ typedef struct vkptc_batch_tuning {
   uint32_t occupancy;        /* traversal kernels' register variant: 0..3 = at least 1..4 resident
                                 256-thread blocks per SM (fewer registers, more warps; the loop
                                 driver's kernels run four for each of them); 4 (loop
-                                driver; the persistent driver takes it as 3) = at least 7 resident
-                                128-thread blocks per SM (72 registers), and the launch's block
+                                driver; the persistent driver takes it as 3) = at least 8 resident
+                                128-thread blocks per SM (64 registers), and the launch's block
                                 size becomes 128 */
   uint32_t barrier_spins;    /* persistent mode: bound of a grid-barrier wait in sleeps of ~128 ns
                                 (0 = 2^26, about 8.6 s); a block that waits longer aborts the run,

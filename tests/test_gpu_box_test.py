@@ -1,0 +1,96 @@
+"""The node test places a slab where fma(lo, 1/d, -o/d) does: the wide nodes
+hold the binary nodes' bounds as they are, an origin on a face of a box is
+inside where the ray runs along that face, and rays aimed at vertices from far
+away differ from the oracle's hits no more often than corner bounds' rounding
+makes them.
+"""
+import numpy as np
+import pytest
+
+import oracle
+from tests.test_gpu_traversal import tracer
+from vkpathtracer_b200 import native, scenes
+
+pytestmark = pytest.mark.gpu
+
+
+def wide_boxes(t):
+    """(box (N,6), ref (N,)) of the used slots."""
+    w = t.read_accel(native.ACCEL_WIDE_NODES).reshape(-1, 32)
+    b = w[:, :24].view(np.float32).reshape(-1, 3, 2, 4)           # axis, lo / hi, slot
+    boxes = b.transpose(0, 3, 2, 1).reshape(-1, 6)                # node and slot, lo xyz, hi xyz
+    refs = w[:, 24:28].view(np.int32).reshape(-1)
+    used = refs != np.iinfo(np.int32).min
+    return boxes[used], refs[used]
+
+
+def cubes(n, origin, seed):
+    """n axis-aligned cubes with integer corners around an integer origin."""
+    r = np.random.RandomState(seed)
+    corner = np.array([[x, y, z] for x in (0, 1) for y in (0, 1) for z in (0, 1)], np.float64)
+    faces = np.array([[0, 1, 3], [0, 3, 2], [4, 6, 7], [4, 7, 5], [0, 4, 5], [0, 5, 1],
+                      [2, 3, 7], [2, 7, 6], [0, 2, 6], [0, 6, 4], [1, 5, 7], [1, 7, 3]])
+    at, size = r.randint(-20, 20, (n, 1, 3)), r.randint(1, 4, (n, 1, 3))
+    sc = scenes.cornell_box(seed=4)
+    sc.vertices = np.ascontiguousarray((corner * size + at + origin).reshape(-1, 3), np.float32)
+    sc.indices = np.ascontiguousarray((faces[None] + 8 * np.arange(n)[:, None, None]).reshape(-1, 3), np.uint32)
+    sc.instances = np.array([[0, sc.indices.shape[0], 0]], np.uint32)
+    return sc
+
+
+def test_wide_boxes_are_the_binary_nodes():
+    sc = scenes.displaced_sphere(24, scale=16.0, seed=5)
+    with tracer(sc, bvh="reference") as t:
+        boxes, _ = wide_boxes(t)
+        tie = t.read_accel(native.ACCEL_TIE_NODES).reshape(-1, 8).view(np.float32)
+    binary = {row.tobytes() for row in np.ascontiguousarray(tie[:, (0, 1, 2, 4, 5, 6)])}
+    assert all(row.tobytes() in binary for row in np.ascontiguousarray(boxes))
+
+
+@pytest.mark.parametrize("bvh", ["reference", "sah"])
+@pytest.mark.parametrize("origin", [0, 1024, 4096, -4096, 70000])
+def test_rays_along_faces(origin, bvh):
+    """From 1024 on the boxes' padding of 1e-4 is an ulp or nothing, so the faces
+    of the boxes are the surfaces that rays between integer points run along."""
+    sc = cubes(40, origin, 3)
+    r = np.random.RandomState(7)
+    n = 20000
+    rays = np.zeros((n, 6), np.float32)
+    rays[:, :3] = r.randint(-26, 27, (n, 3)) + origin
+    rays[np.arange(n), 3 + r.randint(0, 3, n)] = r.choice([-1.0, 1.0], n)
+    rays[::5, 3:] *= np.float32(0.37)
+    if bvh == "reference":   # the nodes apply the inside rule up to 1e-4, too
+        k = np.arange(1, n, 3)
+        rows, axis = np.nonzero(rays[k, 3:] == 0.0)
+        rays[k[rows], 3 + axis] = r.choice([0.0, -0.0, 1e-30, -1e-10, 9e-5], rows.size)
+    rp, rt, _, _ = oracle.load("port").intersect(sc, rays, threads=8)
+    with tracer(sc, bvh=bvh) as t:
+        p, tt = t.trace_rays(rays)
+        u, _ = t.trace_rays(rays, mode=native.QUERY_ANY)
+    assert np.mean(np.isfinite(rt)) > 0.05
+    assert np.array_equal(tt.view(np.uint32), rt.view(np.uint32)) and np.array_equal(p, rp)
+    assert np.array_equal(u.astype(bool), np.isfinite(rt))
+
+
+@pytest.mark.parametrize("bvh,corner_bounds", [("reference", 285), ("sah", 724)])
+def test_vertex_rays_from_far(bvh, corner_bounds):
+    """60,000 rays aimed at the vertices of a sphere from 20 radii away: there
+    triangles that graze report distances some ulps outside their boxes, and
+    rounding decides which of them is visited.  Corner bounds tested in the
+    reference's order of children differed from the oracle in 285 and 724 hits;
+    another order of the same test moves that by its own scatter, taken as 30 %
+    (boxes as centre and half extent: 477 and 996)."""
+    sc = scenes.displaced_sphere(60, seed=5)
+    sc.vertices = np.ascontiguousarray(sc.vertices * np.float32(16.0))
+    r = np.random.RandomState(3)
+    v = np.asarray(sc.vertices, np.float64)
+    mid, half = 0.5 * (v.min(0) + v.max(0)), 0.5 * (v.max(0) - v.min(0)).max()
+    unit = lambda a: a / np.linalg.norm(a, axis=1, keepdims=True)
+    o = mid + unit(r.normal(size=(60000, 3))) * half * 20.0
+    rays = np.ascontiguousarray(np.concatenate([o, unit(v[r.randint(0, len(v), 60000)] - o)], 1), np.float32)
+    rp, rt, _, _ = oracle.load("port").intersect(sc, rays, threads=8)
+    with tracer(sc, bvh=bvh) as t:
+        p, tt = t.trace_rays(rays)
+    differ = p != rp
+    print(f"{bvh}: {differ.sum()} of {p.size} hits differ")
+    assert differ.sum() <= 1.3 * corner_bounds

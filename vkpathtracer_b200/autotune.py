@@ -24,8 +24,8 @@ DEFAULT_BLOCKS = (128, 256)
 DEFAULT_STACKS = (8, 16)
 DEFAULT_STEPS = (8, 16)
 DEFAULT_OCCUPANCY = (1, 2, 3)
-# Register variants only the loop driver has; they run its stages in 128-thread
-# blocks (variant 4: traversal stages at 72 registers, 28 warps per SM).
+# Variants only the loop driver has; they run its stages in 128-thread blocks
+# (variant 4: eight of them per SM, traversal stages at 64 registers).
 DEFAULT_LOOP_VARIANTS = (4,)
 LOOP_VARIANT_BLOCK = 128
 

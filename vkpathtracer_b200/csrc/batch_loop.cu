@@ -3,7 +3,7 @@
 // The persistent driver (batch.cu) runs the five stages of an iteration in
 // one cooperative kernel with grid barriers between them.  This driver runs
 // each stage as its own kernel, so a stage gets the register budget and
-// occupancy it needs (the traversal stages run at 64-72 registers, shading at
+// occupancy it needs (the traversal stages run at 64 registers, shading at
 // 80), and the iterations are driven by the device: the stages form the body
 // of a CUDA graph while-node whose condition the last stage sets.  One
 // graph launch renders every job; no kernel ever waits on another.
@@ -430,26 +430,24 @@ cudaError_t set_smem_attr(K kernel, int bytes) {
 }
 
 // Traversal stage variants: [triangle test][stats][register variant].
-// Variants 0..3: four resident 256-thread blocks per SM (64 registers).  The
-// 64-job workload at 256 threads takes 519 ms with it, 537 with three blocks
-// (80 registers) and 10 % more with the 86-90 registers the compiler takes
-// when fewer are asked for.  Variant 4: at least 7 resident 128-thread blocks
-// (72 registers, 28 warps; launched with at most 128 threads), 513 ms.  Stats
-// runs use the unconstrained variant at the launch's block size.
+// 64 registers in both: four resident 256-thread blocks per SM (variants 0..3) or
+// eight of 128 threads (variant 4; launched with at most 128 threads), which
+// take the 64-job workload in 510 ms; seven (72 registers) take 522, six 519.
+// Stats runs use the unconstrained variant at the launch's block size.
 using LoopTraceFn = void (*)(const DevJob*, LoopPool, int, int2*, int, int, DevCounters*, uint32_t*);
 LoopTraceFn extend_fn(bool stats, int occ, bool wt) {
   static const LoopTraceFn t[2][2][2] = {
-      {{k_lp_extend<false, 256, 4, false>, k_lp_extend<false, 128, 7, false>},
+      {{k_lp_extend<false, 256, 4, false>, k_lp_extend<false, 128, 8, false>},
        {k_lp_extend<true, 256, 1, false>, k_lp_extend<true, 128, 1, false>}},
-      {{k_lp_extend<false, 256, 4, true>, k_lp_extend<false, 128, 7, true>},
+      {{k_lp_extend<false, 256, 4, true>, k_lp_extend<false, 128, 8, true>},
        {k_lp_extend<true, 256, 1, true>, k_lp_extend<true, 128, 1, true>}}};
   return t[wt ? 1 : 0][stats ? 1 : 0][occ >= 4 ? 1 : 0];
 }
 LoopTraceFn shadow_fn(bool stats, int occ, bool wt) {
   static const LoopTraceFn t[2][2][2] = {
-      {{k_lp_shadow<false, 256, 4, false>, k_lp_shadow<false, 128, 7, false>},
+      {{k_lp_shadow<false, 256, 4, false>, k_lp_shadow<false, 128, 8, false>},
        {k_lp_shadow<true, 256, 1, false>, k_lp_shadow<true, 128, 1, false>}},
-      {{k_lp_shadow<false, 256, 4, true>, k_lp_shadow<false, 128, 7, true>},
+      {{k_lp_shadow<false, 256, 4, true>, k_lp_shadow<false, 128, 8, true>},
        {k_lp_shadow<true, 256, 1, true>, k_lp_shadow<true, 128, 1, true>}}};
   return t[wt ? 1 : 0][stats ? 1 : 0][occ >= 4 ? 1 : 0];
 }

@@ -22,14 +22,13 @@ struct BinNode {
   int32_t left, right, first, count;
 };
 
-// Wide node: the children's boxes as centre and half extent -- (x, y) pairs of
-// the four centres, of the four half extents, then the four centres' z and half
-// extents' z (the operands of the node test's packed arithmetic) --, then int4
-// child refs, then int4 meta (x = valid child count).  Child ref >= 0: wide node index; < 0: leaf,
+// Wide node: six float4 of child bounds (lo.x[4], hi.x[4], lo.y[4], hi.y[4],
+// lo.z[4], hi.z[4]: the node test takes its near and far planes by the ray's
+// signs), then int4 child refs, then int4 meta (x = valid child count).  Child ref >= 0: wide node index; < 0: leaf,
 // ~ref = (first_triangle << 3) | (count - 1); kEmptyChild: an unused slot
 // (so the traversal needs no child count).  128 bytes, one cache line.
 struct alignas(16) WideNode {
-  float cxy[8], hxy[8], cz[4], hz[4];
+  float lox[4], hix[4], loy[4], hiy[4], loz[4], hiz[4];
   int32_t child[4];
   int32_t meta[4];
 };
@@ -41,28 +40,21 @@ static_assert(sizeof(WideNode) == 128, "wide node must be one 128-byte line");
 #define VKPTC_HD
 #endif
 
-// Child k's box, enclosing [lo, hi] and larger than it by no more than the
-// rounding of centre and half extent: the reference culls with [lo, hi], and a
-// triangle whose distance is badly conditioned (|det| near 1e-4) can report one
-// outside its box, so a box visited beyond the reference's can change the hit.
-// A bound that is not finite makes its axis NaN, which the node test passes.
-// Plain multiplications and additions, so the host and the device builds store
-// the same words.
+// Child k's box: the binary node's bounds.  From 1024 on, where the padding of
+// 1e-4 is an ulp or nothing, the upper ones are an ulp or two higher: a ray with
+// a component of 0 along an upper face (the surface itself there) would get the
+// far distance 0 from the node test, and the reference counts it as inside.
+VKPTC_HD inline float UpperFace(float hi) {
+  const float a = hi < 0.0f ? -hi : hi;
+  return a >= 1024.0f ? hi + a * 1.1920928955078125e-7f : hi;   // 2^-23
+}
 VKPTC_HD inline void SetWideSlot(WideNode& n, int k, const float* lo, const float* hi) {
-  float c[3], h[3];
-  for (int a = 0; a < 3; ++a) {
-    c[a] = 0.5f * lo[a] + 0.5f * hi[a];
-    const float u = hi[a] - c[a], v = c[a] - lo[a];
-    const float m = u > v ? u : v;
-    h[a] = m + m * 1.1920928955078125e-7f;   // 2^-23: above the rounding of u, v and this sum
-    if (!(h[a] - h[a] == 0.0f)) c[a] = h[a] = c[a] - c[a] + (h[a] - h[a]);
-  }
-  n.cxy[2 * k] = c[0];
-  n.cxy[2 * k + 1] = c[1];
-  n.cz[k] = c[2];
-  n.hxy[2 * k] = h[0];
-  n.hxy[2 * k + 1] = h[1];
-  n.hz[k] = h[2];
+  n.lox[k] = lo[0];
+  n.loy[k] = lo[1];
+  n.loz[k] = lo[2];
+  n.hix[k] = UpperFace(hi[0]);
+  n.hiy[k] = UpperFace(hi[1]);
+  n.hiz[k] = UpperFace(hi[2]);
 }
 // The wide collapse.  A wide node takes up to four subtrees of the binary tree
 // as its slots, chosen bottom-up for the least expected cost (area times work):
@@ -122,8 +114,8 @@ VKPTC_HD inline uint32_t CollapseNode(const float* l, const float* r, float area
 
 // An unused slot: no box (its ref, kEmptyChild, is what the traversal tests).
 VKPTC_HD inline void ClearWideSlot(WideNode& n, int k) {
-  n.cxy[2 * k] = n.cxy[2 * k + 1] = n.cz[k] = 0.0f;
-  n.hxy[2 * k] = n.hxy[2 * k + 1] = n.hz[k] = -1.0f;
+  n.lox[k] = n.loy[k] = n.loz[k] = 1.0f;
+  n.hix[k] = n.hiy[k] = n.hiz[k] = -1.0f;
   n.child[k] = kEmptyChild;
 }
 

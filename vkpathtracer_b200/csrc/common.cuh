@@ -197,6 +197,7 @@ struct DevScene {
   float iris_sector, iris_cos_half, iris_rot, iris_round, iris_one_minus_round;
   float squeeze;
   uint32_t stack_required;
+  float box_eps;             // |d| up to which an axis of the node test uses the inside rule (traverse.cuh)
   uint32_t watertight;       // 1: triangle records hold vertices, tested watertight
   const float4* sdf;         // SDF primitive records (sdf.cuh), tested after the triangles
   uint32_t sdf_count;

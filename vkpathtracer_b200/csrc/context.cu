@@ -311,6 +311,8 @@ DevScene dev_scene(const vkptc_ctx* c) {
   s.squeeze = std::isfinite(c->cam.squeeze) ? std::max(0.01f, c->cam.squeeze) : 1.0f;
   s.stack_required = c->wide.stack_required;
   s.watertight = c->config.triangle_test == VKPTC_TRIANGLE_WATERTIGHT ? 1u : 0u;
+  // the watertight mode tests every box geometrically
+  s.box_eps = c->wide.reference_topology && !s.watertight ? 1e-4f : 1e-20f;
   s.sdf = c->sdf_count ? c->d_sdf.ptr : nullptr;
   s.sdf_count = c->sdf_count;
   return s;
@@ -997,7 +999,7 @@ int32_t build_on_device(vkptc_ctx* c, bool* done) {
     if (reinterpret_cast<uintptr_t>(out.nodes) % 32u == 0u) {
       c->d_nodes.adopt_pooled(out.nodes, 8ull * out.wide_nodes, c->stream);
     } else {
-      // the traversal reads node bounds with 32-byte loads: move the nodes to an aligned allocation
+      // a node's planes lie in whole 32-byte sectors: move the nodes to an aligned allocation
       VKPTC_CUDA(c, c->d_nodes.alloc(8ull * out.wide_nodes), "bvh alloc");
       VKPTC_CUDA(c, cudaMemcpyAsync(c->d_nodes.ptr, out.nodes, 128ull * out.wide_nodes, cudaMemcpyDeviceToDevice,
                                     c->stream), "bvh copy");
@@ -1974,8 +1976,7 @@ int32_t batch_run_pool(vkptc_batch* b, const vkptc_batch_tuning& t, uint32_t mod
   }
   // Register variant of the traversal kernels: 0..3 for both drivers; the loop
   // driver's variant 4 runs its stages in 128-thread blocks.  Variant 0 leaves
-  // the number of registers open: blocks that variant 4 can run take its 72
-  // (the 64-job workload 513 ms, 520 at 64 registers).
+  // the choice open: blocks that variant 4 can run take it.
   bl.occupancy = static_cast<int>(std::min(loop ? 4u : 3u, t.occupancy));
   if (loop && bl.occupancy == 4) bl.block = 128;
   if (loop && bl.occupancy == 0 && bl.block <= 128) bl.occupancy = 4;

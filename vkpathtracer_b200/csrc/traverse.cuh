@@ -7,14 +7,17 @@
 //    accepted when 1e-4 < t < best; evaluated in the reference's exact
 //    operation order without fused multiply-adds, so t is bit-identical.
 //  * Boxes only cull.  Every triangle box is padded by 1e-4 as in the reference.
-//    The node test below places a slab within about 2^-24 (|o| + 3 |c - o|) of
+//    The node test below places a slab within about 2^-24 (|o| + |lo - o|) of
 //    where it is, which the padding covers for coordinates of a few hundred, so
-//    every triangle the reference could hit is reached there.
+//    the box of a triangle that a ray meets is not missed there.  (A triangle
+//    whose distance is badly conditioned, |det| near 1e-4, can report one
+//    outside its box; whether it is visited then depends on rounding.)
 //  * The reference treats an axis with |d| <= 1e-4 as "parallel" and there only
 //    checks that the origin lies inside the slab, which decides which triangles
-//    it can test at all.  That rule is monotone under box inclusion, so the box
-//    of the triangle's leaf in the reference's tree decides it: leaf_rule_ok()
-//    applies it to a found hit, and the node test needs no such case.
+//    it can test at all.  In its own tree the node test does the same.  In another
+//    tree it does not, and leaf_rule_ok() applies the rule to a found hit: it is
+//    monotone under box inclusion, so the box of the triangle's leaf in the
+//    reference's tree decides it.
 //  * Exact distance ties: the reference keeps the first triangle it visits
 //    (strict t < best), i.e. the earlier lane of one leaf, or for two leaves
 //    the one under the nearer child of their lowest common binary ancestor
@@ -25,23 +28,28 @@
 // The traversal is bound by issued instructions under divergence (about ten of
 // a warp's lanes are active per instruction) with L1's load pipe next (66 % of
 // its wavefronts), not by memory bandwidth, so a step is kept short:
-//  * A wide node holds its children's boxes as centre and half extent, (x, y)
-//    pairs and z per child.  On an axis, with i = 1/d, the slab distances are
-//    c*i - o*i -+ h*|i|: three packed multiply-adds (f32x2, two floats an
-//    instruction) and no minimum/maximum per slab, 24 packed instructions for
-//    the four children against 24 scalar multiply-adds and 24 min/max (which
-//    run at half rate) with corner bounds.
-//  * |d| is clamped to [1e-20, 1e20] for the box test, so there is no special
-//    case for a zero component.
+//  * A wide node holds its children's boxes as lo[4], hi[4] per axis.  On an
+//    axis, with i = 1/d, the slab distances are lo*i - o*i and hi*i - o*i; the
+//    sign of d says which is the nearer one, so the node test loads the near
+//    and the far four from addresses that depend on it and needs no minimum or
+//    maximum per slab: twelve packed multiply-adds (f32x2, two children an
+//    instruction), where corner bounds in any order took 24 scalar multiply-adds
+//    and 24 min/max, which run at half rate.
 //  * The children are ordered by three compare-exchanges: the nearest is exact,
 //    the rest are pushed as they come.  A full sort (five) measured 1-3 % slower.
 //  * A leaf is its own cursor: the leaf reference of the triangles not yet
 //    tested, so no range is kept beside it.
 //  * The best hit is kept as its triangle record's index; primitive id, leaf
 //    and lane are read from the record when they are needed.
-// Against corner bounds with a full sort, on the 1,046,904-triangle sphere (SAH
-// tree, eight steps between refills): camera rays 3.26 -> 4.28 G/s, rays from
-// hit points in random directions 2.01 -> 2.52 G/s, random rays 3.58 -> 4.40 G/s.
+// Against boxes as centre and half extent (three 256-bit loads, 24 packed
+// instructions): closest hits of 8,388,608 rays on the 1,046,904-triangle sphere
+// 1,459 -> 1,434 us, the 64-job batch 513.6 -> 511.2 ms, a full-HD frame of the
+// 2,064,386-triangle grid 19.2 -> 19.8 ms, of the closed box 1.085 -> 1.107 (more
+// load instructions).  Those place a slab within 2^-24 (|o| + 3 |c - o|) only: of
+// rays aimed at a sphere's vertices from 20 radii away 477 and 996 hits of 60,000
+// (reference and SAH tree) differed from the reference's, 344 and 826 now, and
+// a ray along a box face beyond coordinates of 1024 could miss the surface in it.
+// Three 256-bit loads with the planes swapped by selects: 1,525 us, 527 ms, 19.7 ms.
 #pragma once
 
 #include "bvh_layout.h"
@@ -52,7 +60,7 @@ namespace vkptc {
 #define kInf __int_as_float(0x7f800000)
 
 // ------------------------------------------------------------ packed floats
-// Two floats in one register pair, and the f32x2 operations on them (each lane
+// Two floats in one register pair, and the f32x2 multiply-add on them (each lane
 // rounded to nearest as the scalar operation is).
 typedef unsigned long long F2;
 __device__ __forceinline__ F2 pack2(float a, float b) {
@@ -68,58 +76,42 @@ __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
   return r;
 }
-__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
-  F2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ F2 add2(F2 a, F2 b) {
-  F2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ F2 sub2(F2 a, F2 b) {
-  F2 r;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-// 256-bit read-only load of four pairs (sm_100); wide nodes are 128-byte
-// records of allocations whose base the host checks for 32-byte alignment.
-__device__ __forceinline__ void ldg256(const float4* p, F2& a, F2& b, F2& c, F2& d) {
-  asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(a), "=l"(b), "=l"(c), "=l"(d) : "l"(p));
+// 128-bit read-only load of two pairs.
+__device__ __forceinline__ void ldg_pairs(const char* p, F2& a, F2& b) {
+  asm("ld.global.nc.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p));
 }
 
 // ------------------------------------------------------------ the ray
-// Box-test constants: 1/d, -o/d and |1/d|, the x and y axes as a pair, z twice.
+// Box-test constants, each twice: 1/d and -o/d per axis.  An axis with
+// |d| <= box_eps asks whether the origin lies in the slab, by the reference's rule:
+// its 1/d is 2^66, a power of two, so that 2^66 (lo - o) and 2^66 (hi - o) have the
+// right signs (on an upper face the far distance is 0: SetWideSlot).  box_eps is
+// the reference's 1e-4 where the nodes are the reference's own, 1e-20 (components
+// of 0) in other trees, whose boxes can be smaller than the reference's leaves.
 struct BoxRay {
-  F2 ixy, nxy, axy, iz, nz, az;
+  F2 ix, iy, iz, nx, ny, nz;
+  uint32_t signs;   // byte k: 16 where axis k's d is negative (its near plane is hi)
 };
 struct RayPrep {
   float ox, oy, oz, dx, dy, dz;
   BoxRay b;
 };
 
-// 1/d for the box test: |d| clamped to [1e-20, 1e20] keeps it finite and
-// non-zero (a component of 0 tests as a very long slab, i.e. whether the origin
-// lies inside).  The approximate reciprocal was 0.5 % faster, and one grazing hit
-// in ten more differed from the reference's on rays aimed at vertices from 20
-// scene radii away.
-__device__ __forceinline__ float box_inverse(float d) {
-  return copysignf(__frcp_rn(fminf(fmaxf(fabsf(d), 1e-20f), 1e20f)), d);
+__device__ __forceinline__ void box_axis(float o, float d, float box_eps, uint32_t axis, F2& i2, F2& n2, uint32_t& signs) {
+  const float i = fabsf(d) > box_eps ? __frcp_rn(d) : 0x1p66f, n = -(o * i);
+  i2 = pack2(i, i);
+  n2 = pack2(n, n);
+  signs |= i < 0.0f ? 16u << (8u * axis) : 0u;
 }
 
-__device__ __forceinline__ RayPrep prep_ray(V3 o, V3 d) {
+__device__ __forceinline__ RayPrep prep_ray(V3 o, V3 d, float box_eps) {
   RayPrep r;
   r.ox = o.x; r.oy = o.y; r.oz = o.z;
   r.dx = d.x; r.dy = d.y; r.dz = d.z;
-  const float ix = box_inverse(d.x), iy = box_inverse(d.y), iz = box_inverse(d.z);
-  const float nz = -(o.z * iz), az = fabsf(iz);
-  r.b.ixy = pack2(ix, iy);
-  r.b.nxy = pack2(-(o.x * ix), -(o.y * iy));
-  r.b.axy = pack2(fabsf(ix), fabsf(iy));
-  r.b.iz = pack2(iz, iz);
-  r.b.nz = pack2(nz, nz);
-  r.b.az = pack2(az, az);
+  r.b.signs = 0u;
+  box_axis(o.x, d.x, box_eps, 0u, r.b.ix, r.b.nx, r.b.signs);
+  box_axis(o.y, d.y, box_eps, 1u, r.b.iy, r.b.ny, r.b.signs);
+  box_axis(o.z, d.z, box_eps, 2u, r.b.iz, r.b.nz, r.b.signs);
   return r;
 }
 
@@ -327,31 +319,36 @@ struct TraceStats {
 // Entry distances of a wide node's children (infinity: missed, or farther than
 // tmax) and their refs.  A NaN bound or ray component passes its axis.
 __device__ __forceinline__ void node_test(const float4* np, const BoxRay& b, float tmax, float (&t)[4], int32_t (&c)[4]) {
-  F2 cxy[4], hxy[4], cz[2], hz[2];
-  ldg256(np, cxy[0], cxy[1], cxy[2], cxy[3]);
-  ldg256(np + 2, hxy[0], hxy[1], hxy[2], hxy[3]);
-  ldg256(np + 4, cz[0], cz[1], hz[0], hz[1]);
+  const char* p = reinterpret_cast<const char*>(np);
+  const uint32_t sx = b.signs & 16u, sy = (b.signs >> 8) & 16u, sz = b.signs >> 16;
+  F2 nx[2], ny[2], nz[2], fx[2], fy[2], fz[2];
+  ldg_pairs(p + sx, nx[0], nx[1]);
+  ldg_pairs(p + (sx ^ 16u), fx[0], fx[1]);
+  ldg_pairs(p + 32 + sy, ny[0], ny[1]);
+  ldg_pairs(p + 32 + (sy ^ 16u), fy[0], fy[1]);
+  ldg_pairs(p + 64 + sz, nz[0], nz[1]);
+  ldg_pairs(p + 64 + (sz ^ 16u), fz[0], fz[1]);
   const int4 ch = __ldg(reinterpret_cast<const int4*>(np + 6));
   c[0] = ch.x;
   c[1] = ch.y;
   c[2] = ch.z;
   c[3] = ch.w;
-  float nz[4], fz[4];
 #pragma unroll
   for (int k = 0; k < 2; ++k) {
-    const F2 m = fma2(cz[k], b.iz, b.nz), e = mul2(hz[k], b.az);
-    unpack2(sub2(m, e), nz[2 * k], nz[2 * k + 1]);
-    unpack2(add2(m, e), fz[2 * k], fz[2 * k + 1]);
-  }
+    float ax[2], ay[2], az[2], bx[2], by[2], bz[2];
+    unpack2(fma2(nx[k], b.ix, b.nx), ax[0], ax[1]);
+    unpack2(fma2(ny[k], b.iy, b.ny), ay[0], ay[1]);
+    unpack2(fma2(nz[k], b.iz, b.nz), az[0], az[1]);
+    unpack2(fma2(fx[k], b.ix, b.nx), bx[0], bx[1]);
+    unpack2(fma2(fy[k], b.iy, b.ny), by[0], by[1]);
+    unpack2(fma2(fz[k], b.iz, b.nz), bz[0], bz[1]);
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const F2 m = fma2(cxy[k], b.ixy, b.nxy), e = mul2(hxy[k], b.axy);
-    float nx, ny, fx, fy;
-    unpack2(sub2(m, e), nx, ny);
-    unpack2(add2(m, e), fx, fy);
-    const float tn = fmaxf(fmaxf(fmaxf(nx, ny), nz[k]), kEps);
-    const float tf = fminf(fminf(fminf(fx, fy), fz[k]), tmax);
-    t[k] = tn <= tf && (k == 0 || c[k] != kEmptyChild) ? tn : kInf;   // slot 0 is never empty
+    for (int e = 0; e < 2; ++e) {
+      const int s = 2 * k + e;
+      const float tn = fmaxf(fmaxf(fmaxf(ax[e], ay[e]), az[e]), kEps);
+      const float tf = fminf(fminf(fminf(bx[e], by[e]), bz[e]), tmax);
+      t[s] = tn <= tf && (s == 0 || c[s] != kEmptyChild) ? tn : kInf;   // slot 0 is never empty
+    }
   }
 }
 
@@ -388,10 +385,11 @@ struct GeoView {
   const float4* tris;
   const float4* tie;
   uint32_t prim_count;
+  float box_eps;   // |d| up to which an axis of the node test uses the inside rule
 };
 
 __host__ __device__ __forceinline__ GeoView geo_of(const DevScene& s) {
-  return GeoView{s.nodes, s.tris, s.tie, s.prim_count};
+  return GeoView{s.nodes, s.tris, s.tie, s.prim_count, s.box_eps};
 }
 
 // What a kernel's queries ask for: the closest hit, any hit, or a mixture that
@@ -410,8 +408,8 @@ struct LaneState {
 
 // tmax: hits at or beyond it do not count (infinity: no bound).
 template <bool kWt>
-__device__ __forceinline__ void lane_begin(LaneState& L, V3 o, V3 d, float tmax) {
-  L.r = prep_ray(o, d);
+__device__ __forceinline__ void lane_begin(LaneState& L, V3 o, V3 d, float tmax, float box_eps) {
+  L.r = prep_ray(o, d, box_eps);
   if constexpr (kWt) L.w = prep_wt(L.r);
   L.t = tmax;
   L.best = -1;
@@ -535,7 +533,7 @@ __device__ __forceinline__ void trace_closest(const DevScene& s, V3 o, V3 d, con
   best_prim = kMiss;
   if (s.prim_count == 0u) return;
   LaneState L;
-  lane_begin<kWt>(L, o, d, kInf);
+  lane_begin<kWt>(L, o, d, kInf, s.box_eps);
   const auto tie = [&]() { return s.tie; };
   while (!lane_step<kQueryClosest, kStats, kWt>(L, s.nodes, s.tris, tie, stk, st, err)) {
   }
@@ -549,7 +547,7 @@ __device__ __forceinline__ bool trace_any(const DevScene& s, V3 o, V3 d, float t
                                           TraceStats& st, uint32_t& err) {
   if (s.prim_count == 0u || !(tmax > kEps)) return false;
   LaneState L;
-  lane_begin<kWt>(L, o, d, tmax);
+  lane_begin<kWt>(L, o, d, tmax, s.box_eps);
   const auto tie = [&]() { return s.tie; };
   while (!lane_step<kQueryAny, kStats, kWt>(L, s.nodes, s.tris, tie, stk, st, err)) {
   }
@@ -608,7 +606,7 @@ __device__ __forceinline__ void persistent_traverse(const Src& src, uint32_t n, 
       const V3 d = mk(l.r.dx, l.r.dy, l.r.dz);
       float tmax;
       if (src.finish(j, l.t, prim, o, d, tmax)) {
-        lane_begin<kWt>(l, o, d, tmax);
+        lane_begin<kWt>(l, o, d, tmax, src.geo_at(j).box_eps);
         return true;
       }
     } else {
@@ -649,7 +647,7 @@ __device__ __forceinline__ void persistent_traverse(const Src& src, uint32_t n, 
             tris = g.tris;
           }
           if constexpr (kMode == kQueryMixed) L.any = src.any(j);
-          lane_begin<kWt>(L, o, d, kMode == kQueryClosest ? kInf : tmax);
+          lane_begin<kWt>(L, o, d, kMode == kQueryClosest ? kInf : tmax, g.box_eps);
           if (g.prim_count == 0u || (kMode != kQueryClosest && !(tmax > kEps))) {
             finish(j, L);
           } else {
