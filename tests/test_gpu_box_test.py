@@ -24,6 +24,14 @@ def wide_boxes(t):
     return boxes[used], refs[used]
 
 
+def leaf_members(t):
+    """Per wide leaf: the reference leaves that its triangles are in."""
+    tri = t.read_accel(native.ACCEL_TRIANGLES).reshape(-1, 12)
+    _, refs = wide_boxes(t)
+    u = ~refs[refs < 0]
+    return [set(tri[f:f + n, 10]) for f, n in zip(u >> 3, (u & 7) + 1)]
+
+
 def cubes(n, origin, seed):
     """n axis-aligned cubes with integer corners around an integer origin."""
     r = np.random.RandomState(seed)
@@ -45,6 +53,16 @@ def test_wide_boxes_are_the_binary_nodes():
         tie = t.read_accel(native.ACCEL_TIE_NODES).reshape(-1, 8).view(np.float32)
     binary = {row.tobytes() for row in np.ascontiguousarray(tie[:, (0, 1, 2, 4, 5, 6)])}
     assert all(row.tobytes() in binary for row in np.ascontiguousarray(boxes))
+
+
+@pytest.mark.parametrize("build", ["device", "host"])
+def test_leaves_of_the_reference_tree_stay_whole(build):
+    """A triangle is tested in the reference's tree only where its leaf's own box is met."""
+    for sc in (scenes.cornell_box(seed=4), scenes.displaced_sphere(24, scale=16.0, seed=5)):
+        with tracer(sc, bvh="reference", build=build) as t:
+            members = leaf_members(t)
+        assert all(len(m) == 1 for m in members)
+        assert len(members) == len(set().union(*members))
 
 
 @pytest.mark.parametrize("bvh", ["reference", "sah"])

@@ -1176,7 +1176,7 @@ struct WideArrays {
 // leaf walks up, the second child to arrive does the parent.
 __global__ void k_collapse_cost(const BinNode* __restrict__ bin, uint32_t n, const int32_t* __restrict__ parent,
                                 uint32_t* __restrict__ visits, float4* __restrict__ cost, uint2* __restrict__ range,
-                                uint8_t* __restrict__ choice) {
+                                uint8_t* __restrict__ choice, bool merge) {
   uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= n || bin[x].count == 0) return;
   {
@@ -1195,7 +1195,7 @@ __global__ void k_collapse_cost(const BinNode* __restrict__ bin, uint32_t n, con
     const uint2 rl = __ldcg(range + b.left), rr = __ldcg(range + b.right);
     const float lc[4] = {l.x, l.y, l.z, l.w}, rc[4] = {r.x, r.y, r.z, r.w};
     float o[4];
-    choice[p] = static_cast<uint8_t>(CollapseNode(lc, rc, HalfArea(b.lo, b.hi), static_cast<int32_t>(rl.y + rr.y), o));
+    choice[p] = static_cast<uint8_t>(CollapseNode(lc, rc, HalfArea(b.lo, b.hi), static_cast<int32_t>(rl.y + rr.y), merge, o));
     cost[p] = make_float4(o[0], o[1], o[2], o[3]);
     range[p] = make_uint2(rl.x, rl.y + rr.y);
     x = static_cast<uint32_t>(p);
@@ -1515,7 +1515,7 @@ __global__ void k_parents(const BinNode* __restrict__ nodes, uint32_t n, int32_t
 uint32_t wide_capacity(uint32_t n_bin) { return n_bin / 2u + 1u; }
 
 cudaError_t collapse(const BinNode* bin, uint32_t n_bin, WideNode* out, uint32_t& n_wide, uint32_t& depth,
-                     uint32_t& stack_required, Scratch& sc, int32_t* slot_bin = nullptr) {
+                     uint32_t& stack_required, Scratch& sc, bool merge, int32_t* slot_bin = nullptr) {
   cudaStream_t s = sc.s;
   const uint32_t cap = wide_capacity(n_bin);
   int32_t* parent = sc.get<int32_t>(n_bin);
@@ -1530,7 +1530,7 @@ cudaError_t collapse(const BinNode* bin, uint32_t n_bin, WideNode* out, uint32_t
   if (sc.err != cudaSuccess) return sc.err;
   k_parents<<<grid_for(n_bin), kThreads, 0, s>>>(bin, n_bin, parent);
   BB_TRY(cudaMemsetAsync(visits, 0, n_bin * sizeof(uint32_t), s));
-  k_collapse_cost<<<grid_for(n_bin), kThreads, 0, s>>>(bin, n_bin, parent, visits, cost, range, choice);
+  k_collapse_cost<<<grid_for(n_bin), kThreads, 0, s>>>(bin, n_bin, parent, visits, cost, range, choice, merge);
   WTemp root{};
   root.slot[0] = 0;
   root.parent = -1;
@@ -1918,7 +1918,7 @@ cudaError_t BuildAccelOnDevice(const DeviceSceneArrays& sc_in, bool sah, cudaStr
   BB_TRY(dmalloc(wide, wide_capacity(n_trav), stream));
   out.nodes = reinterpret_cast<float4*>(wide);
   if (keep_refit) BB_TRY(dmalloc(out.refit->slot_bin, 4ull * n_trav, stream));
-  BB_TRY(collapse(trav, n_trav, wide, out.wide_nodes, out.depth, out.stack_required, sc,
+  BB_TRY(collapse(trav, n_trav, wide, out.wide_nodes, out.depth, out.stack_required, sc, sah,
                   keep_refit ? out.refit->slot_bin : nullptr));
   TriRecord* tris = nullptr;
   BB_TRY(dmalloc(tris, n, stream));

@@ -486,7 +486,8 @@ void CollapseToWide(const SceneGeometry& geo, const std::vector<BinNode>& bin,
       } else {
         const size_t l = static_cast<size_t>(nd.left), r = static_cast<size_t>(nd.right);
         count[id] = count[l] + count[r];
-        choice[id] = static_cast<uint8_t>(CollapseNode(cost[l].data(), cost[r].data(), area, count[id], cost[id].data()));
+        choice[id] = static_cast<uint8_t>(CollapseNode(cost[l].data(), cost[r].data(), area, count[id], !out.reference_topology,
+                                                        cost[id].data()));
       }
     }
   }

@@ -59,7 +59,9 @@ VKPTC_HD inline void SetWideSlot(WideNode& n, int k, const float* lo, const floa
 // The wide collapse.  A wide node takes up to four subtrees of the binary tree
 // as its slots, chosen bottom-up for the least expected cost (area times work):
 // cost(i) of a subtree is that of at most i roots for it, where one root is a
-// leaf of all its triangles (at most 8) or a wide node over its best four.
+// leaf of all its triangles (at most 8; see CollapseNode) or a wide node over its
+// best four (the dynamic programme of Ylitie, Karras and Laine, "Efficient
+// Incoherent Ray Traversal on GPUs Through Compressed Wide BVHs", HPG 2017, 3.1).
 // Opening the largest slot greedily, top-down, filled 3.05 of 4 slots on the
 // 1,046,904-triangle sphere and kept the binary tree's leaves.
 // Choosing it this way makes 31 % fewer wide nodes there; rays from hit points
@@ -82,8 +84,12 @@ VKPTC_HD inline float HalfArea(const float* lo, const float* hi) {
   return dx * dy + dy * dz + dz * dx;
 }
 // Costs and choices of an internal node from its children's; plain float
-// arithmetic, so the host and the device collapse choose the same.
-VKPTC_HD inline uint32_t CollapseNode(const float* l, const float* r, float area, int32_t count, float* out) {
+// arithmetic, so the host and the device collapse choose the same.  merge: the
+// subtree may become one leaf.  Not in the reference's own tree: a triangle whose
+// distance is badly conditioned can be hit outside its box, so one that the
+// reference's leaf box culls must not be tested under the box of several leaves.
+VKPTC_HD inline uint32_t CollapseNode(const float* l, const float* r, float area, int32_t count, bool merge,
+                                     float* out) {
   const float d2 = l[0] + r[0];
   const float a3 = l[0] + r[1], b3 = l[1] + r[0];
   const float d3 = b3 < a3 ? b3 : a3;
@@ -100,7 +106,7 @@ VKPTC_HD inline uint32_t CollapseNode(const float* l, const float* r, float area
   }
   uint32_t bits = ((b3 < a3 ? 2u : 1u) << 4) | (k4 << 6);
   const float node = area + d4, leaf = area * (kTriangleCost * static_cast<float>(count));
-  const bool is_leaf = count <= kWideLeafMax && !(node < leaf);
+  const bool is_leaf = merge && count <= kWideLeafMax && !(node < leaf);
   out[0] = is_leaf ? leaf : node;
   if (is_leaf) bits |= 1u;
   const float d[3] = {d2, d3, d4};
@@ -197,8 +203,9 @@ bool ValidateBinaryBvh(const std::vector<BinNode>& nodes, const std::vector<uint
                        size_t prim_count, std::string& error);
 
 // Collapses a binary traversal tree into the wide layout.  Each wide child
-// slot is a binary node with its exact float bounds; leaves stay whole binary
-// leaves.  Triangle records and tie nodes come from the REFERENCE tree
+// slot is a binary node with its bounds (SetWideSlot).  The leaves of the
+// reference's tree stay whole; in another tree subtrees of up to eight triangles
+// may become one leaf (CollapseNode).  Triangle records and tie nodes come from the REFERENCE tree
 // (ref_nodes / ref_prims): each triangle carries its reference leaf and lane,
 // so exact-distance ties and the parallel-axis rule follow the reference even
 // when the traversal tree is a different one.
