@@ -637,17 +637,16 @@ int AdjBlocksPerSm(AdjKernel k, int block, size_t smem, bool parity) {
   return n > 0 ? n : 1;
 }
 
-cudaError_t ConfigureAdjSmem(size_t bytes) {
-  const int b = static_cast<int>(bytes);
+cudaError_t ConfigureAdjSmem() {
   cudaError_t e;
-  if ((e = cudaFuncSetAttribute(k_adj_forward<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, b))) return e;
-  if ((e = cudaFuncSetAttribute(k_adj_forward<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, b))) return e;
-  if ((e = cudaFuncSetAttribute(k_adj_forward<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, b))) return e;
-  if ((e = cudaFuncSetAttribute(k_adj_forward<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, b))) return e;
-  if ((e = cudaFuncSetAttribute(k_adj_replay<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, b))) return e;
-  if ((e = cudaFuncSetAttribute(k_adj_replay<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, b))) return e;
-  if ((e = cudaFuncSetAttribute(k_adj_reverse<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, b))) return e;
-  return cudaFuncSetAttribute(k_adj_reverse<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+  if ((e = allow_full_smem(k_adj_forward<true, false>))) return e;
+  if ((e = allow_full_smem(k_adj_forward<false, false>))) return e;
+  if ((e = allow_full_smem(k_adj_forward<true, true>))) return e;
+  if ((e = allow_full_smem(k_adj_forward<false, true>))) return e;
+  if ((e = allow_full_smem(k_adj_replay<true>))) return e;
+  if ((e = allow_full_smem(k_adj_replay<false>))) return e;
+  if ((e = allow_full_smem(k_adj_reverse<true>))) return e;
+  return allow_full_smem(k_adj_reverse<false>);
 }
 
 cudaError_t LaunchAdjForward(const DevScene& s, const DevSettings& st, const float* mat0, const AdjLaunch& l,
@@ -665,9 +664,7 @@ cudaError_t LaunchAdjForward(const DevScene& s, const DevSettings& st, const flo
   return cudaGetLastError();
 }
 
-cudaError_t ConfigureAdjTraceSmem(size_t bytes) {
-  return cudaFuncSetAttribute(k_adj_trace, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
-}
+cudaError_t ConfigureAdjTraceSmem() { return allow_full_smem(k_adj_trace); }
 
 cudaError_t LaunchAdjRecord(const DevScene& s, const DevSettings& st, const float* mat0, const AdjWaveLaunch& l,
                             const AdjWave& w, float4* rad, float4* recs, uint32_t* nrec, uint32_t* err) {

@@ -49,7 +49,7 @@ struct AdjWaveLaunch {
 cudaError_t LaunchAdjRecord(const DevScene& s, const DevSettings& st, const float* mat0, const AdjWaveLaunch& l,
                             const AdjWave& w, float4* rad, float4* recs, uint32_t* nrec, uint32_t* err);
 // Raises its trace kernel's dynamic shared-memory limit (stacks above 48 KB per block).
-cudaError_t ConfigureAdjTraceSmem(size_t bytes);
+cudaError_t ConfigureAdjTraceSmem();
 
 // Image (sample-order accumulation exactly as the film does), loss partials
 // per block, and the per-pixel adjoint dL/d(sample radiance) (0 without a target).
@@ -81,6 +81,6 @@ size_t AdjBackwardSmem(int block, int stack_cap, uint32_t materials);
 size_t AdjReverseSmem(int block, uint32_t materials);
 size_t AdjForwardSmem(int block, int stack_cap);
 int AdjBlocksPerSm(AdjKernel k, int block, size_t smem, bool parity);
-cudaError_t ConfigureAdjSmem(size_t bytes);
+cudaError_t ConfigureAdjSmem();
 
 }  // namespace vkptc

@@ -375,13 +375,6 @@ cudaError_t LaunchBatchInit(const BatchPool& pool, cudaStream_t stream) {
   return cudaGetLastError();
 }
 
-namespace {
-template <typename K>
-cudaError_t set_smem_attr(K kernel, int bytes) {
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-}
-}  // namespace
-
 // Kernel variant table: [triangle test][parity][stats][occupancy variant].
 namespace {
 using BatchFn = void (*)(const DevJob*, uint32_t, unsigned long long, BatchPool, int, int2*, int, int, DevCounters*,
@@ -406,14 +399,13 @@ BatchFn batch_fn(bool parity, bool stats, int occ, bool wt) {
 }
 }  // namespace
 
-cudaError_t ConfigureBatchSmem(size_t bytes) {
-  const int b = static_cast<int>(bytes);
+cudaError_t ConfigureBatchSmem() {
   cudaError_t e = cudaSuccess;
   for (int wt = 0; wt < 2 && e == cudaSuccess; ++wt)
     for (int p = 0; p < 2 && e == cudaSuccess; ++p)
       for (int st = 0; st < 2 && e == cudaSuccess; ++st)
         for (int o = 0; o < kOccVariants && e == cudaSuccess; ++o)
-          e = set_smem_attr(batch_fn(p != 0, st != 0, o, wt != 0), b);
+          e = allow_full_smem(batch_fn(p != 0, st != 0, o, wt != 0));
   return e;
 }
 

@@ -96,7 +96,7 @@ cudaError_t LaunchBatchInit(const BatchPool& pool, cudaStream_t stream);
 
 // Resident blocks per SM of the persistent batch kernel.
 int BatchBlocksPerSm(int block, size_t smem, bool parity, bool stats, int occ, bool watertight = false);
-cudaError_t ConfigureBatchSmem(size_t bytes);
+cudaError_t ConfigureBatchSmem();
 
 // ------------------------------------------------------------ loop driver
 // The same five stages as separate kernels (each with its own register
@@ -143,7 +143,7 @@ struct LoopGrids {
 };
 LoopGrids BatchLoopGrids(int block, size_t smem, bool parity, bool stats, int occupancy, int sm_count,
                          bool watertight = false, bool effects = true, bool sdf = true, bool exotic = true);
-cudaError_t ConfigureBatchLoopSmem(size_t bytes);
+cudaError_t ConfigureBatchLoopSmem();
 cudaError_t LaunchBatchLoopInit(const LoopPool& pool, cudaStream_t stream);
 // A second stream and two events: the shadow stage of an iteration (the
 // previous shading stage's NEE queries) then runs beside REGEN and EXTEND.

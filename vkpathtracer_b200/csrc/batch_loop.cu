@@ -424,11 +424,6 @@ int blocks_per_sm(K kernel, int block, size_t smem) {
   return n;
 }
 
-template <typename K>
-cudaError_t set_smem_attr(K kernel, int bytes) {
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-}
-
 // Traversal stage variants: [triangle test][stats][register variant].
 // 64 registers in both: four resident 256-thread blocks per SM (variants 0..3) or
 // eight of 128 threads (variant 4; launched with at most 128 threads), which
@@ -479,14 +474,13 @@ LoopGrids BatchLoopGrids(int block, size_t smem, bool parity, bool stats, int oc
   return g;
 }
 
-cudaError_t ConfigureBatchLoopSmem(size_t bytes) {
-  const int b = static_cast<int>(bytes);
+cudaError_t ConfigureBatchLoopSmem() {
   cudaError_t e = cudaSuccess;
   for (int wt = 0; wt < 2 && e == cudaSuccess; ++wt)
     for (int st = 0; st < 2 && e == cudaSuccess; ++st)
       for (int o = 3; o < 5 && e == cudaSuccess; ++o) {
-        e = set_smem_attr(extend_fn(st != 0, o, wt != 0), b);
-        if (e == cudaSuccess) e = set_smem_attr(shadow_fn(st != 0, o, wt != 0), b);
+        e = allow_full_smem(extend_fn(st != 0, o, wt != 0));
+        if (e == cudaSuccess) e = allow_full_smem(shadow_fn(st != 0, o, wt != 0));
       }
   return e;
 }

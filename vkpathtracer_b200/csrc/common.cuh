@@ -214,6 +214,23 @@ struct DevSettings {
   uint32_t frame;
 };
 
+// Raises a kernel's dynamic shared-memory limit to all that a block can have.  The
+// limit belongs to the function, not to the context that asks, so it is never a
+// context's own need: one with a smaller need would lower it under another's
+// launches.
+template <typename K>
+cudaError_t allow_full_smem(K kernel) {
+  int device = 0, optin = 0;
+  cudaFuncAttributes a{};
+  cudaError_t e = cudaGetDevice(&device);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, kernel);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             optin - static_cast<int>(a.sharedSizeBytes));
+  return e;
+}
+
 // Camera paths are handed out in 8x4 pixel tiles, so a warp's rays cover a
 // compact block.  Each path still writes its own pixel, so films do not depend
 // on the order.

@@ -218,7 +218,7 @@ struct vkptc_ctx {
   // wave state
   DevBuf<uint8_t> w_arena;
   uint32_t wave_capacity = 0;
-  size_t smem_configured = 48 * 1024;
+  bool smem_raised = false;               // ConfigureStackSmem() has been called (launches above 48 KB need it)
   int max_smem_optin = 0;                 // the device's shared-memory limit per block
   int shape_block = 0, shape_per_sm = 0;  // resident blocks per SM of the last launch shape
   size_t shape_smem = 0;
@@ -344,6 +344,7 @@ int stack_cap(const vkptc_ctx* c) {
   return static_cast<int>(std::max<uint32_t>(1u, c->wide.stack_required));
 }
 
+constexpr size_t kDefaultSmemLimit = 48 * 1024;   // dynamic shared memory a kernel may have without asking
 constexpr int kDefaultSmemEntries = 12;
 constexpr int kDefaultSteps = 8;
 
@@ -393,9 +394,9 @@ int32_t ensure_stack_smem(vkptc_ctx* c, const LaunchShape& ls) {
   if (need > static_cast<size_t>(c->max_smem_optin)) {
     return fail(c, VKPTC_UNSUPPORTED, "traversal stack does not fit in shared memory (BVH too deep for this block size)");
   }
-  if (need > c->smem_configured) {
-    VKPTC_CUDA(c, ConfigureStackSmem(need), "shared memory limit");
-    c->smem_configured = need;
+  if (need > kDefaultSmemLimit && !c->smem_raised) {
+    VKPTC_CUDA(c, ConfigureStackSmem(), "shared memory limit");
+    c->smem_raised = true;
   }
   return VKPTC_OK;
 }
@@ -1815,14 +1816,13 @@ struct vkptc_batch {
   DevBuf<uint8_t> l_arena;
   DevBuf<DevCounters> d_ctr;
   DevBuf<uint32_t> d_err;
-  size_t smem_configured = 48 * 1024;
+  bool smem_raised = false, loop_smem_raised = false;   // as vkptc_ctx's, of the two drivers' kernels
   cudaGraphExec_t graph = nullptr;
   std::string graph_key;
   cudaStream_t body_stream = nullptr;   // captures the device-driven loop's body
   cudaStream_t side_stream = nullptr;   // the body's forked shadow branch
   cudaEvent_t fork_ev[2] = {nullptr, nullptr};
   cudaEvent_t marks[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};   // stage timing
-  size_t loop_smem_configured = 48 * 1024;
   vkptc_batch_stats stats{};
 };
 
@@ -1986,9 +1986,9 @@ int32_t batch_run_pool(vkptc_batch* b, const vkptc_batch_tuning& t, uint32_t mod
   if (smem > static_cast<size_t>(max_optin)) return bfail(b, VKPTC_UNSUPPORTED, "stack does not fit in shared memory");
   LoopGrids lg{};
   if (loop) {
-    if (smem > b->loop_smem_configured) {
-      VKPTC_BCUDA(b, ConfigureBatchLoopSmem(smem), "shared memory limit");
-      b->loop_smem_configured = smem;
+    if (smem > kDefaultSmemLimit && !b->loop_smem_raised) {
+      VKPTC_BCUDA(b, ConfigureBatchLoopSmem(), "shared memory limit");
+      b->loop_smem_raised = true;
     }
     lg = BatchLoopGrids(bl.block, smem, parity, bl.stats, bl.occupancy, b->sm_count, watertight, bl.effects, bl.sdf,
                         bl.exotic);
@@ -1997,9 +1997,9 @@ int32_t batch_run_pool(vkptc_batch* b, const vkptc_batch_tuning& t, uint32_t mod
     }
     bl.grid = std::max(lg.extend, lg.shadow);   // the traversal stages own the spill area
   } else {
-    if (smem > b->smem_configured) {
-      VKPTC_BCUDA(b, ConfigureBatchSmem(smem), "shared memory limit");
-      b->smem_configured = smem;
+    if (smem > kDefaultSmemLimit && !b->smem_raised) {
+      VKPTC_BCUDA(b, ConfigureBatchSmem(), "shared memory limit");
+      b->smem_raised = true;
     }
     const int per_sm = BatchBlocksPerSm(bl.block, smem, parity, bl.stats, bl.occupancy, watertight);
     if (per_sm <= 0) return bfail(b, VKPTC_UNSUPPORTED, "persistent batch kernel does not fit on an SM with this block size");
@@ -2529,8 +2529,8 @@ AdjLaunch adj_launch(vkptc_ctx* c, bool backward, int32_t& rc) {
     rc = fail(c, VKPTC_UNSUPPORTED, "adjoint: traversal stack and gradient slots do not fit in shared memory");
     return l;
   }
-  if (smem > 48 * 1024) {
-    const cudaError_t e = ConfigureAdjSmem(smem);
+  if (smem > kDefaultSmemLimit) {
+    const cudaError_t e = ConfigureAdjSmem();
     if (e != cudaSuccess) {
       rc = cuda_fail(c, e, "adjoint shared memory limit");
       return l;
@@ -2555,7 +2555,7 @@ int32_t adj_wave_launch(vkptc_ctx* c, AdjWaveLaunch& l) {
   const int32_t rc = launch_shape(c, c->stream, ls);
   if (rc != VKPTC_OK) return rc;
   const size_t smem = StackSmemBytes(ls.block, ls.smem_entries);
-  if (smem > 48 * 1024) VKPTC_CUDA(c, ConfigureAdjTraceSmem(smem), "adjoint shared memory limit");
+  if (smem > kDefaultSmemLimit) VKPTC_CUDA(c, ConfigureAdjTraceSmem(), "adjoint shared memory limit");
   l = AdjWaveLaunch{ls.grid, ls.block, ls.smem_entries, ls.stack_cap, ls.steps, ls.spill, c->adj.desc.spp,
                     c->adj.desc.first_sample, c->config.math_mode == 0u, c->stream};
   return VKPTC_OK;

@@ -739,26 +739,20 @@ cudaError_t LaunchResolveLdr(const Film& film, const LdrResolve& rs, bool parity
   return cudaGetLastError();
 }
 
-template <typename K>
-static cudaError_t set_smem(K kernel, int bytes) {
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-}
-
-cudaError_t ConfigureStackSmem(size_t bytes) {
-  const int b = static_cast<int>(bytes);
+cudaError_t ConfigureStackSmem() {
   cudaError_t e = cudaSuccess;
   const auto all = [&](auto wt) {
     constexpr bool W = decltype(wt)::value;
-    if (e == cudaSuccess) e = set_smem(k_trace_rays<true, true, W>, b);
-    if (e == cudaSuccess) e = set_smem(k_trace_rays<true, false, W>, b);
-    if (e == cudaSuccess) e = set_smem(k_trace_rays<false, true, W>, b);
-    if (e == cudaSuccess) e = set_smem(k_trace_rays<false, false, W>, b);
-    if (e == cudaSuccess) e = set_smem(k_trace<true, W, false>, b);
-    if (e == cudaSuccess) e = set_smem(k_trace<true, W, true>, b);
-    if (e == cudaSuccess) e = set_smem(k_trace<false, W, false>, b);
-    if (e == cudaSuccess) e = set_smem(k_trace<false, W, true>, b);
-    if (e == cudaSuccess) e = set_smem(k_shadow_transmissive<true, W>, b);
-    if (e == cudaSuccess) e = set_smem(k_shadow_transmissive<false, W>, b);
+    if (e == cudaSuccess) e = allow_full_smem(k_trace_rays<true, true, W>);
+    if (e == cudaSuccess) e = allow_full_smem(k_trace_rays<true, false, W>);
+    if (e == cudaSuccess) e = allow_full_smem(k_trace_rays<false, true, W>);
+    if (e == cudaSuccess) e = allow_full_smem(k_trace_rays<false, false, W>);
+    if (e == cudaSuccess) e = allow_full_smem(k_trace<true, W, false>);
+    if (e == cudaSuccess) e = allow_full_smem(k_trace<true, W, true>);
+    if (e == cudaSuccess) e = allow_full_smem(k_trace<false, W, false>);
+    if (e == cudaSuccess) e = allow_full_smem(k_trace<false, W, true>);
+    if (e == cudaSuccess) e = allow_full_smem(k_shadow_transmissive<true, W>);
+    if (e == cudaSuccess) e = allow_full_smem(k_shadow_transmissive<false, W>);
   };
   all(std::false_type{});
   all(std::true_type{});

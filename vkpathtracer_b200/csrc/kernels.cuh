@@ -66,7 +66,7 @@ size_t SpillEntries(const LaunchShape& ls);
 // Resident blocks per SM of the traversal stage for this block size and stack.
 int ExtendBlocksPerSm(int block, size_t smem, bool watertight = false);
 // Raises the dynamic shared-memory limit of every stack-using kernel.
-cudaError_t ConfigureStackSmem(size_t bytes);
+cudaError_t ConfigureStackSmem();
 
 // Ray queries over one scene (rays: 6 floats each).
 // `fetch` is a device counter the persistent kernel claims query ids from.
