@@ -85,3 +85,17 @@ def test_batches_with_different_stacks_side_by_side(mode):
             r.run(mode, block_size=256, stack_depth=depth)
             films.append(r.film(0)[0].copy())
     assert all(np.array_equal(films[0].view(np.uint32), f.view(np.uint32)) for f in films)
+
+
+def test_deep_glass_scene():
+    """Transmissive shadow queries spill their stacks like all others.  Only next
+    to SDF primitives they run in a kernel that holds them whole."""
+    sc = deep_scene(60, glass=True)
+    with tracer(sc, block_size=256) as t, tracer(sc, block_size=32) as other:
+        assert t.accel_info()["stack_required"] * 256 * 8 > 227 * 1024
+        assert np.array_equal(frame(t).view(np.uint32), frame(other).view(np.uint32))
+    sc.sdf = scenes.sdf_gallery(seed=3).sdf
+    with tracer(sc, block_size=256) as t:
+        with pytest.raises(native.VkptcError) as e:
+            t.render_frame(0, 1)
+        assert e.value.code == native.UNSUPPORTED

@@ -388,8 +388,9 @@ int32_t launch_shape(vkptc_ctx* c, cudaStream_t stream, LaunchShape& ls, bool al
 
 int32_t ensure_stack_smem(vkptc_ctx* c, const LaunchShape& ls) {
   const size_t smem = StackSmemBytes(ls.block, ls.smem_entries);
-  // The transmissive shadow kernel keeps its whole stack in shared memory.
-  const size_t smem_full = c->has_transmissive ? StackSmemBytes(ls.block, ls.stack_cap) : smem;
+  // The shadow kernel of scenes with transmissive materials and SDF primitives
+  // keeps its whole stack in shared memory.
+  const size_t smem_full = c->has_transmissive && c->sdf_count ? StackSmemBytes(ls.block, ls.stack_cap) : smem;
   const size_t need = std::max(smem, smem_full);
   if (need > static_cast<size_t>(c->max_smem_optin)) {
     return fail(c, VKPTC_UNSUPPORTED, "traversal stack does not fit in shared memory (BVH too deep for this block size)");
