@@ -1866,6 +1866,14 @@ void release_graph(vkptc_batch* b) {
   b->graph_key.clear();
 }
 
+// Grows a buffer that the captured graph holds the address of: the graph goes
+// with the old allocation (its key names the launch parameters only).
+template <class T>
+cudaError_t batch_alloc(vkptc_batch* b, DevBuf<T>& buf, size_t n) {
+  if (!buf.ptr || n > buf.count) release_graph(b);
+  return buf.alloc(n);
+}
+
 int32_t batch_clear_films(vkptc_batch* b) {
   for (vkptc_ctx* c : b->jobs) {
     VKPTC_BCUDA(b, cudaMemsetAsync(c->d_film_sum.ptr, 0, c->d_film_sum.bytes(), b->stream), "film clear");
@@ -1948,13 +1956,13 @@ int32_t batch_run_pool(vkptc_batch* b, const vkptc_batch_tuning& t, uint32_t mod
     staging_px += static_cast<unsigned long long>(J.pixels) * J.spp;
     stack_cap = std::max(stack_cap, static_cast<int>(std::max<uint32_t>(1u, c->wide.stack_required)));
   }
-  VKPTC_BCUDA(b, b->staging.alloc(std::max<unsigned long long>(1, staging_px)), "staging alloc");
+  VKPTC_BCUDA(b, batch_alloc(b, b->staging, std::max<unsigned long long>(1, staging_px)), "staging alloc");
   unsigned long long off = 0;
   for (DevJob& J : table) {
     J.staging = b->staging.ptr + off;
     off += static_cast<unsigned long long>(J.pixels) * J.spp;
   }
-  VKPTC_BCUDA(b, b->d_jobs.alloc(table.size()), "job table alloc");
+  VKPTC_BCUDA(b, batch_alloc(b, b->d_jobs, table.size()), "job table alloc");
   VKPTC_BCUDA(b, cudaMemcpy(b->d_jobs.ptr, table.data(), table.size() * sizeof(DevJob), cudaMemcpyHostToDevice),
               "job table upload");
   // ---- launch shape
@@ -2009,7 +2017,7 @@ int32_t batch_run_pool(vkptc_batch* b, const vkptc_batch_tuning& t, uint32_t mod
   const size_t spill_entries =
       bl.stack_cap > bl.smem_entries ? static_cast<size_t>(bl.grid) * bl.block * (bl.stack_cap - bl.smem_entries) : 0;
   // The loop driver's shadow stage may run beside EXTEND: it spills into a second half.
-  if (spill_entries) VKPTC_BCUDA(b, b->spill.alloc(loop ? 2 * spill_entries : spill_entries), "spill alloc");
+  if (spill_entries) VKPTC_BCUDA(b, batch_alloc(b, b->spill, loop ? 2 * spill_entries : spill_entries), "spill alloc");
   bl.spill = spill_entries ? b->spill.ptr : nullptr;
   bl.spill_shadow = spill_entries && loop ? b->spill.ptr + spill_entries : bl.spill;
   // ---- pool
@@ -2020,7 +2028,7 @@ int32_t batch_run_pool(vkptc_batch* b, const vkptc_batch_tuning& t, uint32_t mod
   BatchPool P{};
   LoopPool LP{};
   if (loop) {
-    VKPTC_BCUDA(b, b->l_arena.alloc(carve_count(n) * kLoopBytesPerPath + kCtlStride * kLoopCtlWords * sizeof(uint32_t)), "pool alloc");
+    VKPTC_BCUDA(b, batch_alloc(b, b->l_arena, carve_count(n) * kLoopBytesPerPath + kCtlStride * kLoopCtlWords * sizeof(uint32_t)), "pool alloc");
     Carve carve{b->l_arena.ptr, carve_count(n)};
     for (PathSoA& gen : LP.gen) {
       carve.take(gen.o);
@@ -2043,24 +2051,24 @@ int32_t batch_run_pool(vkptc_batch* b, const vkptc_batch_tuning& t, uint32_t mod
     LP.ctl = reinterpret_cast<uint32_t*>(carve.at);
     LP.capacity = cap;
   } else {
-  VKPTC_BCUDA(b, b->p_job.alloc(n), "pool alloc");
-  VKPTC_BCUDA(b, b->p_local.alloc(n), "pool alloc");
-  VKPTC_BCUDA(b, b->p_depth.alloc(n), "pool alloc");
-  VKPTC_BCUDA(b, b->p_q0.alloc(n), "pool alloc");
-  VKPTC_BCUDA(b, b->p_q1.alloc(n), "pool alloc");
-  VKPTC_BCUDA(b, b->p_shq.alloc(n), "pool alloc");
-  VKPTC_BCUDA(b, b->p_fin.alloc(n), "pool alloc");
-  VKPTC_BCUDA(b, b->p_free.alloc(n), "pool alloc");
-  VKPTC_BCUDA(b, b->p_ctl.alloc(kBatchCtlWords), "pool alloc");
-  VKPTC_BCUDA(b, b->p_rng.alloc(n), "pool alloc");
-  VKPTC_BCUDA(b, b->p_o.alloc(n), "pool alloc");
-  VKPTC_BCUDA(b, b->p_d.alloc(n), "pool alloc");
-  VKPTC_BCUDA(b, b->p_thr.alloc(n), "pool alloc");
-  VKPTC_BCUDA(b, b->p_rad.alloc(n), "pool alloc");
-  VKPTC_BCUDA(b, b->p_sh_o.alloc(n), "pool alloc");
-  VKPTC_BCUDA(b, b->p_sh_d.alloc(n), "pool alloc");
-  VKPTC_BCUDA(b, b->p_sh_c.alloc(n), "pool alloc");
-  VKPTC_BCUDA(b, b->p_hit.alloc(n), "pool alloc");
+  VKPTC_BCUDA(b, batch_alloc(b, b->p_job, n), "pool alloc");
+  VKPTC_BCUDA(b, batch_alloc(b, b->p_local, n), "pool alloc");
+  VKPTC_BCUDA(b, batch_alloc(b, b->p_depth, n), "pool alloc");
+  VKPTC_BCUDA(b, batch_alloc(b, b->p_q0, n), "pool alloc");
+  VKPTC_BCUDA(b, batch_alloc(b, b->p_q1, n), "pool alloc");
+  VKPTC_BCUDA(b, batch_alloc(b, b->p_shq, n), "pool alloc");
+  VKPTC_BCUDA(b, batch_alloc(b, b->p_fin, n), "pool alloc");
+  VKPTC_BCUDA(b, batch_alloc(b, b->p_free, n), "pool alloc");
+  VKPTC_BCUDA(b, batch_alloc(b, b->p_ctl, kBatchCtlWords), "pool alloc");
+  VKPTC_BCUDA(b, batch_alloc(b, b->p_rng, n), "pool alloc");
+  VKPTC_BCUDA(b, batch_alloc(b, b->p_o, n), "pool alloc");
+  VKPTC_BCUDA(b, batch_alloc(b, b->p_d, n), "pool alloc");
+  VKPTC_BCUDA(b, batch_alloc(b, b->p_thr, n), "pool alloc");
+  VKPTC_BCUDA(b, batch_alloc(b, b->p_rad, n), "pool alloc");
+  VKPTC_BCUDA(b, batch_alloc(b, b->p_sh_o, n), "pool alloc");
+  VKPTC_BCUDA(b, batch_alloc(b, b->p_sh_d, n), "pool alloc");
+  VKPTC_BCUDA(b, batch_alloc(b, b->p_sh_c, n), "pool alloc");
+  VKPTC_BCUDA(b, batch_alloc(b, b->p_hit, n), "pool alloc");
   P.capacity = cap;
   P.job = b->p_job.ptr;
   P.local = b->p_local.ptr;
@@ -2154,9 +2162,7 @@ int32_t batch_run_pool(vkptc_batch* b, const vkptc_batch_tuning& t, uint32_t mod
                             std::to_string(bl.block) + "/" + std::to_string(bl.smem_entries) +
                             "/o" + std::to_string(bl.occupancy) + "/b" + std::to_string(t.barrier_spins) +
                             "/" + std::to_string(bl.steps) + "/" + std::to_string(t.sample_limit) + "/" +
-                            std::to_string(b->jobs.size()) + "/" +
-                            std::to_string(reinterpret_cast<uintptr_t>(b->staging.ptr)) + "/" +
-                            std::to_string(reinterpret_cast<uintptr_t>(loop ? static_cast<void*>(b->l_arena.ptr) : static_cast<void*>(b->p_job.ptr)));
+                            std::to_string(b->jobs.size());
     if (!b->graph || b->graph_key != key) {
       release_graph(b);
       VKPTC_BCUDA(b, cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal), "graph capture");
