@@ -471,6 +471,8 @@ int32_t vkptc_trace_rays(vkptc_ctx* ctx, const float* rays, const float* tmax, u
                          uint32_t mode, uint32_t* prim_out, float* t_out);
 /* Same with DEVICE pointers already resident in HBM, enqueued on `stream`
  * (a cudaStream_t; 0 = the context's stream).  No host synchronisation.
+ * d_rays must be 8-byte aligned, the other arrays 4-byte aligned
+ * (VKPTC_INVALID_ARGUMENT otherwise).
  * When `stream` is not the context's stream, it first waits for the work
  * queued on the context's stream and the context's stream then waits for the
  * query (two events made with the context), so a later rebuild or upload on

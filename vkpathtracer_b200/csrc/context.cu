@@ -1755,6 +1755,11 @@ int32_t vkptc_trace_rays_device(vkptc_ctx* ctx, const float* d_rays, const float
   if (!ctx->accel_valid) return fail(ctx, VKPTC_NOT_READY, "acceleration structure not built");
   if (mode > VKPTC_QUERY_ANY) return fail(ctx, VKPTC_INVALID_ARGUMENT, "unknown query mode");
   if (ray_count && (!d_rays || !d_prim_out)) return fail(ctx, VKPTC_INVALID_ARGUMENT, "ray or output pointer is null");
+  // The kernel reads a ray as three pairs of floats.
+  if (ray_count && ((reinterpret_cast<uintptr_t>(d_rays) & 7u) ||
+                    ((reinterpret_cast<uintptr_t>(d_tmax) | reinterpret_cast<uintptr_t>(d_prim_out) |
+                      reinterpret_cast<uintptr_t>(d_t_out)) & 3u)))
+    return fail(ctx, VKPTC_INVALID_ARGUMENT, "d_rays must be 8-byte aligned, the other arrays 4-byte aligned");
   cudaSetDevice(ctx->device);
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
   LaunchShape ls;

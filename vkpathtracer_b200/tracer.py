@@ -468,7 +468,8 @@ class CudaPathTracer:
         return prim, t
 
     def trace_rays_device(self, d_rays: int, d_tmax: int, n: int, mode: int, d_prim: int, d_t: int, stream: int = 0):
-        """Device-pointer variant (e.g. torch tensors' data_ptr()); enqueued, not synchronised."""
+        """Device-pointer variant (e.g. torch tensors' data_ptr(); d_rays 8-byte
+        aligned); enqueued, not synchronised."""
         self._check(self._lib.vkptc_trace_rays_device(self._ctx, d_rays, d_tmax or None, n, mode, d_prim,
                                                       d_t or None, stream or None))
 
