@@ -87,6 +87,8 @@ struct WaveTraceSource {
   __device__ __forceinline__ const GeoView& geo_at(uint32_t) const { return geo; }
   __device__ __forceinline__ bool shadow(uint32_t j) const { return j >= n_ext; }
   __device__ __forceinline__ bool any(uint32_t j) const { return !kTrans && j >= n_ext; }
+  // A query that an SDF primitive occludes is no traversal ray.
+  __device__ __forceinline__ bool traced(uint32_t j) const { return j < n_ext || sh_path[j - n_ext] != kDroppedQuery; }
   __device__ __forceinline__ void load(uint32_t j, V3& o, V3& d, float& tm, GeoView& g) const {
     g = geo;
     const bool sh = j >= n_ext;

@@ -562,7 +562,8 @@ __device__ __forceinline__ bool trace_any(const DevScene& s, V3 o, V3 d, float t
 //   of the tie records.
 // kQueryMixed: Src::any(j) says whether query j ends at its first hit, and
 // Src::finish(j, t, prim, o, d, tmax) may return true to go on with a new
-// origin and bound (o and tmax updated) as the same query.
+// origin and bound (o and tmax updated) as the same query; with kStats,
+// Src::traced(j) whether it counts as a ray.
 // Each warp keeps its lanes busy: whenever lanes are idle it claims that many
 // query ids with one atomic (warp-aggregated) and refills them.  `steps`
 // packs two limits: the low 16 bits are the most traversal steps between
@@ -611,6 +612,9 @@ __device__ __forceinline__ void persistent_traverse(const Src& src, uint32_t n, 
       }
     } else {
       src.finish(j, l.t, prim);
+    }
+    if constexpr (kStats && kMode == kQueryMixed) {
+      if (!src.traced(j)) return false;
     }
     if (kStats) ++(any ? st_any : st).rays;
     return false;
