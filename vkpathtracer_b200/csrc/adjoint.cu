@@ -471,7 +471,7 @@ __device__ __forceinline__ void adj_reverse(const DevScene& s, const DevSettings
         if (mj != kMiss) {
           float2& c = slots[mj * kAdjParams];
           const float y = src[param] - c.y, sum = c.x + y;
-          c.y = (sum - c.x) - y;
+          c.y = isfinite(sum) ? (sum - c.x) - y : 0.0f;   // (an infinite sum has no error; inf - inf would be NaN)
           c.x = sum;
         }
       }
