@@ -57,8 +57,12 @@ struct DevBuf {
     release();
     if (n == 0) return cudaSuccess;
     cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&ptr), n * sizeof(T));
-    if (e == cudaSuccess) count = n;
-    else ptr = nullptr;
+    if (e == cudaSuccess) {
+      count = n;
+    } else {
+      ptr = nullptr;
+      cudaGetLastError();   // the caller gets e; the next launch's check must not
+    }
     return e;
   }
   size_t bytes() const { return count * sizeof(T); }
@@ -218,6 +222,7 @@ struct vkptc_ctx {
   // wave state
   DevBuf<uint8_t> w_arena;
   uint32_t wave_capacity = 0;
+  bool wave_short = false;                // the default wave did not fit: waves of wave_capacity until configured anew
   bool smem_raised = false;               // ConfigureStackSmem() has been called (launches above 48 KB need it)
   int max_smem_optin = 0;                 // the device's shared-memory limit per block
   int shape_block = 0, shape_per_sm = 0;  // resident blocks per SM of the last launch shape
@@ -600,8 +605,19 @@ int32_t run_wave(vkptc_ctx* c, const WaveTile& tile, uint32_t frame) {
 // paths, 21.3 at 2^23, 19.9 at 2^24; 140 bytes a path, allocated as needed).
 constexpr uint32_t kDefaultWavePaths = 1u << 24;
 
-uint32_t wave_paths(const vkptc_ctx* c) {
-  return c->config.wave_paths ? c->config.wave_paths : kDefaultWavePaths;
+// Samples per wave of a frame of px pixels, and the wave's arrays.  A default wave
+// that does not fit in memory is halved; one the caller asked for is not.
+int32_t frame_wave(vkptc_ctx* c, uint32_t px, uint32_t sample_count, uint32_t& per_wave) {
+  const uint32_t asked = c->config.wave_paths;
+  const uint32_t paths = asked ? asked : (c->wave_short ? c->wave_capacity : kDefaultWavePaths);
+  per_wave = std::max(1u, std::min(sample_count, paths / px));
+  int32_t rc;
+  while ((rc = ensure_wave(c, px * per_wave)) == VKPTC_ALLOC_FAILED && !asked && per_wave > 1u) {
+    per_wave = (per_wave + 1u) / 2u;
+    c->wave_short = true;
+  }
+  if (rc == VKPTC_OK && c->wave_short) c->last_error.clear();
+  return rc;
 }
 
 }  // namespace
@@ -702,6 +718,7 @@ int32_t vkptc_configure(vkptc_ctx* ctx, const vkptc_render_settings* settings) {
   cudaSetDevice(ctx->device);
   VKPTC_CUDA(ctx, drain(ctx), "waiting for the work queued on the context's stream");
   ctx->settings = *settings;
+  ctx->wave_short = false;
   VKPTC_CUDA(ctx, ctx->d_film_sum.alloc(std::max<uint64_t>(1, px)), "film alloc");
   VKPTC_CUDA(ctx, ctx->d_film_count.alloc(std::max<uint64_t>(1, px)), "film alloc");
   VKPTC_CUDA(ctx, ctx->d_film_invalid.alloc(std::max<uint64_t>(1, px)), "film alloc");
@@ -1459,7 +1476,9 @@ int32_t vkptc_render_frame(vkptc_ctx* ctx, uint32_t first_sample, uint32_t sampl
   cudaSetDevice(ctx->device);
   const uint32_t px = ctx->settings.width * ctx->settings.height;
   if (px == 0 || sample_count == 0) return VKPTC_OK;
-  const uint32_t per_wave = std::max(1u, std::min(sample_count, wave_paths(ctx) / px));
+  uint32_t per_wave = 1u;
+  const int32_t fits = frame_wave(ctx, px, sample_count, per_wave);
+  if (fits != VKPTC_OK) return fits;
   for (uint32_t s = 0; s < sample_count; s += per_wave) {
     const uint32_t n = std::min(per_wave, sample_count - s);
     WaveTile wt{0u, 0u, ctx->settings.width, ctx->settings.height, first_sample + s, n};
@@ -2028,12 +2047,22 @@ int32_t batch_run_pool(vkptc_batch* b, const vkptc_batch_tuning& t, uint32_t mod
   // ---- pool
   const uint32_t by_default =
       loop ? static_cast<uint32_t>(std::min<unsigned long long>(kDefaultLoopPoolPaths, total)) : kDefaultPoolPaths;
-  const uint32_t cap = std::max<uint32_t>(1024u, t.pool_paths ? t.pool_paths : by_default);
+  uint32_t cap = std::max<uint32_t>(1024u, t.pool_paths ? t.pool_paths : by_default);
+  const auto loop_bytes = [](uint32_t paths) {
+    return carve_count(paths) * kLoopBytesPerPath + kCtlStride * kLoopCtlWords * sizeof(uint32_t);
+  };
+  if (loop) {
+    // a default pool that does not fit in memory is halved, down to the persistent driver's
+    cudaError_t e;
+    while ((e = batch_alloc(b, b->l_arena, loop_bytes(cap))) == cudaErrorMemoryAllocation && !t.pool_paths &&
+           cap > kDefaultPoolPaths)
+      cap = std::max(kDefaultPoolPaths, cap / 2u);
+    VKPTC_BCUDA(b, e, "pool alloc");
+  }
   const size_t n = cap;
   BatchPool P{};
   LoopPool LP{};
   if (loop) {
-    VKPTC_BCUDA(b, batch_alloc(b, b->l_arena, carve_count(n) * kLoopBytesPerPath + kCtlStride * kLoopCtlWords * sizeof(uint32_t)), "pool alloc");
     Carve carve{b->l_arena.ptr, carve_count(n)};
     for (PathSoA& gen : LP.gen) {
       carve.take(gen.o);
