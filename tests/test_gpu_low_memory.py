@@ -1,12 +1,12 @@
-"""Default waves and pools where they do not fit: a frame and a batch go on with
-smaller ones (the film does not depend on their size); sizes that the caller asked
-for are not changed.
+"""Default waves and pools where they do not fit: a frame, a batch and an adjoint
+forward go on with smaller ones (the film does not depend on their size) or, the
+forward, with a path per thread; sizes that the caller asked for are not changed.
 """
 import numpy as np
 import pytest
 
 from vkpathtracer_b200 import native, scenes
-from vkpathtracer_b200.tracer import BatchRenderer, CudaPathTracer
+from vkpathtracer_b200.tracer import BatchRenderer, CudaPathTracer, material_params
 
 pytestmark = pytest.mark.gpu
 
@@ -80,3 +80,23 @@ def test_batch():
                 b.run("loop", pool_paths=1 << 24)
             assert e.value.code == native.ALLOC_FAILED
         assert b.run("loop")["pool_paths"] == 1 << 23
+
+
+def test_adjoint_forward():
+    """2^19 paths: 256 MiB of vertex records and 70 MiB of wave."""
+    sc, st = scenes.inverse_box_scene(), scenes.inverse_settings(256, 256, 8)
+    params, target = material_params(sc.materials), np.full((256, 256, 3), 0.25, np.float32)
+    out = []
+    for leave in (None, 300 * MIB):
+        with CudaPathTracer(bvh="reference") as t:
+            assert t.configure(st) and t.load_scene_snapshot(sc) and t.build_or_update_acceleration()
+            t.adjoint_setup(8, target)
+            if leave is None:
+                loss, image = t.forward(params, image=True)
+            else:
+                with Filled(leave):
+                    loss, image = t.forward(params, image=True)
+            out.append((loss, image, t.backward()))
+    assert out[0][0] == out[1][0]
+    for a, b in zip(out[0][1:], out[1][1:]):
+        assert np.array_equal(bits(a), bits(b))

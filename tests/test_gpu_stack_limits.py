@@ -7,7 +7,7 @@ import pytest
 
 import oracle
 from vkpathtracer_b200 import native, scenes
-from vkpathtracer_b200.tracer import BatchRenderer, CudaPathTracer
+from vkpathtracer_b200.tracer import BatchRenderer, CudaPathTracer, material_params
 
 pytestmark = pytest.mark.gpu
 
@@ -99,3 +99,21 @@ def test_deep_glass_scene():
         with pytest.raises(native.VkptcError) as e:
             t.render_frame(0, 1)
         assert e.value.code == native.UNSUPPORTED
+
+
+def test_adjoint_forward_with_a_stack_too_large_for_its_wavefront():
+    """More paths than the per-path kernel has threads take the renderer's launch
+    shape; where that does not fit, a path per thread."""
+    sc, side = deep_scene(60), 320
+    st = scenes.RenderSettings(width=side, height=side, spp=1, max_depth=3, seed=5)
+    out = []
+    for kw in ({}, dict(block_size=256, stack_depth=1024)):
+        with CudaPathTracer(bvh="reference", **kw) as t:
+            assert t.configure(st) and t.load_scene_snapshot(sc) and t.build_or_update_acceleration()
+            assert t.accel_info()["stack_required"] * 256 * 8 > 227 * 1024
+            t.adjoint_setup(1, np.full((side, side, 3), 0.25, np.float32))
+            loss, image = t.forward(material_params(sc.materials), image=True)
+            out.append((loss, image, t.backward()))
+    assert out[0][0] == out[1][0]
+    for a, b in zip(out[0][1:], out[1][1:]):
+        assert np.array_equal(np.ascontiguousarray(a).view(np.uint32), np.ascontiguousarray(b).view(np.uint32))

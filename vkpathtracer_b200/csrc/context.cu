@@ -2707,7 +2707,7 @@ int32_t vkptc_forward(vkptc_ctx* ctx, const float* params, uint32_t param_count,
   // wavefront: 65,536 paths 0.23 ms with a path per thread against 0.27 as a
   // wavefront, 98,304 0.35 against 0.31, 524,288 1.38 against 0.84 (94,720
   // resident threads).
-  const bool wavefront = record && a.stats.paths > static_cast<uint64_t>(l.grid) * l.block;
+  bool wavefront = record && a.stats.paths > static_cast<uint64_t>(l.grid) * l.block;
   a.recorded = false;
   AdjWaveLaunch wl{};
   if (record) {
@@ -2715,8 +2715,12 @@ int32_t vkptc_forward(vkptc_ctx* ctx, const float* params, uint32_t param_count,
                "adjoint record alloc");
     VKPTC_CUDA(ctx, a.fwd_nrec.alloc(std::max<size_t>(1, a.stats.paths)), "adjoint record alloc");
     if (wavefront && ((rc = ensure_wave(ctx, static_cast<uint32_t>(a.stats.paths))) != VKPTC_OK ||
-                      (rc = adj_wave_launch(ctx, wl)) != VKPTC_OK))
-      return rc;
+                      (rc = adj_wave_launch(ctx, wl)) != VKPTC_OK)) {
+      // no memory for the wave, or no launch with the context's stack settings: a path per thread
+      if (rc != VKPTC_ALLOC_FAILED && rc != VKPTC_UNSUPPORTED) return rc;
+      wavefront = false;
+      ctx->last_error.clear();
+    }
   }
   VKPTC_CUDA(ctx, cudaEventRecord(a.ev[0], ctx->stream), "event");
   if (wavefront) {
