@@ -76,3 +76,18 @@ def test_loop_register_variants_run_at_128_threads(tmp_path, monkeypatch):
     v4 = [c for c in b.calls if c[6] == 4]
     assert v4 and all(c[0] == "loop" and c[3] == 128 for c in v4)
     assert {(c[4], c[5]) for c in v4} == {(8, 8), (16, 8)}     # every stack / steps pair
+
+
+def test_loop_launches_are_timed_once(tmp_path, monkeypatch):
+    """Variants 1 to 3 are one launch of the loop driver, three of the persistent one."""
+    monkeypatch.setenv("VKPTC_AUTOTUNE_CACHE", str(tmp_path / "tune.json"))
+    b = FakeBatch()
+    autotune.tune_batch(b, "k", refine_samples=None, repeats=1)
+    pool = {m: max((c[2] for c in b.calls if c[0] == m), key=[c[2] for c in b.calls if c[0] == m].count) for m in ("loop", "persistent")}
+    shapes = {m: {c[3:] for c in b.calls if c[0] == m and c[2] == pool[m] and c[3]} for m in pool}
+    # two block sizes, two stacks, two step counts; variant 4 beside them
+    assert len(shapes["loop"]) == 8 + 4 and len(shapes["persistent"]) == 3 * 8
+    assert {s[3] for s in shapes["loop"]} == {1, 4}
+    assert autotune._loop_kernels(128, 0) == autotune._loop_kernels(128, 4) == autotune._loop_kernels(256, 4)
+    assert autotune._loop_kernels(64, 0) != autotune._loop_kernels(128, 0)
+    assert autotune._loop_kernels(256, 0) == autotune._loop_kernels(256, 2) != autotune._loop_kernels(128, 2)

@@ -30,6 +30,15 @@ DEFAULT_LOOP_VARIANTS = (4,)
 LOOP_VARIANT_BLOCK = 128
 
 
+def _loop_kernels(block: int, occupancy: int) -> tuple:
+    """What the loop driver launches for a block size and variant: 1 to 3 are the
+    same kernels, and so is 0 above 128 threads; 0 at up to 128 threads has variant
+    4's, which itself sets the block size."""
+    if occupancy >= 4:
+        block = LOOP_VARIANT_BLOCK
+    return block, 4 if occupancy >= 4 or (occupancy == 0 and block <= LOOP_VARIANT_BLOCK) else 3
+
+
 def cache_path() -> str:
     base = os.environ.get("VKPTC_AUTOTUNE_CACHE")
     if base:
@@ -150,6 +159,10 @@ def tune_batch(batch, key: str, modes=DEFAULT_MODES, pools=DEFAULT_POOLS, blocks
         if mode == "loop":
             shapes += [(LOOP_VARIANT_BLOCK, stack, st, occ)
                        for stack, st, occ in itertools.product(stacks, steps, loop_variants)]
+            same = {}   # a launch once, though several variants name it
+            for shape in shapes:
+                same.setdefault((_loop_kernels(shape[0], shape[3]),) + shape[1:3], shape)
+            shapes = list(same.values())
         for block, stack, st, occ in shapes:
             run({"mode": mode, "pool_paths": pool, "block_size": block, "stack_depth": stack, "steps": st,
                  "occupancy": occ})
