@@ -2739,8 +2739,9 @@ int32_t vkptc_forward(vkptc_ctx* ctx, const float* params, uint32_t param_count,
   double host_loss = 0.0;
   VKPTC_CUDA(ctx, cudaMemcpyAsync(&host_loss, a.loss.ptr, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream), "loss readback");
   if (image_rgb) {
-    VKPTC_CUDA(ctx, cudaMemcpyAsync(image_rgb, a.image.ptr, a.image.count * sizeof(float), cudaMemcpyDeviceToHost,
-                                    ctx->stream), "image readback");
+    const size_t floats = 3ull * st.width * st.height;   // the buffer may be larger, from an earlier set-up
+    VKPTC_CUDA(ctx, cudaMemcpyAsync(image_rgb, a.image.ptr, floats * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream),
+               "image readback");
   }
   rc = check_device_error(ctx);
   if (rc != VKPTC_OK) return rc;
