@@ -383,7 +383,10 @@ __device__ __forceinline__ void sdf_persistent(const Src& src, uint32_t n, uint3
         }
       }
     }
-    if (!__any_sync(0xffffffffu, active)) break;
+    if (!__any_sync(0xffffffffu, active)) {
+      if (exhausted) break;
+      continue;   // every query claimed ended at load: there may be more
+    }
     if (active) {
       for (int s = 0; s < steps; ++s) {
         if (sdf_lane_step<kAny>(L, cnt)) {

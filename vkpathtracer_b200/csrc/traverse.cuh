@@ -661,7 +661,10 @@ __device__ __forceinline__ void persistent_traverse(const Src& src, uint32_t n, 
         }
       }
     }
-    if (!__any_sync(0xffffffffu, active)) break;
+    if (!__any_sync(0xffffffffu, active)) {
+      if (exhausted) break;
+      continue;   // every query claimed ended at load: there may be more
+    }
     if (refill_min == 0) {
       if (active) {
         for (int k = 0; k < max_steps; ++k) {
