@@ -2707,7 +2707,8 @@ int32_t vkptc_forward(vkptc_ctx* ctx, const float* params, uint32_t param_count,
   // wavefront: 65,536 paths 0.23 ms with a path per thread against 0.27 as a
   // wavefront, 98,304 0.35 against 0.31, 524,288 1.38 against 0.84 (94,720
   // resident threads).
-  bool wavefront = record && a.stats.paths > static_cast<uint64_t>(l.grid) * l.block;
+  // (At a depth of 0 no shading launch would write the record counts.)
+  bool wavefront = record && st.max_depth > 0u && a.stats.paths > static_cast<uint64_t>(l.grid) * l.block;
   a.recorded = false;
   AdjWaveLaunch wl{};
   if (record) {
