@@ -41,23 +41,23 @@ WORKLOAD = "batch_64_uneven_jobs"
 NODE_BYTES, TRI_BYTES, RAY_IO_BYTES = 128, 48, 32   # wide node line, triangle record, ray in + hit out
 PATH_STATE_BYTES = 2 * 64                            # path state read + written per segment
 # DRAM bytes (read + write) per extension ray of k_lp_extend, from one ncu
-# capture of a steady-state launch of the 4-job case (105.03 MB read + 10.88 MB
+# capture of a steady-state launch of the 4-job case (105.49 MB read + 9.44 MB
 # written for a launch of 2,097,152 rays).
-TRAFFIC_BYTES_PER_EXT_RAY = (105033472 + 10883584) / 2097152
+TRAFFIC_BYTES_PER_EXT_RAY = (105493760 + 9443840) / 2097152
 
 
 def l2_roofline(device, achieved_gbs):
-    """The L2 side of the traversal roofline: the device's L2 read bandwidth,
-    measured here by the library's own probe kernel (vkptc_measure_read_bandwidth:
-    16-byte loads cached in L2 only, 64 passes over a 48 MiB buffer, well under
-    the 126 MB L2), and the traversal stage's algorithmic bytes per second as a
-    fraction of it.  The probe's figure is measured by this function, apart
-    from the HBM peak read from MEASURED_PEAKS.json."""
+    """The traversal roofline: the device's L2 read bandwidth, measured here by
+    the library's own probe kernel (vkptc_measure_read_bandwidth: 16-byte loads
+    cached in L2 only, 64 passes over a 48 MiB buffer, well under the 126 MB L2),
+    and the traversal's algorithmic bytes per second as a fraction of it.  L1 and
+    L2 serve nearly all of these bytes, so they are no fraction of the HBM peak."""
     from vkpathtracer_b200.tracer import CudaPathTracer
     with CudaPathTracer(device=device) as t:
         l2 = max(t.read_bandwidth(48 << 20, 64) for _ in range(3))
-    return {"l2_peak": l2, "l2_peak_kind": "measured here: L2-resident read probe (48 MiB x 64, ld.global.cg)",
-            "l2_frac": achieved_gbs / l2,
+    return {"bound": "l2", "achieved": achieved_gbs, "peak": l2, "unit": "GB/s", "frac": achieved_gbs / l2,
+            "peak_kind": "measured here: L2-resident read probe (48 MiB x 64, ld.global.cg)",
+            "l2_peak": l2, "l2_frac": achieved_gbs / l2,
             "bound_note": "the stage's DRAM traffic is a few percent of its algorithmic bytes (upper BVH levels "
                           "and small scenes stay in L2/L1); l2_frac says how close the node and triangle "
                           "stream is to the L2 bandwidth"}
@@ -851,9 +851,9 @@ def run_ours(args, world, rank, local):
             iters = max(1, tt["iterations"])
             achieved = alg / (stage["extend"] / 1e3) / 1e9
             traffic = TRAFFIC_BYTES_PER_EXT_RAY * ss["ext_rays"] / iters
-            roof = {"kernel": "k_lp_extend (closest-hit traversal stage of the loop driver)", "bound": "hbm",
-                    "achieved": achieved, "peak": hbm_peak, "unit": "GB/s", "frac": achieved / hbm_peak,
-                    "peak_kind": f"{peak_kind} HBM copy bandwidth", "traffic": traffic,
+            roof = {"kernel": "k_lp_extend (closest-hit traversal stage of the loop driver)", "traffic": traffic,
+                    "hbm_peak": hbm_peak, "hbm_peak_kind": f"{peak_kind} HBM copy bandwidth",
+                    "hbm_frac": traffic / (stage["extend"] / iters / 1e3) / 1e9 / hbm_peak,
                     "traffic_note": "per launch: DRAM bytes per extension ray from an ncu capture of a "
                                     "steady-state launch of the 4-job case x extension rays per launch",
                     "alg_bytes_per_launch": alg / iters, "avg_launch_ms": stage["extend"] / iters,
@@ -862,17 +862,15 @@ def run_ours(args, world, rank, local):
                     "shadow_stage_achieved_gbs": (NODE_BYTES * ss["shadow_nodes"] + TRI_BYTES * ss["shadow_tris"]
                                                   + RAY_IO_BYTES * ss["shadow_queries"]) / (stage["shadow"] / 1e3) / 1e9,
                     "nodes_per_ray": nodes / max(1, rays), "tris_per_ray": tris / max(1, rays)}
-            roof.update(l2_roofline(local, achieved))
         else:
             alg = NODE_BYTES * nodes + TRI_BYTES * tris + RAY_IO_BYTES * rays + PATH_STATE_BYTES * ss["segments"] \
                 + 16 * ss["paths"]
             kernel_ms = st0["device_ms"]
             achieved = alg / (kernel_ms / 1e3) / 1e9
             roof = {"kernel": "k_batch (persistent wavefront: regen, closest-hit, shade, any-hit, finish)",
-                    "bound": "hbm", "achieved": achieved, "peak": hbm_peak, "unit": "GB/s", "frac": achieved / hbm_peak,
-                    "peak_kind": f"{peak_kind} HBM copy bandwidth", "traffic": None,
-                    "alg_bytes_per_launch": alg, "avg_launch_ms": kernel_ms, "launches": 1,
+                    "traffic": None, "alg_bytes_per_launch": alg, "avg_launch_ms": kernel_ms, "launches": 1,
                     "nodes_per_ray": nodes / max(1, rays), "tris_per_ray": tris / max(1, rays)}
+        roof.update(l2_roofline(local, achieved))
         if not args.no_rayquery:
             rq = ray_query(local)
         if not args.no_fullframe:

@@ -68,7 +68,8 @@ typedef struct vkptc_config {
                                 spill to global memory); 0 = 12 */
   uint32_t math_mode;        /* 0 = parity (transcendentals in FP64, rounded once), 1 = fast FP32 */
   uint32_t collect_stats;    /* 1 = count node/leaf/triangle visits (device counters) */
-  uint32_t wave_paths;       /* paths per wavefront wave (0 = 16 Mi) */
+  uint32_t wave_paths;       /* paths per wavefront wave, 140 bytes each (0 = 16 Mi, fewer if they do not
+                                fit in memory) */
   uint32_t stage_timing;     /* 1 = CUDA-event timing of every stage launch */
   uint32_t steps;            /* traversal steps between warp refills in the low 16 bits (0 = 8); the
                                 high 16 bits, when non-zero, refill a warp as soon as that many of its
@@ -500,7 +501,8 @@ typedef struct vkptc_batch vkptc_batch;
 #define VKPTC_BATCH_LOOP 2u
 
 typedef struct vkptc_batch_tuning {
-  uint32_t pool_paths;       /* path slots of the persistent launch ("queue capacity"); 0 = default */
+  uint32_t pool_paths;       /* path slots of the persistent launch ("queue capacity"); 0 = default (the
+                                loop driver's is halved down to 2 Mi where it does not fit in memory) */
   uint32_t block_size;       /* 0 = default */
   uint32_t stack_depth;      /* traversal stack entries in shared memory; 0 = default */
   uint32_t steps;            /* traversal steps between warp refills (low 16 bits; 0 = default) and

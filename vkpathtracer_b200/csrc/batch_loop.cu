@@ -276,7 +276,7 @@ __global__ void __launch_bounds__(256) k_lp_sdf_shadow(const DevJob* __restrict_
 // stage takes their hits); without, the shading code carries no SDF steps.
 // kExotic: some job has a transmissive, clear-coat, sheen or toon material or
 // an environment map; without, those branches are compiled out.
-// 80 registers: the 64-job step takes 522 ms, 526 at 64 registers, 538 at 48.
+// 80 registers: the 64-job step took 522 ms, 526 at 64 registers, 538 at 48.
 // Path state is read once and written once per iteration and far larger than
 // L2: streaming loads and stores leave the caches to the scenes (the step 509.2
 // -> 506.6 ms, eight small jobs 11.29 -> 11.25).

@@ -24,7 +24,9 @@
 //      cheapest four subtrees per wide node, wide nodes in depth-first pre-order,
 //      found the same way), triangle records in leaf order and the tie records of the
 //      reference tree.
-// Every array equals the host path's bit for bit (tested).  A non-finite
+// With the reference tree every array equals the host path's bit for bit
+// (tested); the SAH tree's small subtrees are split at other planes than the
+// host's, and its hits are the same.  A non-finite
 // vertex, edge or bound sends the build back to the host path (min/max of NaN
 // depends on operand order, and NaN payloads differ between x86 and the GPU).
 #include "bvh_build.h"

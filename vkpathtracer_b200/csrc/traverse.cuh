@@ -11,7 +11,8 @@
 //    where it is, which the padding covers for coordinates of a few hundred, so
 //    the box of a triangle that a ray meets is not missed there.  (A triangle
 //    whose distance is badly conditioned, |det| near 1e-4, can report one
-//    outside its box; whether it is visited then depends on rounding.)
+//    outside its box; whether it is visited, and whether a bound on the distance
+//    culls its box, then depends on rounding.)
 //  * The reference treats an axis with |d| <= 1e-4 as "parallel" and there only
 //    checks that the origin lies inside the slab, which decides which triangles
 //    it can test at all.  In its own tree the node test does the same.  In another
@@ -26,8 +27,8 @@
 //    evaluates exactly that order from the binary tree kept beside the wide one.
 //
 // The traversal is bound by issued instructions under divergence (about ten of
-// a warp's lanes are active per instruction) with L1's load pipe next (66 % of
-// its wavefronts), not by memory bandwidth, so a step is kept short:
+// a warp's lanes are active per instruction) and by L1 (at 76-80 % of its
+// throughput), not by memory bandwidth, so a step is kept short:
 //  * A wide node holds its children's boxes as lo[4], hi[4] per axis.  On an
 //    axis, with i = 1/d, the slab distances are lo*i - o*i and hi*i - o*i; the
 //    sign of d says which is the nearer one, so the node test loads the near
